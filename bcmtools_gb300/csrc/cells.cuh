@@ -108,13 +108,19 @@ __device__ __forceinline__ float div_pre(float a, float b, float y) {
   r = __fmaf_rn(-b, q, a);
   return __fmaf_rn(r, y, q);
 }
+// FP64: the guards compare the quotient's exponent field, an integer test,
+// because floating-point compares issue on the FP64 pipe (1/64 of the FP32
+// rate on GB300): with six compares a division cost as much of the pipe as
+// the sweep's six products.  2^-60 <= |q| < 2^60 with y != 0 (so 2^-60 <= |b|
+// <= 2^60) puts |a| above 2^-121: no subnormal remainder.  y = 0, a = 0 and
+// everything else outside that range take the other branch.
 __device__ __forceinline__ double div_pre(double a, double b, double y) {
   double q = __dmul_rn(a, y);
-  const double aq = fabs(q);
-  if (y == 0.0 || !(aq <= 0x1p+60) || (aq < 0x1p-60 && aq != 0.0) ||
-      (fabs(a) < 0x1p-900 && a != 0.0))
+  const unsigned e = ((unsigned)__double2hiint(q) >> 20) & 0x7ffu;
+  if (e - (1023u - 60u) >= 120u) {
+    if (a == 0.0 && y != 0.0) return q;  // the sign of a/b
     return __ddiv_rn(a, b);
-  if (aq == 0.0) return q;
+  }
   double r = __fma_rn(-b, q, a);
   q = __fma_rn(r, y, q);
   r = __fma_rn(-b, q, a);

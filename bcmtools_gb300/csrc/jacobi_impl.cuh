@@ -669,65 +669,139 @@ __global__ void __launch_bounds__(NT_, (JacStream<T, N, VC, S, RES, ZERO, NT_, P
       }
     }
   };
-  const bool ok = plane_walk(ring, X0, C, base, a.err, tid, [&](int m) {
-    xlev(m);
-    const T* xm = ring.xp(m);
-    const T* xc = ring.xp(m + 1);
-    const T* xu = ring.xp(m + 2);
-    const T* bp = ring.cp(ZERO ? m : m + 1, 0);
-    T* out = X1 + base + (int64_t)(VC + m) * LXY;
-    T* bout = const_cast<T*>(Bv) + base + (int64_t)(VC + m) * LXY;
+  // x1 of cell c of plane m, to its brick and to every same-level ghost cell it
+  // feeds: the ghost layers of the faces it lies within VC cells of
+  auto put = [&](int m, int c, T v) {
+    const int j = j0 + c * JSTEP;
+    X1[base + (int64_t)(VC + m) * LXY + o[c]] = v;
+    if (XW && xcol >= 0)
+      xface[((xcol >> 1) * 3 + m % 3) * 2 * N + j * 2 + (xcol & 1)] = (float)v;
+    if (xdst) xdst[BL::at(xg, j, m)] = v;
+    if (c == 0 && ylo >= 0) X1[(int64_t)ylo * g.bstride + BL::at(i0, N + j, m)] = v;
+    if (c == CPT - 1 && yhi >= 0) X1[(int64_t)yhi * g.bstride + BL::at(i0, j - N, m)] = v;
     const int zd = m < VC ? zlo : (m >= N - VC ? zhi : -1);
     const int zg = m < VC ? N + m : m - N;
+    if (zd >= 0) X1[(int64_t)zd * g.bstride + BL::at(i0, j, zg)] = v;
+  };
+  // b of a cell: streamed, or made here from the BiCGSTAB vectors streamed
+  auto rhs = [&](int m, int q) -> T {
+    const T* bp = ring.cp(ZERO ? m : m + 1, 0);
+    T* bout = const_cast<T*>(Bv) + base + (int64_t)(VC + m) * LXY;
+    T r = bp[q];
+    if (PRE == kPreP)  // kr_p: p = r + beta (p - gamma q)
+      r = xadd(r, xmul(s_beta, xadd(ring.cp(m, 1)[q], xmul(s_ng, ring.cp(m, NB - 1)[q]))));
+    else if (PRE == kPreS)  // kr_s: s = r - alpha q
+      r = xadd(xmul(s_na, ring.cp(m, NB - 1)[q]), r);
+    if (PRE != 0) bout[q] = r;  // kPreCopy, the first iteration: p = r
+    return r;
+  };
+  bool ok;
+  if constexpr (ZERO && sizeof(T) == 8) {
+    // x0 = 0 in FP64: every product with a coefficient is a zero and r keeps
+    // its value; x1 = 0 - omega (0 - r/Ap) = omega r/Ap, a zero positive.  6 of
+    // the 20 operations.  A coefficient that is not finite would make every
+    // product NaN: so then is omega.
+    const T zz = xadd(xadd(xmul(c1, T(0)), xmul(c2, T(0))),
+                      xadd(xadd(xmul(c3, T(0)), xmul(c4, T(0))), xadd(xmul(c5, T(0)), xmul(c6, T(0)))));
+    const T omz = zz == T(0) ? om : zz;
+    ok = plane_walk(ring, X0, C, base, a.err, tid, [&](int m) {
 #pragma unroll
-    for (int c = 0; c < CPT; c++) {
-      const int q = o[c];
-      T xw, xe, xs_, xn, xmv, up, xcv;
-      if (ZERO) {
-        xw = xe = xs_ = xn = xmv = up = xcv = T(0);
-      } else {
-        xw = xc[q - 1];
-        xe = xc[q + 1];
-        xs_ = xc[q - LX];
-        xn = xc[q + LX];
-        xmv = xm[q];
-        up = xu[q];
-        xcv = xc[q];
+      for (int c = 0; c < CPT; c++) {
+        const T r = rhs(m, o[c]);
+        if (RES) acc.add(r);
+        const T v = xmul(omz, sweep_div(r, c0, rc0));
+        put(m, c, __double_as_longlong(v) == (long long)0x8000000000000000ull ? T(0) : v);
       }
-      T r;
-      if (PRE == kPreP) {  // kr_p: p = r + beta (p - gamma q)
-        r = xadd(bp[q], xmul(s_beta, xadd(ring.cp(m, 1)[q], xmul(s_ng, ring.cp(m, NB - 1)[q]))));
-        bout[q] = r;
-      } else if (PRE == kPreS) {  // kr_s: s = r - alpha q
-        r = xadd(xmul(s_na, ring.cp(m, NB - 1)[q]), bp[q]);
-        bout[q] = r;
-      } else if (PRE == kPreCopy) {  // the first iteration: p = r
-        r = bp[q];
-        bout[q] = r;
-      } else {
-        r = bp[q];
+    });
+  } else {
+    bool iso = false;
+    if constexpr (sizeof(T) == 8) {
+      iso = one_coefficient(c1, c2, c3, c4, c5, c6);
+      if (iso) {
+        ScaledPlanes<N, VC, NT, R> sp;
+        ok = plane_walk(ring, X0, C, base, a.err, tid, [&](int m) {
+          if (m == 0) sp.begin(ring, c1, o, tid);
+          sp.take(ring, c1, o, m, tid);
+          const T* pc = ring.xp(m + 1);
+#pragma unroll
+          for (int c = 0; c < CPT; c++) {
+            const int q = o[c];
+            T r = xsub(rhs(m, q), pc[q - 1]);
+            r = xsub(r, pc[q + 1]);
+            r = xsub(r, pc[q - LX]);
+            r = xsub(r, pc[q + LX]);
+            r = xsub(r, sp.pm[c]);
+            r = xsub(r, sp.pu[c]);
+            if (RES) acc.add(xsub(r, xmul(c0, sp.xc[c])));
+            const T xt = sweep_div(r, c0, rc0);
+            put(m, c, xsub(sp.xc[c], xmul(om, xsub(sp.xc[c], xt))));
+          }
+          sp.shift();
+        });
       }
-      r = xsub(r, xmul(c1, xw));
-      r = xsub(r, xmul(c2, xe));
-      r = xsub(r, xmul(c3, xs_));
-      r = xsub(r, xmul(c4, xn));
-      r = xsub(r, xmul(c5, xmv));
-      r = xsub(r, xmul(c6, up));
-      if (RES) acc.add(xsub(r, xmul(c0, xcv)));
-      const T xt = sweep_div(r, c0, rc0);
-      const T v = xsub(xcv, xmul(om, xsub(xcv, xt)));
-      out[q] = v;
-      // same-level copies: this cell feeds the ghost layer of every face it
-      // lies within VC cells of
-      const int j = j0 + c * JSTEP;
-      if (XW && xcol >= 0)
-        xface[((xcol >> 1) * 3 + m % 3) * 2 * N + j * 2 + (xcol & 1)] = (float)v;
-      if (xdst) xdst[BL::at(xg, j, m)] = v;
-      if (c == 0 && ylo >= 0) X1[(int64_t)ylo * g.bstride + BL::at(i0, N + j, m)] = v;
-      if (c == CPT - 1 && yhi >= 0) X1[(int64_t)yhi * g.bstride + BL::at(i0, j - N, m)] = v;
-      if (zd >= 0) X1[(int64_t)zd * g.bstride + BL::at(i0, j, zg)] = v;
     }
-  });
+    if (!iso) {
+      ok = plane_walk(ring, X0, C, base, a.err, tid, [&](int m) {
+        xlev(m);
+        const T* xm = ring.xp(m);
+        const T* xc = ring.xp(m + 1);
+        const T* xu = ring.xp(m + 2);
+        const T* bp = ring.cp(ZERO ? m : m + 1, 0);
+        T* out = X1 + base + (int64_t)(VC + m) * LXY;
+        T* bout = const_cast<T*>(Bv) + base + (int64_t)(VC + m) * LXY;
+        const int zd = m < VC ? zlo : (m >= N - VC ? zhi : -1);
+        const int zg = m < VC ? N + m : m - N;
+#pragma unroll
+        for (int c = 0; c < CPT; c++) {
+          const int q = o[c];
+          T xw, xe, xs_, xn, xmv, up, xcv;
+          if (ZERO) {
+            xw = xe = xs_ = xn = xmv = up = xcv = T(0);
+          } else {
+            xw = xc[q - 1];
+            xe = xc[q + 1];
+            xs_ = xc[q - LX];
+            xn = xc[q + LX];
+            xmv = xm[q];
+            up = xu[q];
+            xcv = xc[q];
+          }
+          T r;
+          if (PRE == kPreP) {  // kr_p: p = r + beta (p - gamma q)
+            r = xadd(bp[q], xmul(s_beta, xadd(ring.cp(m, 1)[q], xmul(s_ng, ring.cp(m, NB - 1)[q]))));
+            bout[q] = r;
+          } else if (PRE == kPreS) {  // kr_s: s = r - alpha q
+            r = xadd(xmul(s_na, ring.cp(m, NB - 1)[q]), bp[q]);
+            bout[q] = r;
+          } else if (PRE == kPreCopy) {  // the first iteration: p = r
+            r = bp[q];
+            bout[q] = r;
+          } else {
+            r = bp[q];
+          }
+          r = xsub(r, xmul(c1, xw));
+          r = xsub(r, xmul(c2, xe));
+          r = xsub(r, xmul(c3, xs_));
+          r = xsub(r, xmul(c4, xn));
+          r = xsub(r, xmul(c5, xmv));
+          r = xsub(r, xmul(c6, up));
+          if (RES) acc.add(xsub(r, xmul(c0, xcv)));
+          const T xt = sweep_div(r, c0, rc0);
+          const T v = xsub(xcv, xmul(om, xsub(xcv, xt)));
+          out[q] = v;
+          // same-level copies: this cell feeds the ghost layer of every face it
+          // lies within VC cells of
+          const int j = j0 + c * JSTEP;
+          if (XW && xcol >= 0)
+            xface[((xcol >> 1) * 3 + m % 3) * 2 * N + j * 2 + (xcol & 1)] = (float)v;
+          if (xdst) xdst[BL::at(xg, j, m)] = v;
+          if (c == 0 && ylo >= 0) X1[(int64_t)ylo * g.bstride + BL::at(i0, N + j, m)] = v;
+          if (c == CPT - 1 && yhi >= 0) X1[(int64_t)yhi * g.bstride + BL::at(i0, j - N, m)] = v;
+          if (zd >= 0) X1[(int64_t)zd * g.bstride + BL::at(i0, j, zg)] = v;
+        }
+      });
+    }
+  }
   if (!ok) return;  // a copy never arrived: the error word says so
   xlev(N);  // the walk's last barrier made planes N-2 and N-1 visible
   if (RES) {

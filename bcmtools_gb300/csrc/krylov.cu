@@ -112,6 +112,22 @@ struct AxStream {
   static constexpr int MINB = stream_minb<SMEM + 256, (NT_ == 256 ? 6 : 2048 / NT_)>();
 };
 
+// The block's inner products into its partial sums.  A copy that never arrived
+// (the error word says so) makes the sums NaN, so the segment's scalars break
+// down instead of going on.
+template <int NDOT, typename T>
+__device__ __forceinline__ void kr_ax_finish(bool ok, const DotAcc<T>& a0, const DotAcc<T>& a1,
+                                             double* red, double* __restrict__ partial, int b,
+                                             int nb) {
+  const double nan = __longlong_as_double(0x7ff8000000000000ll);
+  const double v0 = kr_block_sum(ok ? a0.value() : nan, red);
+  const double v1 = NDOT == 2 ? kr_block_sum(ok ? a1.value() : nan, red) : 0.0;
+  if (threadIdx.x == 0) {
+    partial[b] = v0;
+    if (NDOT == 2) partial[nb + b] = v1;
+  }
+}
+
 template <typename T, int N, int VC, int NDOT, int S, int NT_ = 256>
 __global__ void __launch_bounds__(NT_, (AxStream<T, N, VC, S, NT_>::MINB)) kr_ax_stream_kernel(
     T* __restrict__ out, const T* __restrict__ x, const T* __restrict__ cf8,
@@ -139,7 +155,36 @@ __global__ void __launch_bounds__(NT_, (AxStream<T, N, VC, S, NT_>::MINB)) kr_ax
   }
   DotAcc<T> a0, a1;
   __syncthreads();  // the ring's barriers are initialised
-  const bool ok = plane_walk(ring, x, C, base, err, tid, [&](int m) {
+  bool ok;
+  if constexpr (sizeof(T) == 8) {
+    if (one_coefficient(c[1], c[2], c[3], c[4], c[5], c[6])) {
+      ScaledPlanes<N, VC, NT, R> sp;
+      ok = plane_walk(ring, x, C, base, err, tid, [&](int m) {
+        if (m == 0) sp.begin(ring, c[1], o, tid);
+        sp.take(ring, c[1], o, m, tid);
+        const T* pc = ring.xp(m + 1);
+        const T* yp = ring.cp(m + 1, 0);
+        T* op = out + base + (int64_t)(VC + m) * LXY;
+#pragma unroll
+        for (int k = 0; k < CPT; k++) {
+          const int q = o[k];
+          T a = xadd(pc[q - 1], pc[q + 1]);
+          a = xadd(a, pc[q - LX]);
+          a = xadd(a, pc[q + LX]);
+          a = xadd(a, sp.pm[k]);
+          a = xadd(a, sp.pu[k]);
+          a = xadd(a, xmul(c[0], sp.xc[k]));
+          op[q] = a;
+          a0.add(a, yp[q]);
+          if (NDOT == 2) a1.add(a, a);
+        }
+        sp.shift();
+      });
+      kr_ax_finish<NDOT>(ok, a0, a1, red, partial, b, g.nb);
+      return;
+    }
+  }
+  ok = plane_walk(ring, x, C, base, err, tid, [&](int m) {
     const T* xm = ring.xp(m);
     const T* xc = ring.xp(m + 1);
     const T* xu = ring.xp(m + 2);
@@ -160,15 +205,7 @@ __global__ void __launch_bounds__(NT_, (AxStream<T, N, VC, S, NT_>::MINB)) kr_ax
       if (NDOT == 2) a1.add(a, a);
     }
   });
-  // a copy that never arrived (the error word says so) makes the sums NaN,
-  // so the segment's scalars break down instead of going on
-  const double nan = __longlong_as_double(0x7ff8000000000000ll);
-  const double v0 = kr_block_sum(ok ? a0.value() : nan, red);
-  const double v1 = NDOT == 2 ? kr_block_sum(ok ? a1.value() : nan, red) : 0.0;
-  if (tid == 0) {
-    partial[b] = v0;
-    if (NDOT == 2) partial[g.nb + b] = v1;
-  }
+  kr_ax_finish<NDOT>(ok, a0, a1, red, partial, b, g.nb);
 }
 
 template <typename T, int N, int VC, int NDOT, int S>
