@@ -83,18 +83,30 @@ __device__ __forceinline__ float lin_r(int i, int I) {
 template <typename T>
 struct C2F;
 
+// (1 - r) a + r b in double for r = -1/4, 1/4, 3/4 or 5/4, the only weights
+// of linearInterpolate: one of the two weights is +-1/4, whose product is exact
+// (a subnormal one apart), so it can go into the sum's FMA without changing the
+// rounded result -- two FP64 operations instead of three.  Weights and operands
+// are picked with integer instructions, since FP64 ones, and conversions from
+// float, issue at 1/64 of the FP32 rate on GB300.
+__device__ __forceinline__ double lerp64(float r, double a, double b) {
+  const bool up = r > 0.5f;  // 3/4, 5/4: the quarter weighs a
+  const float q = up ? 1.0f - r : r;
+  const double wq = __hiloint2double(q < 0.f ? (int)0xbfd00000u : 0x3fd00000, 0);  // +-1/4
+  const double wl = __hiloint2double(q < 0.f ? 0x3ff40000 : 0x3fe80000, 0);        // 5/4, 3/4
+  return __fma_rn(wq, up ? a : b, xmul(wl, up ? b : a));
+}
+
 template <>
 struct C2F<double> {
   // The reference's expression, in double, products and sums in its order.
-  static __device__ __forceinline__ double value(const double* c, int sy, int sz, float rf,
-                                                 float sf, float tf) {
-    const double r = rf, s = sf, t = tf, r1 = 1.0 - r, s1 = 1.0 - s, t1 = 1.0 - t;
-    const double a00 = xadd(xmul(r1, c[0]), xmul(r, c[1]));
-    const double a10 = xadd(xmul(r1, c[sy]), xmul(r, c[sy + 1]));
-    const double a01 = xadd(xmul(r1, c[sz]), xmul(r, c[sz + 1]));
-    const double a11 = xadd(xmul(r1, c[sy + sz]), xmul(r, c[sy + sz + 1]));
-    return xadd(xmul(t1, xadd(xmul(s1, a00), xmul(s, a10))),
-                xmul(t, xadd(xmul(s1, a01), xmul(s, a11))));
+  static __device__ __forceinline__ double value(const double* c, int sy, int sz, float r, float s,
+                                                 float t) {
+    const double a00 = lerp64(r, c[0], c[1]);
+    const double a10 = lerp64(r, c[sy], c[sy + 1]);
+    const double a01 = lerp64(r, c[sz], c[sz + 1]);
+    const double a11 = lerp64(r, c[sy + sz], c[sy + sz + 1]);
+    return lerp64(t, lerp64(s, a00, a10), lerp64(s, a01, a11));
   }
 };
 

@@ -202,9 +202,8 @@ __device__ __forceinline__ void c2f_entry_sep(const VcTask& t, double* __restric
       const int xi = e % X, yi = (e / X) % Y, zi = e / (X * Y);
       const int fx = AX == 0 ? fn : fb[0] + xi;
       const int I = lin_I(fx, N);
-      const double r = (double)lin_r(fx, I), r1 = 1.0 - r;
       const double* c = sf + TL::at(I, lo[1] + yi, lo[2] + zi);
-      scr[e] = xadd(xmul(r1, c[0]), xmul(r, c[1]));
+      scr[e] = lerp64(lin_r(fx, I), c[0], c[1]);
     }
     __syncwarp();
     // stage 2: y- and z-steps of every ghost of this layer
@@ -215,13 +214,11 @@ __device__ __forceinline__ void c2f_entry_sep(const VcTask& t, double* __restric
       face_xyz<AX>(minus ? u - VC : N + u, a, cc, x, y, z);
       face_xyz<AX>(fn, a + P0, cc + P1, fx, fy, fz);
       const int J = lin_I(fy, N), K = lin_I(fz, N);
-      const double s = (double)lin_r(fy, J), s1 = 1.0 - s;
-      const double tt = (double)lin_r(fz, K), t1 = 1.0 - tt;
+      const float s = lin_r(fy, J), tt = lin_r(fz, K);
       const int xi = AX == 0 ? 0 : fx - fb[0];
       const double* A = scr + xi + X * ((J - lo[1]) + Y * (K - lo[2]));
       const double a00 = A[0], a10 = A[X], a01 = A[X * Y], a11 = A[X + X * Y];
-      dst[g.at(x, y, z)] = xadd(xmul(t1, xadd(xmul(s1, a00), xmul(s, a10))),
-                                xmul(tt, xadd(xmul(s1, a01), xmul(s, a11))));
+      dst[g.at(x, y, z)] = lerp64(tt, lerp64(s, a00, a10), lerp64(s, a01, a11));
     }
     __syncwarp();  // the next layer overwrites the scratch
   }
