@@ -17,6 +17,23 @@ struct SorCell<double, FORM> {
     const double* cf = a.coef + 4 * b;
     c0 = cf[0]; cx = cf[1]; cy = cf[2]; cz = cf[3]; om = a.omega; om1 = 1.0 - a.omega;
   }
+  // sor2 on cubic cells whose size is a power of two: cx = cy = cz = 2^k, 0 <=
+  // k <= 60.  Scaling by 2^k commutes with every rounding (short of overflow,
+  // above 2^960), so the update sums first and scales once, in an FMA whose
+  // product is exact: 10 operations a cell instead of 13, the same bits.  The
+  // sweep is bound by the FP64 pipe: 531 -> 411 us an iteration on 4432 blocks
+  // of 16^3, vc = 2 (with the C2F weights of lerp64, ghost.cuh).
+  __device__ __forceinline__ bool power_of_two() const {
+    const long long x = __double_as_longlong(cx);
+    const unsigned e = (unsigned)((unsigned long long)x >> 52);  // with the sign
+    return FORM != 1 && x == __double_as_longlong(cy) && x == __double_as_longlong(cz) &&
+           (x & 0xfffffffffffffll) == 0 && e - 1023u <= 60u;
+  }
+  __device__ __forceinline__ double scaled(double fc, double sw, double ss, double sbt,
+                                           double src) const {
+    const double a = __fma_rn(cx, xadd(xadd(sw, ss), sbt), -src);
+    return xadd(xmul(om, xmul(c0, a)), xmul(om1, fc));
+  }
   __device__ __forceinline__ double operator()(double fc, double sw, double ss, double sbt,
                                                double src) const {
     if (FORM == 1) {

@@ -476,36 +476,47 @@ __global__ void __launch_bounds__(N * N, (pipe_min_blocks<T, N, OP, STAGES>()))
       cell.om = a.omega; cell.om1 = a.om1;
       T* col = tile + TL::at(i, j, 0);
       const T* scol = PS::SPACK ? sv + tid : sv + PS::s_at(i, j, 0);
-      for (int it = 0; it < a.n_inner; it++) {
+      auto sweep = [&](auto&& upd) {
+        for (int it = 0; it < a.n_inner; it++) {
 #pragma unroll
-        for (int c = 0; c < 2; c++) {
-          const int k0 = (c + i + j) & 1;  // cells with (i + j + k) % 2 == c
-          static_assert((N / 2) % 4 == 0, "colour cells in groups of four");
-          for (int h = 0; h < N / 2; h += 4) {
-            // four cells of the colour: every load before the first store
-            // (their neighbours have the other colour, which this half-pass
-            // does not write), so the loads overlap
-            T sw[4], sn[4], sb[4], pc[4], sr[4];
+          for (int c = 0; c < 2; c++) {
+            const int k0 = (c + i + j) & 1;  // cells with (i + j + k) % 2 == c
+            static_assert((N / 2) % 4 == 0, "colour cells in groups of four");
+            for (int h = 0; h < N / 2; h += 4) {
+              // four cells of the colour: every load before the first store
+              // (their neighbours have the other colour, which this half-pass
+              // does not write), so the loads overlap
+              T sw[4], sn[4], sb[4], pc[4], sr[4];
 #pragma unroll
-            for (int u = 0; u < 4; u++) {
-              const int k = k0 + 2 * (h + u);
-              const T* p = col + k * TP;
-              sw[u] = xadd(p[-1], p[1]);
-              sn[u] = xadd(p[-LX], p[LX]);
-              sb[u] = xadd(p[-TP], p[TP]);
-              pc[u] = p[0];
-              sr[u] = PS::HAS_S ? scol[k * PS::SP] : (T)0;
+              for (int u = 0; u < 4; u++) {
+                const int k = k0 + 2 * (h + u);
+                const T* p = col + k * TP;
+                sw[u] = xadd(p[-1], p[1]);
+                sn[u] = xadd(p[-LX], p[LX]);
+                sb[u] = xadd(p[-TP], p[TP]);
+                pc[u] = p[0];
+                sr[u] = PS::HAS_S ? scol[k * PS::SP] : (T)0;
+              }
+#pragma unroll
+              for (int u = 0; u < 4; u++)
+                col[(k0 + 2 * (h + u)) * TP] = upd(pc[u], sw[u], sn[u], sb[u], sr[u]);
             }
-#pragma unroll
-            for (int u = 0; u < 4; u++)
-              col[(k0 + 2 * (h + u)) * TP] = cell(pc[u], sw[u], sn[u], sb[u], sr[u]);
+            __syncthreads();
           }
-          __syncthreads();
+          if (dmask) {
+            tile_dirichlet<T, N, VC, TL>(tile, dmask, dval, a.bc.bcx, tid, NT, dv2f);
+            __syncthreads();
+          }
         }
-        if (dmask) {
-          tile_dirichlet<T, N, VC, TL>(tile, dmask, dval, a.bc.bcx, tid, NT, dv2f);
-          __syncthreads();
-        }
+      };
+      const auto general = [&](T f, T x, T y, T z, T src) { return cell(f, x, y, z, src); };
+      if constexpr (sizeof(T) == 8 && OP != kOpSor1) {
+        if (cell.power_of_two())
+          sweep([&](T f, T x, T y, T z, T src) { return cell.scaled(f, x, y, z, src); });
+        else
+          sweep(general);
+      } else {
+        sweep(general);
       }
       img = tile + TP + (PS::OUT_Y0 + 1) * LX;
       ipitch = TP;
