@@ -1522,6 +1522,7 @@ static int make_op(bcmg_ctx c, int opid, const Field& like, Op<T>* out) {
   out->cc = it->second.d_cc;
   out->cf8 = sizeof(T) == 4 ? (const T*)(const void*)it->second.d_jc32
                             : (const T*)(const void*)it->second.d_jc64;
+  out->rA0 = nullptr;
   for (int k = 0; k < 7; k++) out->A[k] = nullptr;
   if (!out->cc) {
     for (int k = 0; k < 7; k++) {
@@ -1541,13 +1542,36 @@ static bool same_shape(const Field* a, const Field* b) {
   return a && b && a->dtype == b->dtype && a->vc == b->vc;
 }
 
+// RN(1/Ap) of an FP64 operator of coefficient fields, in a work field kept with
+// the context and made anew by every run or solve that takes several sweeps
+// (about a third of a sweep; each sweep then divides in 5 FP64 operations, half
+// of the division sequence's).  Null, and the sweeps divide, for other
+// operators and where the memory budget has no room for the field.
+static const double* op_recip(bcmg_ctx c, int op, int vc, cudaStream_t st) {
+  auto it = c->ops.find(op);
+  if (it == c->ops.end() || it->second.d_cc) return nullptr;
+  const Field* a0 = get_field(c, it->second.fields[0]);
+  if (!a0 || a0->dtype != BCMG_F64 || a0->vc != vc) return nullptr;
+  int id;
+  if (work_field(c, BCMG_F64, vc, 35, &id)) return nullptr;
+  double* out = (double*)get_field(c, id)->d;
+  prof_mark(c, K_OTHER, st, true);
+  const cudaError_t e = launch_recip<double>(out, (const double*)a0->d, geom_of(c, *a0), st);
+  prof_mark(c, K_OTHER, st, false);
+  c->launches++;
+  return e == cudaSuccess ? out : nullptr;
+}
+// Fewest sweeps for which a run makes it.
+constexpr int kRecipMinSweeps = 4;
+
 static int jacobi_sweep(bcmg_ctx c, int op, Field& x1, Field& x0, Field& b, double omega,
-                        cudaStream_t st) {
+                        cudaStream_t st, const double* recip = nullptr) {
   Geom g = geom_of(c, x0);
   if (x0.dtype == BCMG_F64) {
     Op<double> o;
     int rc = make_op(c, op, x0, &o);
     if (rc) return rc;
+    o.rA0 = recip;
     LAUNCH(c, K_JACOBI, st, launch_jacobi<double>((double*)x1.d, (const double*)x0.d, (const double*)b.d, o, g,
                                     omega, st));
   } else {
@@ -1710,8 +1734,7 @@ static int jacobi_choice(bcmg_ctx c, const Field& x) {
   return c->nb <= 1024 ? kJacPush : kJacPullTile;
 }
 
-// pre (with zero_x0, 32^3 streamed pass): the vector update that makes b,
-// fused into the launch (JacPre): kind, r, q and the segments' scalars.
+// pre (with zero_x0): the vector update that makes b, fused into the launch (JacPre): kind, r, q and the segments' scalars.
 struct PreArgs {
   int kind;
   const Field* r;
@@ -1791,10 +1814,11 @@ BCMG_API int bcmg_jacobi_run(bcmg_ctx c, int op, int x, int b, double omega, int
     // between x and a work copy that starts equal to x (cells that neither the
     // sweep nor the ghost update writes keep x's values in both)
     CUDA_TRY(c, cudaMemcpyAsync(fw->d, fx->d, fx->bytes, cudaMemcpyDeviceToDevice, stream));
+    const double* recip = iters >= kRecipMinSweeps ? op_recip(c, op, fx->vc, stream) : nullptr;
     Field* A = fx;
     Field* B = fw;
     for (int k = 0; k < iters; k++) {
-      if ((rc = jacobi_sweep(c, op, *B, *A, *fb, omega, stream))) return rc;
+      if ((rc = jacobi_sweep(c, op, *B, *A, *fb, omega, stream, recip))) return rc;
       if ((rc = impose(c, *B, false, stream))) return rc;
       std::swap(A, B);
     }
@@ -2005,37 +2029,66 @@ BCMG_API int bcmg_jacobi_solve(bcmg_ctx c, int op, int x, int b, double omega, i
   return status == BCMG_DIVERGED ? BCMG_DIVERGED : BCMG_SUCCESS;
 }
 
+// The pass from zero outside the fused kernels: x1's interior from b.
+static int zero_sweep(bcmg_ctx c, int op, Field& x1, Field& b, double omega, const PreArgs* pre,
+                      const double* recip, cudaStream_t st) {
+  const Geom g = geom_of(c, x1);
+  int rc;
+  if (x1.dtype == BCMG_F64) {
+    Op<double> o;
+    if ((rc = make_op(c, op, x1, &o))) return rc;
+    o.rA0 = recip;
+    const JacPre<double> jp{pre ? pre->kind : kPreNone, pre ? (const double*)pre->r->d : nullptr,
+                            pre && pre->q ? (const double*)pre->q->d : nullptr,
+                            pre ? pre->segs : KSegs{}};
+    LAUNCH(c, K_JACOBI, st, launch_kr_zero_pass<double>((double*)x1.d, (double*)b.d, jp, o, g,
+                                                        omega, st));
+  } else {
+    Op<float> o;
+    if ((rc = make_op(c, op, x1, &o))) return rc;
+    const JacPre<float> jp{pre ? pre->kind : kPreNone, pre ? (const float*)pre->r->d : nullptr,
+                           pre && pre->q ? (const float*)pre->q->d : nullptr,
+                           pre ? pre->segs : KSegs{}};
+    LAUNCH(c, K_JACOBI, st, launch_kr_zero_pass<float>((float*)x1.d, (float*)b.d, jp, o, g,
+                                                       (float)omega, st));
+  }
+  return BCMG_SUCCESS;
+}
+
 // Jacobi_PreConditioner (ILS3D.h:452-475) on homogeneous boundary values.
 // n Jacobi passes (sweep, swap, homogeneous ghosts) of the preconditioner.
 // Where the push-form fused sweep applies and no face keeps unupdated ghosts
 // (whose values would then come from the input instead of staying as the
 // output buffer had them), each pass is one fused launch.
-// zero_start: x is zero (ghosts included) before the first pass -- cleared
-// here, or, for the 32^3 push-form kernel, taken as zero without a read.
-// The zero-start pass of a 32^3 preconditioner can also make its right-hand
-// side (PreArgs): the streamed kernels' shapes, fused sweeps.
+// zero_start: x is zero (ghosts included) before the first pass -- taken as
+// zero without a read, or cleared here where some face's ghosts are written by
+// nothing (the pass would then leave them as an earlier solve had them).
+// A zero-start pass can also make its right-hand side (PreArgs).
 static bool jacobi_pre_fuses(bcmg_ctx c, int op, const Field& x, int n) {
-  return n >= 1 && !c->open_faces && jacobi_fusable(c, op, x) && c->nx == 32 && c->ny == 32 &&
-         c->nz == 32 && (x.vc == 1 || x.vc == 2) && plane_stream_enabled();
+  if (n < 1 || c->open_faces) return false;
+  // 32^3: the streamed kernel alone makes it
+  return !(jacobi_fusable(c, op, x) && c->nx == 32) || plane_stream_enabled();
 }
 
 static int jacobi_pre(bcmg_ctx c, int op, Field& x, Field& x0, Field& b, double omega, int n,
-                      cudaStream_t st, bool zero_start = false, const PreArgs* pre = nullptr) {
+                      cudaStream_t st, bool zero_start = false, const PreArgs* pre = nullptr,
+                      const double* recip = nullptr) {
   const bool fused = !c->open_faces && jacobi_fusable(c, op, x);
-  const bool zero_kernel = zero_start && fused && c->nx == 32 && n >= 1;
-  if (pre && !(zero_kernel && jacobi_pre_fuses(c, op, x, n)))
+  const bool zero_pass = zero_start && !c->open_faces && n >= 1;
+  if (pre && !(zero_pass && jacobi_pre_fuses(c, op, x, n)))
     return fail(c, BCMG_FAILURE, "internal: preconditioner pass cannot make its right-hand side");
-  if (zero_start && !zero_kernel) CUDA_TRY(c, cudaMemsetAsync(x.d, 0, x.bytes, st));
+  if (zero_start && !zero_pass) CUDA_TRY(c, cudaMemsetAsync(x.d, 0, x.bytes, st));
   for (int k = 0; k < n; k++) {
     int rc;
     if (fused) {
       rc = jacobi_fused(c, c->ops[op], x, x0, b, omega, true, false, 0, kJacPush, st,
-                        zero_kernel && k == 0, k == 0 ? pre : nullptr);
+                        zero_pass && k == 0, k == 0 ? pre : nullptr);
       if (rc) return rc;
       std::swap(x.d, x0.d);
       continue;
     }
-    rc = jacobi_sweep(c, op, x0, x, b, omega, st);
+    rc = zero_pass && k == 0 ? zero_sweep(c, op, x0, b, omega, pre, recip, st)
+                             : jacobi_sweep(c, op, x0, x, b, omega, st, recip);
     if (rc) return rc;
     std::swap(x.d, x0.d);
     if ((rc = impose(c, x, true, st))) return rc;
@@ -2079,13 +2132,13 @@ struct KrVecs {
 template <typename T>
 static int kr_iteration(bcmg_ctx c, int op, const KrVecs& v, const Op<T>& o, KSegs S,
                         double omega, int n_pre, int max_iter, double eps2, bool keep_best,
-                        bool first, cudaStream_t st) {
+                        bool first, const double* recip, cudaStream_t st) {
   const Geom g = geom_of(c, *v.x);
   double* part = c->d_kpart;
   int rc;
   auto d = [](Field* f) { return (T*)f->d; };
-  // 32^3 blocks: p's and s's updates made by their preconditioner's first
-  // pass (one launch and one read of p / s fewer each)
+  // p's and s's updates made by their preconditioner's first pass (one launch
+  // and one read of p / s fewer each)
   const bool fuse = jacobi_pre_fuses(c, op, *v.p_, n_pre);
   const PreArgs pre_p{first ? kPreCopy : kPreP, v.r, v.q_, S};
   const PreArgs pre_s{kPreS, v.r, v.q_, S};
@@ -2100,12 +2153,14 @@ static int kr_iteration(bcmg_ctx c, int op, const KrVecs& v, const Op<T>& o, KSe
   // side at the cell only (jacobi_smoother, blas.f90:452-502), and the
   // stencils run on p^ and s^.  Leaving the two ghost updates out changes no
   // value.
-  if ((rc = jacobi_pre(c, op, *v.p_, *v.x0, *v.p, omega, n_pre, st, true, fuse ? &pre_p : nullptr)))
+  if ((rc = jacobi_pre(c, op, *v.p_, *v.x0, *v.p, omega, n_pre, st, true, fuse ? &pre_p : nullptr,
+                       recip)))
     return rc;
   LAUNCH(c, K_RESIDUAL, st, launch_kr_ax<T>(d(v.q_), d(v.p_), o, d(v.r0), 1, g, S, part, c->d_err, st));
   LAUNCH(c, K_DOT, st, launch_kr_scalar(part, c->nb, S, KS_ALPHA, max_iter, eps2, keep_best, st));
   if (!fuse) LAUNCH(c, K_BLAS1, st, launch_kr_s<T>(d(v.s), d(v.r), d(v.q_), g, S, st));
-  if ((rc = jacobi_pre(c, op, *v.s_, *v.x0, *v.s, omega, n_pre, st, true, fuse ? &pre_s : nullptr)))
+  if ((rc = jacobi_pre(c, op, *v.s_, *v.x0, *v.s, omega, n_pre, st, true, fuse ? &pre_s : nullptr,
+                       recip)))
     return rc;
   LAUNCH(c, K_RESIDUAL, st, launch_kr_ax<T>(d(v.t_), d(v.s_), o, d(v.s), 2, g, S, part, c->d_err, st));
   LAUNCH(c, K_DOT, st, launch_kr_scalar(part, c->nb, S, KS_GAMMA, max_iter, eps2, keep_best, st));
@@ -2185,11 +2240,14 @@ static int bicgstab_dev(bcmg_ctx c, int op, KrVecs v, double omega, int n_pre, i
     return false;
   };
   if ((rc = read_back())) return rc;
+  // an iteration takes 2 n_pre sweeps
+  const double* recip =
+      running() && 2 * (int64_t)n_pre * limit >= kRecipMinSweeps ? op_recip(c, op, v.x->vc, st) : nullptr;
   int queued = 0, chunk = 1, step = 0;
   while (running()) {
     for (int k = 0; k < chunk; k++, queued++)
       if ((rc = kr_iteration<T>(c, op, v, o, S, omega, n_pre, max_iter, eps2, keep_best,
-                                queued == 0, st)))
+                                queued == 0, recip, st)))
         return rc;
     if ((rc = read_back())) return rc;
     if (++step >= 2) chunk = std::min(2 * chunk, 16);

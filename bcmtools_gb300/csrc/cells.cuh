@@ -153,4 +153,17 @@ __device__ __forceinline__ double sweep_div(double a, double b, double y) {
   return div_pre(a, b, y);
 }
 
+// v with -0 made +0 (the double on the integer pipe).
+__device__ __forceinline__ float positive_zero(float v) { return __fadd_rn(v, 0.f); }
+__device__ __forceinline__ double positive_zero(double v) {
+  return __double_as_longlong(v) == (long long)0x8000000000000000ull ? 0.0 : v;
+}
+
+// The division by a coefficient field's Ap: FP64 through RN(1/Ap) where the
+// caller has made it (y != 0).
+__device__ __forceinline__ float field_div(float a, float b, float) { return __fdiv_rn(a, b); }
+__device__ __forceinline__ double field_div(double a, double b, double y) {
+  return div_pre(a, b, y);
+}
+
 }  // namespace bcmg

@@ -17,6 +17,8 @@
 // faces) and every ghost value x1's interior feeds in the neighbours' bricks
 // of the output field, reading x1 from shared memory.
 #pragma once
+#include <type_traits>
+
 #include "cells.cuh"
 #include "pipe.cuh"
 #include "stage.cuh"
@@ -334,16 +336,20 @@ __global__ void __launch_bounds__(N * N, (BrickStage<T, N, VC, true>::MIN_BLOCKS
 // back from the brick.  NT threads, one warp per face-table entry, UB cells
 // in flight per lane; !COPIES: the same-level entries were written during
 // the sweep and are skipped here.
-template <typename T, int N, int VC, int NT, int UB = 8, bool COPIES = true>
+// src: x1's interior in the layout SL (default: its brick in X1).
+template <typename T, int N, int VC, int NT, int UB = 8, bool COPIES = true,
+          class SL = BrickTile<T, N, VC>>
 __device__ __forceinline__ void jacobi_push_tail(const T* __restrict__ X0, T* __restrict__ X1,
                                                  const Geom& g, const JacArgs<T>& a, int b,
-                                                 int tid, bool zero, int skip_x = 0) {
+                                                 int tid, bool zero, int skip_x = 0,
+                                                 const T* src = nullptr) {
   using BL = BrickTile<T, N, VC>;
   constexpr int NW = NT / 32, LX = BL::LX;
   const int w = tid >> 5, lane = tid & 31;
   const int64_t base = (int64_t)b * g.bstride;
   const T* xs = X0 + base;
   T* fb = X1 + base;
+  if constexpr (std::is_same<SL, BL>::value) src = fb;
   {
     constexpr int W = 2 * VC;
     constexpr int NA = W * W * LX;  // z and y outside: whole rows
@@ -392,11 +398,11 @@ __device__ __forceinline__ void jacobi_push_tail(const T* __restrict__ X0, T* __
         const int p = e % N, q = (e / N) % N, u = e / (N * N);
         const int l = minus ? -1 - u : N + u, l0 = minus ? 0 : N - 1;
         int gi, ii;
-        if (ax == 0) { gi = BL::at(l, p, q); ii = BL::at(l0, p, q); }
-        else if (ax == 1) { gi = BL::at(p, l, q); ii = BL::at(p, l0, q); }
-        else { gi = BL::at(p, q, l); ii = BL::at(p, q, l0); }
+        if (ax == 0) { gi = BL::at(l, p, q); ii = SL::at(l0, p, q); }
+        else if (ax == 1) { gi = BL::at(p, l, q); ii = SL::at(p, l0, q); }
+        else { gi = BL::at(p, q, l); ii = SL::at(p, q, l0); }
         T val = zero ? T(0) : xs[gi];
-        if (dir && u == 0) val = to_t<T>(xsub(v2, (double)fb[ii]));
+        if (dir && u == 0) val = to_t<T>(xsub(v2, (double)src[ii]));
         else if (dir && u == 1 && second) val = (T)v;
         fb[gi] = val;
       }
@@ -406,7 +412,7 @@ __device__ __forceinline__ void jacobi_push_tail(const T* __restrict__ X0, T* __
   if (COPIES) {
     for (int q = p0 + w; q < p1; q += NW) {
       const VcTask t = a.push.tasks[q];
-      push_dispatch<T, N, VC, BL, UB>(t, X1 + (int64_t)t.dst * g.bstride, g, fb, lane);
+      push_dispatch<T, N, VC, SL, UB>(t, X1 + (int64_t)t.dst * g.bstride, g, src, lane);
     }
   } else {
     // the same-level entries were written during the sweep, and so were the
@@ -417,9 +423,86 @@ __device__ __forceinline__ void jacobi_push_tail(const T* __restrict__ X0, T* __
       const VcTask t = a.push.tasks[q];
       if (t.kind == VC_COPY) continue;
       if ((t.face >> 1) == 0 && nx++ < skip_x) continue;
-      push_dispatch_cta<T, N, VC, BL, NT, UB>(t, X1 + (int64_t)t.dst * g.bstride, g, fb, tid);
+      push_dispatch_cta<T, N, VC, SL, NT, UB>(t, X1 + (int64_t)t.dst * g.bstride, g, src, tid);
     }
   }
+}
+
+// A block's interior, N^3 densely.
+template <int N>
+struct DenseTile {
+  static constexpr int LX = N, LXY = N * N;
+  static __device__ __forceinline__ int at(int i, int j, int k) { return i + LX * j + LXY * k; }
+};
+
+// Push-form Jacobi pass from x0 = 0 on 8^3 / 16^3 blocks (a preconditioner's
+// first pass): x1 = omega b / Ap, b read or made from the BiCGSTAB vectors and
+// written back (PRE, JacPre), x1 kept densely in shared memory for the push
+// tail.  x0 = 0 as in jacobi_stream_push_kernel: products of zeros are not
+// formed, a zero of x1 is positive, and a coefficient that is not finite makes
+// x1 NaN.  The sweep kernel took a cleared x0 through the same traffic as any
+// other pass: 5 + 18 us on 1001 blocks of 16^3 in FP32, and the update of p or
+// s 16 and 12 us before it.
+template <typename T, int N, int VC, int PRE>
+__global__ void __launch_bounds__(N * N, (N == 8 ? 12 : sizeof(T) == 4 ? (VC == 1 ? 6 : 4) : (VC == 1 ? 4 : 3)))
+    jacobi_zero_push_kernel(T* __restrict__ X1, T* __restrict__ Bv, Geom g, JacArgs<T> a) {
+  using BL = BrickTile<T, N, VC>;
+  constexpr int NT = N * N, LXY = BL::LXY, U = 4;
+  __shared__ T x1s[N * N * N];
+  const int b = blockIdx.x, tid = threadIdx.x;
+  T s_beta = T(0), s_ng = T(0), s_na = T(0);
+  if (PRE != kPreNone) {
+    const KSeg& sg = a.pre.segs.seg[kseg_of(a.pre.segs, b)];
+    if (sg.status != kRunning) return;
+    s_beta = (T)sg.beta;
+    s_ng = (T)(-sg.gamma);
+    s_na = (T)(-sg.alpha);
+  }
+  const T* cf = a.cf + (int64_t)b * 8;
+  const T c0 = cf[0], rc0 = cf[7];
+  T zz = T(0);
+#pragma unroll
+  for (int q = 1; q < 7; q++) zz = xadd(zz, xmul(cf[q], T(0)));
+  const T om = zz == T(0) ? a.omega : zz;
+  const int64_t o0 = (int64_t)b * g.bstride + BL::at(tid % N, tid / N, 0);
+  const T* rp = (PRE == kPreNone ? Bv : a.pre.r) + o0;
+  const T* qp = PRE == kPreP || PRE == kPreS ? a.pre.q + o0 : nullptr;
+  T* bp = Bv + o0;
+  T* xp = X1 + o0;
+#pragma unroll
+  for (int k0 = 0; k0 < N; k0 += U) {
+    T rv[U], pv[U], qv[U];
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+      rv[u] = rp[(k0 + u) * LXY];
+      if (PRE == kPreP) pv[u] = bp[(k0 + u) * LXY];
+      if (PRE == kPreP || PRE == kPreS) qv[u] = qp[(k0 + u) * LXY];
+    }
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+      T r = rv[u];
+      if (PRE == kPreP) r = xadd(r, xmul(s_beta, xadd(pv[u], xmul(s_ng, qv[u]))));  // kr_p
+      if (PRE == kPreS) r = xadd(xmul(s_na, qv[u]), r);                             // kr_s
+      if (PRE != kPreNone) bp[(k0 + u) * LXY] = r;
+      const T v = positive_zero(xmul(om, sweep_div(r, c0, rc0)));
+      xp[(k0 + u) * LXY] = v;
+      x1s[(k0 + u) * NT + tid] = v;
+    }
+  }
+  __syncthreads();
+  jacobi_push_tail<T, N, VC, NT, 8, true, DenseTile<N>>(X1, X1, g, a, b, tid, true, 0, x1s);
+}
+
+template <typename T, int N, int VC>
+static cudaError_t jacobi_zero_push_launch(T* x1, T* b, const Geom& g, const JacArgs<T>& a,
+                                           cudaStream_t st) {
+  switch (a.pre.kind) {
+    case kPreP: jacobi_zero_push_kernel<T, N, VC, kPreP><<<g.nb, N * N, 0, st>>>(x1, b, g, a); break;
+    case kPreS: jacobi_zero_push_kernel<T, N, VC, kPreS><<<g.nb, N * N, 0, st>>>(x1, b, g, a); break;
+    case kPreCopy: jacobi_zero_push_kernel<T, N, VC, kPreCopy><<<g.nb, N * N, 0, st>>>(x1, b, g, a); break;
+    default: jacobi_zero_push_kernel<T, N, VC, kPreNone><<<g.nb, N * N, 0, st>>>(x1, b, g, a); break;
+  }
+  return cudaGetLastError();
 }
 
 // Push-form fused Jacobi on 32^3 blocks (too large to stage in shared
@@ -710,7 +793,7 @@ __global__ void __launch_bounds__(NT_, (JacStream<T, N, VC, S, RES, ZERO, NT_, P
         const T r = rhs(m, o[c]);
         if (RES) acc.add(r);
         const T v = xmul(omz, sweep_div(r, c0, rc0));
-        put(m, c, __double_as_longlong(v) == (long long)0x8000000000000000ull ? T(0) : v);
+        put(m, c, positive_zero(v));
       }
     });
   } else {
@@ -926,8 +1009,6 @@ cudaError_t launch_jacobi_fused_impl(const T* x0, T* x1, const T* b, const Geom&
                                      int shape, double* partial, int* err, const JacPre<T>* pre,
                                      cudaStream_t st) {
   if (g.nb == 0) return cudaSuccess;
-  if (ghost_mode == kGhostPushZero && !(g.nx == 32 && g.ny == 32 && g.nz == 32))
-    return cudaErrorInvalidValue;
   if (g.nx == 32 && g.ny == 32 && g.nz == 32 && (g.vc == 1 || g.vc == 2)) {
     // 32^3: push form only
     if (ghost_mode != kGhostPush && ghost_mode != kGhostPushZero) return cudaErrorInvalidValue;
@@ -943,6 +1024,17 @@ cudaError_t launch_jacobi_fused_impl(const T* x0, T* x1, const T* b, const Geom&
                      : jacobi_cubic_push_launch<T, 32, 2>(x0, x1, b, g, a, st);
   }
   if (!jacobi_tile_ok<T>(g)) return cudaErrorInvalidValue;
+  if (ghost_mode == kGhostPushZero) {
+    if (partial) return cudaErrorInvalidValue;
+    JacArgs<T> a{0, cf, omega, bc, push, nullptr, err, 1,
+                 pre ? *pre : JacPre<T>{kPreNone, nullptr, nullptr, KSegs{}}};
+    T* bw = const_cast<T*>(b);  // written only where pre makes it
+    if (g.nx == 16)
+      return g.vc == 1 ? jacobi_zero_push_launch<T, 16, 1>(x1, bw, g, a, st)
+                       : jacobi_zero_push_launch<T, 16, 2>(x1, bw, g, a, st);
+    return g.vc == 1 ? jacobi_zero_push_launch<T, 8, 1>(x1, bw, g, a, st)
+                     : jacobi_zero_push_launch<T, 8, 2>(x1, bw, g, a, st);
+  }
   if (ghost_mode != kGhostPush && shape == kJacobiPipe) {
     if (!pipe_shape_ok((int)sizeof(T), g.nx, g.vc, true)) return cudaErrorInvalidValue;
     PipeArgs<T> p{cf, omega, (T)0, 0, bc, push.info, push.out_tasks,

@@ -130,7 +130,29 @@ struct Op {
   const double* cc;
   const T* A[7];
   const T* cf8;  // per block {Ap..At, RN(1/Ap)} rounded to T (constant operators), or null
+  const T* rA0;  // coefficient fields: RN(1/Ap) per cell (launch_recip), or null
 };
+
+// Threads for ncol columns: whole warps, the last round of columns as full as
+// the others.
+inline int column_threads(const Geom& g) {
+  const int ncol = g.nx * g.ny, rounds = (ncol + 255) / 256;
+  return ((ncol + rounds - 1) / rounds + 31) / 32 * 32;
+}
+
+// Planes per CTA of the sweeps: whole blocks once they make about 16 CTAs per
+// SM; fewer blocks are cut into chunks of four planes or more until they do.
+inline int sweep_chunk(const Geom& g) {
+  const int want = (152 * 16 + g.nb - 1) / g.nb;
+  const int most = g.nz / 4 > 1 ? g.nz / 4 : 1;
+  const int chunks = want < most ? want : most;
+  return (g.nz + chunks - 1) / chunks;
+}
+
+// RN(1/Ap) of every interior cell of a coefficient field, 0 where the FP64
+// sweeps' division by it does not apply.
+template <typename T>
+cudaError_t launch_recip(T* out, const T* a, const Geom& g, cudaStream_t st);
 
 template <typename T>
 cudaError_t launch_jacobi(T* x1, const T* x0, const T* b, Op<T> op, const Geom& g, T omega,
@@ -150,15 +172,14 @@ cudaError_t launch_jacobi(T* x1, const T* x0, const T* b, Op<T> op, const Geom& 
 // fed face -- x1's ghosts need a ghost update before anything else reads
 // them.  kGhostAsIs: the pull kernel on x0's ghosts as they are (the first
 // launch of a run).
-// kGhostPushZero: the push form on 32^3 blocks with x0 taken as zero
-// everywhere (not read): the first pass of a preconditioner from zero.
+// kGhostPushZero: the push form with x0 taken as zero everywhere (not read):
+// the first pass of a preconditioner from zero.
 enum : int { kGhostPush = 0, kGhostPull = 1, kGhostAsIs = 2, kGhostPushZero = 3 };
 // Kernel shapes of the pull-form Jacobi sweep: one CTA per block, or the
 // persistent double-buffered pipeline.
 enum : int { kJacobiTile = 1, kJacobiPipe = 2 };
 // The BiCGSTAB preconditioner's zero-start pass made in one launch with the
-// vector update that produces its right-hand side b (32^3 blocks, streamed
-// kernel): kind kPreP b = r + beta (b - gamma q) (kr_p), kPreS b = r -
+// vector update that produces its right-hand side b: kind kPreP b = r + beta (b - gamma q) (kr_p), kPreS b = r -
 // alpha q (kr_s), kPreCopy b = r; the new b is written back, the scalars
 // come from the segments' records, blocks of finished segments are skipped.
 enum : int { kPreNone = 0, kPreP = 1, kPreS = 2, kPreCopy = 3 };
@@ -222,6 +243,11 @@ cudaError_t launch_kr_ax(T* out, const T* x, Op<T> op, const T* y0, int ndot, co
 template <typename T>
 cudaError_t launch_kr_xr(T* x, T* r, const T* p_, const T* s_, const T* s, const T* t,
                          const T* r0, const Geom& g, KSegs S, double* partial, int* err, cudaStream_t st);
+// A preconditioner's pass from x0 = 0 on blocks of any shape or coefficient
+// fields: x1's interior from b, or from b made of the BiCGSTAB vectors (pre).
+template <typename T>
+cudaError_t launch_kr_zero_pass(T* x1, T* b, const JacPre<T>& pre, const Op<T>& op, const Geom& g,
+                                T omega, cudaStream_t st);
 template <typename T>
 cudaError_t launch_kr_dot2(const T* x, const T* y, const T* u, const T* v, const Geom& g,
                            double* partial, cudaStream_t st);

@@ -11,6 +11,8 @@
 //                          block sums in FP64)
 //   axpy/xpay/axpyz/axpbypz blas.f90:242-377
 // Decomposition: one CTA per block; sweeps march each (i,j) column along k.
+#include <type_traits>
+
 #include "cells.cuh"
 #include "common.cuh"
 #include "kernels.h"
@@ -34,49 +36,143 @@ __device__ __forceinline__ double block_sum(double v, double* red) {
 }
 
 // ---------------------------------------------------------------------------
-// Operator coefficients of one cell.
-template <typename T, bool CC>
-struct Coefs {
-  T v[7];
-  __device__ __forceinline__ void load_block(const Op<T>& op, int b) {
-    if (CC)
-      for (int c = 0; c < 7; c++) v[c] = to_t<T>(op.cc[b * 7 + c]);
-  }
-  __device__ __forceinline__ T get(const Op<T>& op, int c, int64_t p) const {
-    return CC ? v[c] : op.A[c][p];
-  }
+// Sweeps over blocks of any shape and operators of coefficient fields:
+//   MODE 0 calc_ax, 1 calc_r, 2 calc_r2 (FP64 per-block partials), 3
+//   jacobi_smoother: x1 = x0 - omega (x0 - r/Ap),
+//   r = b - Aw xW - Ae xE - As xS - An xN - Ab xB - At xT.
+// CC: per-block constants cf8 (rounded to T, RN(1/Ap) last); else the fields.
+//
+// CTA (b, z) takes planes [z zc, (z + 1) zc) of block b, a thread a column at a
+// time, the loads of U planes issued before the first of them is used: the
+// float sweep with coefficient fields moves 40 bytes a cell and is bound by the
+// bytes a thread has in flight (4432 blocks of 16^3: 210 us with one plane's).
+// Chunks of planes (sweep_chunk) let a mesh of few blocks fill the chip: 328
+// blocks of 24x20x12 leave some SMs three blocks and others two.
+template <typename T, bool CC, int MODE, int V>
+struct SweepCells {
+  T w[V], e[V], s[V], n[V], up[V], bv[V], c[CC ? 1 : V][7], rc[V];
 };
 
-// jacobi_smoother: x1 = x0 - omega (x0 - r/Ap),
-// r = b - Aw xW - Ae xE - As xS - An xN - Ab xB - At xT.
-template <typename T, bool CC>
-__global__ void __launch_bounds__(256) jacobi_kernel(T* __restrict__ x1, const T* __restrict__ x0,
-                                                     const T* __restrict__ bb, Op<T> op, Geom g,
-                                                     T omega) {
+template <typename T, bool CC, int MODE, int U>
+__global__ void __launch_bounds__(256) sweep_kernel(T* __restrict__ out, const T* __restrict__ x,
+                                                    const T* __restrict__ bb, Op<T> op, Geom g,
+                                                    T omega, int zc,
+                                                    double* __restrict__ partial) {
+  __shared__ double red[32];
   const int b = blockIdx.x;
   const int64_t base = (int64_t)b * g.bstride;
-  Coefs<T, CC> cf;
-  cf.load_block(op, b);
-  const int nx = g.nx, ny = g.ny, nz = g.nz, sy = g.sy, sz = g.sz;
-  for (int ij = threadIdx.x; ij < nx * ny; ij += blockDim.x) {
-    const int i = ij % nx, j = ij / nx;
-    int64_t p = base + g.at(i, j, 0);
-    T xm = x0[p - sz], xc = x0[p];
-    for (int k = 0; k < nz; k++, p += sz) {
-      const T xp = x0[p + sz];
-      T r = bb[p];
-      r = xsub(r, xmul(cf.get(op, 1, p), x0[p - 1]));
-      r = xsub(r, xmul(cf.get(op, 2, p), x0[p + 1]));
-      r = xsub(r, xmul(cf.get(op, 3, p), x0[p - sy]));
-      r = xsub(r, xmul(cf.get(op, 4, p), x0[p + sy]));
-      r = xsub(r, xmul(cf.get(op, 5, p), xm));
-      r = xsub(r, xmul(cf.get(op, 6, p), xp));
-      const T xt = xdiv(r, cf.get(op, 0, p));
-      x1[p] = xsub(xc, xmul(omega, xsub(xc, xt)));
-      xm = xc;
-      xc = xp;
+  const int nx = g.nx, ncol = g.nx * g.ny, sy = g.sy, sz = g.sz;
+  const int z0 = blockIdx.y * zc, z1 = min(g.nz, z0 + zc);
+  const T* xb = x + base;
+  const T* rb = MODE != 0 ? bb + base : nullptr;
+  T* ob = MODE != 2 ? out + base : nullptr;
+  const T* ra = (MODE == 3 && !CC && op.rA0) ? op.rA0 + base : nullptr;
+  T cc[8];
+  if (CC) {
+#pragma unroll
+    for (int q = 0; q < 8; q++) cc[q] = op.cf8[(int64_t)b * 8 + q];
+  }
+  double acc = 0.0;
+  for (int ij = threadIdx.x; ij < ncol; ij += blockDim.x) {
+    int o = g.at(ij % nx, ij / nx, z0);
+    T xm = xb[o - sz], xc = xb[o];
+    auto planes = [&](auto vt) {
+      constexpr int V = decltype(vt)::value;
+      SweepCells<T, CC, MODE, V> d;
+#pragma unroll
+      for (int u = 0; u < V; u++) {
+        const int q = o + u * sz;
+        d.w[u] = xb[q - 1];
+        d.e[u] = xb[q + 1];
+        d.s[u] = xb[q - sy];
+        d.n[u] = xb[q + sy];
+        d.up[u] = xb[q + sz];
+        if (MODE != 0) d.bv[u] = rb[q];
+        if (!CC) {
+#pragma unroll
+          for (int f = 0; f < 7; f++) d.c[u][f] = op.A[f][base + q];
+          if (MODE == 3) d.rc[u] = ra ? ra[q] : T(0);
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < V; u++) {
+        const T* c = CC ? cc : d.c[CC ? 0 : u];
+        const int q = o + u * sz;
+        if (MODE == 0) {
+          T a = xmul(c[1], d.w[u]);
+          a = xadd(a, xmul(c[2], d.e[u]));
+          a = xadd(a, xmul(c[3], d.s[u]));
+          a = xadd(a, xmul(c[4], d.n[u]));
+          a = xadd(a, xmul(c[5], xm));
+          a = xadd(a, xmul(c[6], d.up[u]));
+          ob[q] = xadd(a, xmul(c[0], xc));
+        } else {
+          T r = d.bv[u];
+          r = xsub(r, xmul(c[1], d.w[u]));
+          r = xsub(r, xmul(c[2], d.e[u]));
+          r = xsub(r, xmul(c[3], d.s[u]));
+          r = xsub(r, xmul(c[4], d.n[u]));
+          r = xsub(r, xmul(c[5], xm));
+          r = xsub(r, xmul(c[6], d.up[u]));
+          if (MODE == 3) {
+            const T xt = CC ? sweep_div(r, c[0], cc[7]) : field_div(r, c[0], d.rc[u]);
+            ob[q] = xsub(xc, xmul(omega, xsub(xc, xt)));
+          } else {
+            r = xsub(r, xmul(c[0], xc));
+            if (MODE == 1) ob[q] = r;
+            else acc = __fma_rn((double)r, (double)r, acc);
+          }
+        }
+        xm = xc;
+        xc = d.up[u];
+      }
+      o += V * sz;
+    };
+    int k = z0;
+    for (; k + U <= z1; k += U) planes(std::integral_constant<int, U>{});
+    for (; k < z1; k++) planes(std::integral_constant<int, 1>{});
+  }
+  if (MODE == 2) {
+    acc = block_sum(acc, red);
+    if (threadIdx.x == 0) partial[b] = acc;
+  }
+}
+
+template <typename T, int MODE>
+static cudaError_t launch_sweep(T* out, const T* x, const T* b, const Op<T>& op, const Geom& g,
+                                T omega, double* partial, cudaStream_t st) {
+  const int zc = MODE == 2 ? g.nz : sweep_chunk(g);
+  const dim3 grid(g.nb, (g.nz + zc - 1) / zc);
+  const int nt = column_threads(g);
+  constexpr int UC = sizeof(T) == 4 ? 4 : 2, UF = 2;
+  if (op.cc)
+    sweep_kernel<T, true, MODE, UC><<<grid, nt, 0, st>>>(out, x, b, op, g, omega, zc, partial);
+  else
+    sweep_kernel<T, false, MODE, UF><<<grid, nt, 0, st>>>(out, x, b, op, g, omega, zc, partial);
+  return cudaGetLastError();
+}
+
+// RN(1/Ap) of every interior cell, 0 where the two-FMA division does not cover
+// Ap (div_pre, cells.cuh): made once for the sweeps of a run or solve.
+template <typename T>
+__global__ void __launch_bounds__(256) recip_kernel(T* __restrict__ out, const T* __restrict__ a,
+                                                    Geom g) {
+  const int64_t base = (int64_t)blockIdx.x * g.bstride;
+  const int ncol = g.nx * g.ny;
+  for (int ij = threadIdx.x; ij < ncol; ij += blockDim.x) {
+    int64_t o = base + g.at(ij % g.nx, ij / g.nx, 0);
+    for (int k = 0; k < g.nz; k++, o += g.sz) {
+      const T v = a[o], m = v < T(0) ? -v : v;
+      out[o] = (m >= T(0x1p-60) && m <= T(0x1p+60)) ? xdiv(T(1), v) : T(0);
     }
   }
+}
+
+template <typename T>
+cudaError_t launch_recip(T* out, const T* a, const Geom& g, cudaStream_t st) {
+  if (g.nb == 0) return cudaSuccess;
+  recip_kernel<T><<<g.nb, column_threads(g), 0, st>>>(out, a, g);
+  return cudaGetLastError();
 }
 
 template <typename T>
@@ -154,71 +250,7 @@ cudaError_t launch_jacobi(T* x1, const T* x0, const T* b, Op<T> op, const Geom& 
     }
     return cudaGetLastError();
   }
-  const int threads = min(256, g.nx * g.ny);
-  if (op.cc)
-    jacobi_kernel<T, true><<<g.nb, threads, 0, st>>>(x1, x0, b, op, g, omega);
-  else
-    jacobi_kernel<T, false><<<g.nb, threads, 0, st>>>(x1, x0, b, op, g, omega);
-  return cudaGetLastError();
-}
-
-// calc_ax (mode 0), calc_r (mode 1), calc_r2 (mode 2, FP64 per-block partials).
-template <typename T, bool CC, int MODE>
-__global__ void __launch_bounds__(256) residual_kernel(T* __restrict__ out, const T* __restrict__ x,
-                                                       const T* __restrict__ bb, Op<T> op, Geom g,
-                                                       double* __restrict__ partial) {
-  __shared__ double red[32];
-  const int b = blockIdx.x;
-  const int64_t base = (int64_t)b * g.bstride;
-  Coefs<T, CC> cf;
-  cf.load_block(op, b);
-  const int nx = g.nx, ny = g.ny, nz = g.nz, sy = g.sy, sz = g.sz;
-  double acc = 0.0;
-  for (int ij = threadIdx.x; ij < nx * ny; ij += blockDim.x) {
-    const int i = ij % nx, j = ij / nx;
-    int64_t p = base + g.at(i, j, 0);
-    T xm = x[p - sz], xc = x[p];
-    for (int k = 0; k < nz; k++, p += sz) {
-      const T xp = x[p + sz];
-      if (MODE == 0) {
-        T a = xmul(cf.get(op, 1, p), x[p - 1]);
-        a = xadd(a, xmul(cf.get(op, 2, p), x[p + 1]));
-        a = xadd(a, xmul(cf.get(op, 3, p), x[p - sy]));
-        a = xadd(a, xmul(cf.get(op, 4, p), x[p + sy]));
-        a = xadd(a, xmul(cf.get(op, 5, p), xm));
-        a = xadd(a, xmul(cf.get(op, 6, p), xp));
-        a = xadd(a, xmul(cf.get(op, 0, p), xc));
-        out[p] = a;
-      } else {
-        T r = bb[p];
-        r = xsub(r, xmul(cf.get(op, 1, p), x[p - 1]));
-        r = xsub(r, xmul(cf.get(op, 2, p), x[p + 1]));
-        r = xsub(r, xmul(cf.get(op, 3, p), x[p - sy]));
-        r = xsub(r, xmul(cf.get(op, 4, p), x[p + sy]));
-        r = xsub(r, xmul(cf.get(op, 5, p), xm));
-        r = xsub(r, xmul(cf.get(op, 6, p), xp));
-        r = xsub(r, xmul(cf.get(op, 0, p), xc));
-        if (MODE == 1) out[p] = r;
-        else acc += (double)r * (double)r;
-      }
-      xm = xc;
-      xc = xp;
-    }
-  }
-  if (MODE == 2) {
-    acc = block_sum(acc, red);
-    if (threadIdx.x == 0) partial[b] = acc;
-  }
-}
-
-template <typename T, int MODE>
-static void residual_dispatch(T* out, const T* x, const T* b, Op<T> op, const Geom& g,
-                              double* partial, cudaStream_t st) {
-  const int threads = min(256, g.nx * g.ny);
-  if (op.cc)
-    residual_kernel<T, true, MODE><<<g.nb, threads, 0, st>>>(out, x, b, op, g, partial);
-  else
-    residual_kernel<T, false, MODE><<<g.nb, threads, 0, st>>>(out, x, b, op, g, partial);
+  return launch_sweep<T, 3>(x1, x0, b, op, g, omega, nullptr, st);
 }
 
 // calc_ax / calc_r / calc_r2 on cubic blocks with a constant operator: one
@@ -305,10 +337,9 @@ cudaError_t launch_residual(T* out, const T* x, const T* b, Op<T> op, const Geom
     else residual_cubic<T, 2>(out, x, b, op, g, partial, st);
     return cudaGetLastError();
   }
-  if (mode == 0) residual_dispatch<T, 0>(out, x, b, op, g, partial, st);
-  else if (mode == 1) residual_dispatch<T, 1>(out, x, b, op, g, partial, st);
-  else residual_dispatch<T, 2>(out, x, b, op, g, partial, st);
-  return cudaGetLastError();
+  if (mode == 0) return launch_sweep<T, 0>(out, x, b, op, g, T(0), partial, st);
+  if (mode == 1) return launch_sweep<T, 1>(out, x, b, op, g, T(0), partial, st);
+  return launch_sweep<T, 2>(out, x, b, op, g, T(0), partial, st);
 }
 
 // ---------------------------------------------------------------------------
@@ -316,6 +347,7 @@ template <typename T>
 __global__ void __launch_bounds__(256) dot_partial_kernel(const T* __restrict__ x,
                                                           const T* __restrict__ y, Geom g,
                                                           double* __restrict__ partial) {
+  constexpr int U = 8;
   __shared__ double red[32];
   const int b = blockIdx.x;
   const int64_t base = (int64_t)b * g.bstride;
@@ -331,8 +363,7 @@ __global__ void __launch_bounds__(256) dot_partial_kernel(const T* __restrict__ 
       // per-element FP64 accumulation.
       float s = 0.f, c = 0.f;
       double wide = 0.0;
-      for (int k = 0; k < nz; k++, p += g.sz) {
-        const float xv = x[p], yv = y[p];
+      auto add = [&](float xv, float yv) {
         const ff q = two_prod(xv, yv);
         const float m = fabsf(q.hi);
         if (m >= 0x1p-100f && m < 0x1p100f) {
@@ -342,10 +373,35 @@ __global__ void __launch_bounds__(256) dot_partial_kernel(const T* __restrict__ 
         } else if (xv != 0.f && yv != 0.f) {
           wide += (double)xv * (double)yv;
         }
+      };
+      // the loads of U planes before the first product (whose branch would
+      // keep the next load behind it)
+      int k = 0;
+      for (; k + U <= nz; k += U, p += (int64_t)U * g.sz) {
+        float xv[U], yv[U];
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+          xv[u] = x[p + (int64_t)u * g.sz];
+          yv[u] = y[p + (int64_t)u * g.sz];
+        }
+#pragma unroll
+        for (int u = 0; u < U; u++) add(xv[u], yv[u]);
       }
+      for (; k < nz; k++, p += g.sz) add(x[p], y[p]);
       acc += (double)s + (double)c + wide;
     } else {
-      for (int k = 0; k < nz; k++, p += g.sz) acc += (double)x[p] * (double)y[p];
+      int k = 0;
+      for (; k + U <= nz; k += U, p += (int64_t)U * g.sz) {
+        T xv[U], yv[U];
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+          xv[u] = x[p + (int64_t)u * g.sz];
+          yv[u] = y[p + (int64_t)u * g.sz];
+        }
+#pragma unroll
+        for (int u = 0; u < U; u++) acc += (double)xv[u] * (double)yv[u];
+      }
+      for (; k < nz; k++, p += g.sz) acc += (double)x[p] * (double)y[p];
     }
   }
   acc = block_sum(acc, red);
@@ -375,22 +431,41 @@ cudaError_t launch_reduce_final(const double* partial, int n, double* out, cudaS
 }
 
 // ---------------------------------------------------------------------------
+// CTA (b, z): planes [z zc, (z + 1) zc) of block b (sweep_chunk), the loads of
+// U planes before the first store (z may be x or y: a cell reads only itself).
 template <typename T, int KIND>
-__global__ void __launch_bounds__(256) blas1_kernel(T* __restrict__ z, const T* __restrict__ x,
-                                                    const T* __restrict__ y, T a, T bc, Geom g) {
-  const int b = blockIdx.x;
-  const int64_t base = (int64_t)b * g.bstride;
-  const int nx = g.nx, ny = g.ny, nz = g.nz;
-  for (int ij = threadIdx.x; ij < nx * ny; ij += blockDim.x) {
-    const int i = ij % nx, j = ij / nx;
-    int64_t p = base + g.at(i, j, 0);
-    for (int k = 0; k < nz; k++, p += g.sz) {
-      if (KIND == 0) z[p] = xadd(z[p], xmul(a, x[p]));                       // axpy
-      else if (KIND == 1) z[p] = xadd(x[p], xmul(a, z[p]));                  // xpay
-      else if (KIND == 2) z[p] = xadd(xmul(a, x[p]), y[p]);                  // axpyz
-      else if (KIND == 3) z[p] = xadd(xadd(xmul(a, x[p]), xmul(bc, y[p])), z[p]);  // axpbypz
-      else z[p] = xmul(a, z[p]);                                            // scal
-    }
+__global__ void __launch_bounds__(256) blas1_kernel(T* z, const T* x, const T* y, T a, T bc,
+                                                    Geom g, int zc) {
+  constexpr int U = 4;
+  const int64_t base = (int64_t)blockIdx.x * g.bstride;
+  const int nx = g.nx, ncol = g.nx * g.ny;
+  const int z0 = blockIdx.y * zc, z1 = min(g.nz, z0 + zc);
+  for (int ij = threadIdx.x; ij < ncol; ij += blockDim.x) {
+    int64_t p = base + g.at(ij % nx, ij / nx, z0);
+    auto planes = [&](auto vt) {
+      constexpr int V = decltype(vt)::value;
+      T zv[V], xv[V], yv[V];
+#pragma unroll
+      for (int u = 0; u < V; u++) {
+        const int64_t q = p + (int64_t)u * g.sz;
+        if (KIND != 2) zv[u] = z[q];
+        if (KIND != 4) xv[u] = x[q];
+        if (KIND == 2 || KIND == 3) yv[u] = y[q];
+      }
+#pragma unroll
+      for (int u = 0; u < V; u++) {
+        const int64_t q = p + (int64_t)u * g.sz;
+        if (KIND == 0) z[q] = xadd(zv[u], xmul(a, xv[u]));                                // axpy
+        else if (KIND == 1) z[q] = xadd(xv[u], xmul(a, zv[u]));                           // xpay
+        else if (KIND == 2) z[q] = xadd(xmul(a, xv[u]), yv[u]);                           // axpyz
+        else if (KIND == 3) z[q] = xadd(xadd(xmul(a, xv[u]), xmul(bc, yv[u])), zv[u]);    // axpbypz
+        else z[q] = xmul(a, zv[u]);                                                      // scal
+      }
+      p += (int64_t)V * g.sz;
+    };
+    int k = z0;
+    for (; k + U <= z1; k += U) planes(std::integral_constant<int, U>{});
+    for (; k < z1; k++) planes(std::integral_constant<int, 1>{});
   }
 }
 
@@ -398,13 +473,14 @@ template <typename T>
 cudaError_t launch_blas1(int kind, T* z, const T* x, const T* y, T a, T b, const Geom& g,
                          cudaStream_t st) {
   if (g.nb == 0) return cudaSuccess;
-  const int th = min(256, g.nx * g.ny);
+  const int zc = sweep_chunk(g), th = column_threads(g);
+  const dim3 grid(g.nb, (g.nz + zc - 1) / zc);
   switch (kind) {
-    case 0: blas1_kernel<T, 0><<<g.nb, th, 0, st>>>(z, x, y, a, b, g); break;
-    case 1: blas1_kernel<T, 1><<<g.nb, th, 0, st>>>(z, x, y, a, b, g); break;
-    case 2: blas1_kernel<T, 2><<<g.nb, th, 0, st>>>(z, x, y, a, b, g); break;
-    case 3: blas1_kernel<T, 3><<<g.nb, th, 0, st>>>(z, x, y, a, b, g); break;
-    default: blas1_kernel<T, 4><<<g.nb, th, 0, st>>>(z, x, y, a, b, g); break;
+    case 0: blas1_kernel<T, 0><<<grid, th, 0, st>>>(z, x, y, a, b, g, zc); break;
+    case 1: blas1_kernel<T, 1><<<grid, th, 0, st>>>(z, x, y, a, b, g, zc); break;
+    case 2: blas1_kernel<T, 2><<<grid, th, 0, st>>>(z, x, y, a, b, g, zc); break;
+    case 3: blas1_kernel<T, 3><<<grid, th, 0, st>>>(z, x, y, a, b, g, zc); break;
+    default: blas1_kernel<T, 4><<<grid, th, 0, st>>>(z, x, y, a, b, g, zc); break;
   }
   return cudaGetLastError();
 }
@@ -577,6 +653,7 @@ cudaError_t launch_accumulate_f32_into_f64(double* x, const float* d, const Geom
 }
 
 #define INST(T)                                                                              \
+  template cudaError_t launch_recip<T>(T*, const T*, const Geom&, cudaStream_t);            \
   template cudaError_t launch_jacobi<T>(T*, const T*, const T*, Op<T>, const Geom&, T,      \
                                         cudaStream_t);                                      \
   template cudaError_t launch_residual<T>(T*, const T*, const T*, Op<T>, const Geom&, int,  \
