@@ -592,6 +592,35 @@ __global__ void __launch_bounds__(kr_nt<N>(), (kr_minb<double, N, false>())) kr_
 }
 
 // ---------------------------------------------------------------------------
+// Both sums of blocks [f0, f1), valid in thread 0: each thread adds every
+// blockDim.x-th one in order, then the CTA's tree.  One CTA reads them all, so
+// the loads of eight rounds are issued before the first addition (4432 blocks:
+// 12.7 us with one round's).
+__device__ __forceinline__ void kr_segment_sums(const double* __restrict__ partial, int nb, int f0,
+                                                int f1, double* red, double& v0, double& v1) {
+  constexpr int U = 8;
+  const int bd = blockDim.x;
+  v0 = v1 = 0.0;
+  int q = f0 + threadIdx.x;
+  for (; q < f1; q += U * bd) {
+    double a[U], b[U];
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+      const bool in = q + u * bd < f1;
+      a[u] = in ? partial[q + u * bd] : 0.0;
+      b[u] = in ? partial[nb + q + u * bd] : 0.0;
+    }
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+      if (q + u * bd >= f1) break;
+      v0 = __dadd_rn(v0, a[u]);
+      v1 = __dadd_rn(v1, b[u]);
+    }
+  }
+  v0 = kr_block_sum(v0, red);
+  v1 = kr_block_sum(v1, red);
+}
+
 // Per segment: reduce its blocks' partial sums (fixed order), then one stage
 // of the scalar recurrence of ILS3D.h:663-844 in FP64.
 __global__ void __launch_bounds__(256) kr_scalar_kernel(const double* __restrict__ partial, int nb,
@@ -603,13 +632,8 @@ __global__ void __launch_bounds__(256) kr_scalar_kernel(const double* __restrict
   if (stage != KS_INIT && sg.status != kRunning) return;
   const int f0 = S.seg_first ? S.seg_first[sgi] : 0;
   const int f1 = S.seg_first ? S.seg_first[sgi + 1] : nb;
-  double v0 = 0.0, v1 = 0.0;
-  for (int q = f0 + threadIdx.x; q < f1; q += blockDim.x) {
-    v0 = __dadd_rn(v0, partial[q]);
-    v1 = __dadd_rn(v1, partial[nb + q]);
-  }
-  v0 = kr_block_sum(v0, red);
-  v1 = kr_block_sum(v1, red);
+  double v0, v1;
+  kr_segment_sums(partial, nb, f0, f1, red, v0, v1);
   if (threadIdx.x != 0) return;
   const double fmin = (double)FLT_MIN;
   if (stage == KS_INIT) {
@@ -701,13 +725,8 @@ __global__ void __launch_bounds__(256) kr_segsum_kernel(const double* __restrict
   const int sgi = blockIdx.x;
   const int f0 = S.seg_first ? S.seg_first[sgi] : 0;
   const int f1 = S.seg_first ? S.seg_first[sgi + 1] : nb;
-  double v0 = 0.0, v1 = 0.0;
-  for (int q = f0 + threadIdx.x; q < f1; q += blockDim.x) {
-    v0 = __dadd_rn(v0, partial[q]);
-    v1 = __dadd_rn(v1, partial[nb + q]);
-  }
-  v0 = kr_block_sum(v0, red);
-  v1 = kr_block_sum(v1, red);
+  double v0, v1;
+  kr_segment_sums(partial, nb, f0, f1, red, v0, v1);
   if (threadIdx.x == 0) {
     out[2 * sgi] = v0;
     out[2 * sgi + 1] = v1;
