@@ -104,6 +104,7 @@ struct bcmg_ctx_s {
   VcTask* d_out_tasks = nullptr;   // F2C entries by source block (pull form)
   int ghost_slots = 0;             // side-buffer slots (faces across a level change)
   bool pull_ok = true;             // every block feeds at most kMaxOutEntries of them
+  bool whole_faces = true;         // every fed face is fed over its whole area
   void* d_side[2] = {nullptr, nullptr};  // side buffers of first-layer ghosts
   size_t side_bytes = 0;
   size_t side_es = 0;                    // element size the side buffers are laid out for
@@ -298,6 +299,7 @@ static int build_face_table(bcmg_ctx c) {
   c->d_out_tasks = ft.out_tasks;
   c->ghost_slots = ft.ghost_slots;
   c->pull_ok = ft.pull_ok;
+  c->whole_faces = ft.whole_faces;
   c->open_faces = ft.open_faces;
   c->bc_conflict = ft.bc_conflict;
   c->has_neumann = ft.has_neumann;
@@ -387,6 +389,17 @@ static PushTable push_table(bcmg_ctx c, int seq) {
   unsigned char* s1 = static_cast<unsigned char*>(c->d_side[(seq + 1) & 1]);
   return PushTable{c->d_push_ptr, c->d_push_tasks, c->d_fed, c->d_facein, c->d_binfo,
                    c->d_out_tasks, s0, s1, s0 ? s0 + xo : nullptr, s1 ? s1 + xo : nullptr};
+}
+
+// The pull-form sweeps' other buffer before a run: the cells no launch writes
+// agree with x's.
+static int copy_frame(bcmg_ctx c, const Field& dst, const Field& src, bool rows, cudaStream_t st) {
+  const Geom g = geom_of(c, src);
+  if (src.dtype == BCMG_F64)
+    LAUNCH(c, K_FILL, st, launch_copy_frame<double>((double*)dst.d, (const double*)src.d, g, rows, st));
+  else
+    LAUNCH(c, K_FILL, st, launch_copy_frame<float>((float*)dst.d, (const float*)src.d, g, rows, st));
+  return BCMG_SUCCESS;
 }
 
 // ImposeBoundaryCondition: VC update of all faces, then Dirichlet ghosts.
@@ -1251,8 +1264,17 @@ BCMG_API int bcmg_sor_run(bcmg_ctx c, int fid, int sid, const double* coef, doub
       sd = pf->d;
     }
     // Cells no kernel writes (edges, corners, ghosts without a source) must
-    // agree between the two buffers: start from a copy.
-    CUDA_TRY(c, cudaMemcpyAsync(w->d, f->d, f->bytes, cudaMemcpyDeviceToDevice, stream));
+    // agree between the two buffers: start from a copy of them, which for the
+    // pull form are the ghost rows and planes (43 us for the whole field and 17
+    // for those on 4432 blocks of 16^3, FP32, vc = 2).
+    if (pulled) {
+      if ((rc = copy_frame(c, *w, *f, true, stream))) {
+        cudaFreeAsync(d_coef, stream);
+        return rc;
+      }
+    } else {
+      CUDA_TRY(c, cudaMemcpyAsync(w->d, f->d, f->bytes, cudaMemcpyDeviceToDevice, stream));
+    }
     Field* A = f;
     Field* B = w;
     for (int it = 0; it < n_outer; it++) {
@@ -1745,7 +1767,7 @@ struct PreArgs {
 static int jacobi_fused(bcmg_ctx c, const OpRec& o, const Field& x0, const Field& x1,
                         const Field& b, double omega, bool homogeneous, bool res, int seq,
                         int choice, cudaStream_t st, bool zero_x0 = false,
-                        const PreArgs* pre = nullptr) {
+                        const PreArgs* pre = nullptr, bool close = false) {
   Geom g = geom_of(c, x0);
   BlockBc bc{c->bctype.empty() ? nullptr : c->d_bctype,
              homogeneous ? c->d_bczero : c->d_bcval, c->bcform == BCMG_DIRICHLET_BCX ? 1 : 0,
@@ -1756,6 +1778,7 @@ static int jacobi_fused(bcmg_ctx c, const OpRec& o, const Field& x0, const Field
   }
   PushTable push = push_table(c, seq);
   const int mode = choice == kJacPush ? (zero_x0 ? kGhostPushZero : kGhostPush)
+                   : close ? (seq == 0 ? kGhostAsIsClose : kGhostPullClose)
                    : seq == 0 ? kGhostAsIs : kGhostPull;
   const int shape = choice == kJacPullPipe ? kJacobiPipe : kJacobiTile;
   double* part = res ? c->d_partial : nullptr;
@@ -1828,17 +1851,26 @@ BCMG_API int bcmg_jacobi_run(bcmg_ctx c, int op, int x, int b, double omega, int
   }
   const OpRec& o = c->ops[op];
   const int choice = jacobi_choice(c, *fx);
+  // the one-CTA-per-block pull form ends with a launch that writes the ghosts
+  const bool closes = choice == kJacPullTile && c->whole_faces;
   auto body = [&]() -> int {
-    // the work copy starts equal to x: cells no launch writes agree in both
-    CUDA_TRY(c, cudaMemcpyAsync(fw->d, fx->d, fx->bytes, cudaMemcpyDeviceToDevice, stream));
+    // cells no launch writes agree in x and its work copy: none in the push
+    // form (unless a face is fed in part), the ghost planes (and rows, in the
+    // pipelined kernel) in the pull form
+    if (choice != kJacPush) {
+      if (int r2 = copy_frame(c, *fw, *fx, choice == kJacPullPipe, stream)) return r2;
+    } else if (!c->whole_faces) {
+      CUDA_TRY(c, cudaMemcpyAsync(fw->d, fx->d, fx->bytes, cudaMemcpyDeviceToDevice, stream));
+    }
     Field* A = fx;
     Field* B = fw;
     for (int k = 0; k < iters; k++) {
-      int r2 = jacobi_fused(c, o, *A, *B, *fb, omega, false, false, k, choice, stream);
+      int r2 = jacobi_fused(c, o, *A, *B, *fb, omega, false, false, k, choice, stream, false,
+                            nullptr, closes && k == iters - 1);
       if (r2) return r2;
       std::swap(A, B);
     }
-    if (iters > 0) {
+    if (iters > 0 && !closes) {
       int r2 = finish_fused(c, *A, false, choice, stream);
       if (r2) return r2;
     }
@@ -1852,9 +1884,12 @@ BCMG_API int bcmg_jacobi_run(bcmg_ctx c, int op, int x, int b, double omega, int
   auto it = c->graphs.find(key);
   if (it == c->graphs.end()) {
     if (stream == 0) return fail(c, BCMG_USAGE, "graph capture needs a non-default stream");
-    // One eager launch first (into the work copy; x is untouched) so the
-    // kernel's one-time attribute setup happens outside the capture.
+    // Eager launches first (into the work copy; x is untouched) so the
+    // kernels' one-time attribute setup happens outside the capture.
     if ((rc = jacobi_fused(c, o, *fx, *fw, *fb, omega, false, false, 0, choice, stream)))
+      return rc;
+    if (closes && (rc = jacobi_fused(c, o, *fx, *fw, *fb, omega, false, false, 0, choice, stream,
+                                     false, nullptr, true)))
       return rc;
     CUDA_TRY(c, cudaStreamSynchronize(stream));
     CUDA_TRY(c, cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));

@@ -43,7 +43,11 @@ struct JacArgs {
 template <int N, int VC>
 __device__ __forceinline__ int shell_coord(int u) { return u < VC ? u - VC : N + u - VC; }
 
-template <typename T, int N, int VC, bool RES, bool PULL>
+// CLOSE (with PULL): a run's last launch, which leaves X1 with its ghosts
+// updated: the push form's writes instead of the side buffers, x-face layers
+// and stale ghost cells the next pull would read.  A closing ghost update of
+// its own took 399 us on 32768 blocks of 16^3 (FP32, vc = 1), a sweep 364.
+template <typename T, int N, int VC, bool RES, bool PULL, bool CLOSE = false>
 __global__ void __launch_bounds__(N * N, (BrickStage<T, N, VC, true>::MIN_BLOCKS))
     jacobi_tile_kernel(const T* __restrict__ X0, T* __restrict__ X1, const T* __restrict__ Bv,
                        Geom g, JacArgs<T> a) {
@@ -128,7 +132,7 @@ __global__ void __launch_bounds__(N * N, (BrickStage<T, N, VC, true>::MIN_BLOCKS
   int nout = 0;
   if (PULL) {
     nout = (flags >> BI_OUT_SHIFT) & 0x7f;
-    if (tid < nout) outs[tid] = a.push.out_tasks[inf.out_begin + tid];
+    if (!CLOSE && tid < nout) outs[tid] = a.push.out_tasks[inf.out_begin + tid];
     if (dmask && tid >= 32 && tid < 38) dv2f[tid - 32] = a.bc.v2f[(int64_t)b * 8 + tid - 32];
   }
   if (PULL && a.pull_now) {
@@ -229,7 +233,7 @@ __global__ void __launch_bounds__(N * N, (BrickStage<T, N, VC, true>::MIN_BLOCKS
     a.partial[b] = v;
   }
   T* fb = X1 + (int64_t)b * g.bstride;
-  if (PULL) {
+  if (PULL && !CLOSE) {
     // x1's x-face layers, for the same-level X neighbours of the next launch
     if (XF) {
       T* xo = static_cast<T*>(a.push.xf_out) + (int64_t)b * 2 * NN + tid;
@@ -268,13 +272,15 @@ __global__ void __launch_bounds__(N * N, (BrickStage<T, N, VC, true>::MIN_BLOCKS
   // layers of faces no neighbour feeds (Dirichlet ghosts where the boundary
   // prescribes them, sor1/Solver.cpp:232-294 and bcx.f90's second layer; x0's
   // values elsewhere).  Writing every such cell keeps each 32-byte sector of
-  // the brick whole in L2, so no partial sector costs a DRAM read-fill.
+  // the brick whole in L2, so no partial sector costs a DRAM read-fill.  CLOSE:
+  // the ghost planes in z are not staged, and X1's have held x0's values from
+  // the run's start.
   {
     constexpr int W = 2 * VC;
     constexpr int NA = W * W * LX;  // z and y outside: whole rows
     constexpr int NE = W * N * W;   // z outside, y inside, x outside
     constexpr int NC = N * W * W;   // z inside, y and x outside
-    for (int e = tid; e < NA + NE + NC; e += NT) {
+    for (int e = (CLOSE ? NA + NE : 0) + tid; e < NA + NE + NC; e += NT) {
       int x, y, z;
       if (e < NA) {
         x = e % LX - VC;
@@ -305,6 +311,7 @@ __global__ void __launch_bounds__(N * N, (BrickStage<T, N, VC, true>::MIN_BLOCKS
       if (a.bc.bcx) v = (double)(T)v;
       const double v2 = xmul(2.0, v);
       const int ax = fc >> 1;
+      if (CLOSE && ax == 2 && !dir) continue;
       const bool minus = (fc & 1) == 0;
       const bool second = a.bc.bcx && VC >= 2;
       for (int e = tid; e < VC * N * N; e += NT) {
@@ -314,6 +321,7 @@ __global__ void __launch_bounds__(N * N, (BrickStage<T, N, VC, true>::MIN_BLOCKS
         if (ax == 0) { gi = BL::at(l, p, q); ii = BL::at(l0, p, q); }
         else if (ax == 1) { gi = BL::at(p, l, q); ii = BL::at(p, l0, q); }
         else { gi = BL::at(p, q, l); ii = BL::at(p, q, l0); }
+        if (CLOSE && ax == 2 && u > (second ? 1 : 0)) continue;
         T val = xs[gi];
         if (dir && u == 0) val = to_t<T>(xsub(v2, (double)x1s[ii]));
         else if (dir && u == 1 && second) val = (T)v;
@@ -960,17 +968,18 @@ static cudaError_t jacobi_cubic_push_launch(const T* x0, T* x1, const T* b, cons
 
 template <typename T, int N, int VC>
 static cudaError_t jacobi_tile_launch(const T* x0, T* x1, const T* b, const Geom& g,
-                                      const JacArgs<T>& a, bool pull, cudaStream_t st) {
+                                      const JacArgs<T>& a, bool pull, bool close,
+                                      cudaStream_t st) {
   using L = BrickStage<T, N, VC, true>;
-  if (L::SMEM > kSorMaxSmem) return cudaErrorInvalidValue;
-  const int ki = (a.partial ? 1 : 0) + (pull ? 2 : 0);
+  if (L::SMEM > kSorMaxSmem || (close && (!pull || a.partial))) return cudaErrorInvalidValue;
+  const int ki = close ? 4 : (a.partial ? 1 : 0) + (pull ? 2 : 0);
   auto kern = ki == 0   ? jacobi_tile_kernel<T, N, VC, false, false>
               : ki == 1 ? jacobi_tile_kernel<T, N, VC, true, false>
               : ki == 2 ? jacobi_tile_kernel<T, N, VC, false, true>
-                        : jacobi_tile_kernel<T, N, VC, true, true>;
-  // set once per process (it is not a stream operation, and runs before any
-  // CUDA-graph capture of these launches)
-  static bool attr_set[4] = {false, false, false, false};
+              : ki == 3 ? jacobi_tile_kernel<T, N, VC, true, true>
+                        : jacobi_tile_kernel<T, N, VC, false, true, true>;
+  // set once per process (not a stream operation, allowed during a capture)
+  static bool attr_set[5] = {};
   if (!attr_set[ki]) {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)L::SMEM);
@@ -1036,6 +1045,7 @@ cudaError_t launch_jacobi_fused_impl(const T* x0, T* x1, const T* b, const Geom&
                      : jacobi_zero_push_launch<T, 8, 2>(x1, bw, g, a, st);
   }
   if (ghost_mode != kGhostPush && shape == kJacobiPipe) {
+    if (ghost_mode >= kGhostPullClose) return cudaErrorInvalidValue;
     if (!pipe_shape_ok((int)sizeof(T), g.nx, g.vc, true)) return cudaErrorInvalidValue;
     PipeArgs<T> p{cf, omega, (T)0, 0, bc, push.info, push.out_tasks,
                   static_cast<const T*>(push.side_in), static_cast<T*>(push.side_out),
@@ -1048,12 +1058,13 @@ cudaError_t launch_jacobi_fused_impl(const T* x0, T* x1, const T* b, const Geom&
                      : jacobi_pipe_launch<T, 8, 2>(x0, x1, b, g, p, st);
   }
   const bool pl = ghost_mode != kGhostPush;
-  JacArgs<T> a{ghost_mode == kGhostPull ? 1 : 0, cf, omega, bc, push, partial, err};
+  const bool close = ghost_mode == kGhostPullClose || ghost_mode == kGhostAsIsClose;
+  JacArgs<T> a{ghost_mode == kGhostPull || ghost_mode == kGhostPullClose ? 1 : 0, cf, omega, bc, push, partial, err};
   if (g.nx == 16)
-    return g.vc == 1 ? jacobi_tile_launch<T, 16, 1>(x0, x1, b, g, a, pl, st)
-                     : jacobi_tile_launch<T, 16, 2>(x0, x1, b, g, a, pl, st);
-  return g.vc == 1 ? jacobi_tile_launch<T, 8, 1>(x0, x1, b, g, a, pl, st)
-                   : jacobi_tile_launch<T, 8, 2>(x0, x1, b, g, a, pl, st);
+    return g.vc == 1 ? jacobi_tile_launch<T, 16, 1>(x0, x1, b, g, a, pl, close, st)
+                     : jacobi_tile_launch<T, 16, 2>(x0, x1, b, g, a, pl, close, st);
+  return g.vc == 1 ? jacobi_tile_launch<T, 8, 1>(x0, x1, b, g, a, pl, close, st)
+                   : jacobi_tile_launch<T, 8, 2>(x0, x1, b, g, a, pl, close, st);
 }
 
 }  // namespace bcmg

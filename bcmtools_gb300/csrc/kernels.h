@@ -174,7 +174,10 @@ cudaError_t launch_jacobi(T* x1, const T* x0, const T* b, Op<T> op, const Geom& 
 // launch of a run).
 // kGhostPushZero: the push form with x0 taken as zero everywhere (not read):
 // the first pass of a preconditioner from zero.
-enum : int { kGhostPush = 0, kGhostPull = 1, kGhostAsIs = 2, kGhostPushZero = 3 };
+// kGhostPullClose, kGhostAsIsClose: kGhostPull / kGhostAsIs (one CTA per block)
+// with x1 leaving as the push form leaves it, for a run's last launch.
+enum : int { kGhostPush = 0, kGhostPull = 1, kGhostAsIs = 2, kGhostPushZero = 3,
+             kGhostPullClose = 4, kGhostAsIsClose = 5 };
 // Kernel shapes of the pull-form Jacobi sweep: one CTA per block, or the
 // persistent double-buffered pipeline.
 enum : int { kJacobiTile = 1, kJacobiPipe = 2 };
@@ -266,6 +269,11 @@ cudaError_t launch_kr_seg_to32(float* r32, const double* r64, const Geom& g32, c
 cudaError_t launch_kr_seg_acc(double* x64, const float* d32, const Geom& g32, const Geom& g64,
                               const int* seg_of, const unsigned char* flag, const double* scale,
                               cudaStream_t st);
+
+// The cells of every brick that the pull-form sweeps never write, dst <- src:
+// the ghost planes in z and, with `rows`, the ghost rows in y of the others.
+template <typename T>
+cudaError_t launch_copy_frame(T* dst, const T* src, const Geom& g, bool rows, cudaStream_t st);
 
 template <typename T>
 cudaError_t launch_fill(T* x, int64_t n, T v, cudaStream_t st);

@@ -222,7 +222,8 @@ inline int blocks_for(int n, int t = 256) { return (n + t - 1) / t; }
 
 
 // ---- face tables (BlockManager::setFaceLists, BlockManager.cpp:63-114) -------
-enum : unsigned { FT_CONFLICT = 1, FT_NEUMANN = 2, FT_OPEN = 4, FT_PULL_BAD = 8 };
+// FT_PARTIAL: a face on finer blocks lacks some of its four (inactive leaves)
+enum : unsigned { FT_CONFLICT = 1, FT_NEUMANN = 2, FT_OPEN = 4, FT_PULL_BAD = 8, FT_PARTIAL = 16 };
 
 // Entries of face (b, f) per category: cnt[q * nbf + k], k = b*6+f, q = kind*3
 // + axis; has[ax * nbf + k] = 1 when the face takes F2C entries.
@@ -241,6 +242,7 @@ __global__ void ft_count(int nb, const int* __restrict__ ld, const int* __restri
     for (int s = 0; s < 4; s++) c += id[k * 4 + s] >= 0;
     cnt[(VC_F2C * 3 + ax) * nbf + k] = c;
     has[ax * nbf + k] = c > 0;
+    if (c > 0 && c < 4) atomicOr(flags, FT_PARTIAL);
   }
   if (bctype) {
     const bool neu = bctype[k] == BCMG_BC_NEUMANN;
@@ -466,6 +468,7 @@ cudaError_t build_face_tables(int nb, const int* ld, const int* id, const int* s
   out->has_neumann = (hf & FT_NEUMANN) != 0;
   out->open_faces = (hf & FT_OPEN) != 0;
   out->pull_ok = (hf & FT_PULL_BAD) == 0;
+  out->whole_faces = (hf & FT_PARTIAL) == 0;
   out->tasks = ntasks ? all.release() : nullptr;
   out->push_ptr = pptr.release();
   out->push_tasks = nnd ? push.release() : nullptr;

@@ -29,6 +29,7 @@ struct FaceTables {
   VcTask* out_tasks = nullptr;
   int ghost_slots = 0;
   bool pull_ok = true, open_faces = false, bc_conflict = false, has_neumann = false;
+  bool whole_faces = true;  // every fed face is fed over its whole area
 };
 
 // The face tables of nb blocks from the neighbour table (device arrays:

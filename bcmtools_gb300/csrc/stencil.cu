@@ -419,8 +419,16 @@ cudaError_t launch_dot_partial(const T* x, const T* y, const Geom& g, double* pa
 __global__ void __launch_bounds__(1024) reduce_final_kernel(const double* __restrict__ partial,
                                                             int n, double* __restrict__ out) {
   __shared__ double red[32];
+  constexpr int U = 8;  // loads of eight rounds before the first addition
   double acc = 0.0;
-  for (int i = threadIdx.x; i < n; i += blockDim.x) acc += partial[i];
+  for (int i = threadIdx.x; i < n; i += U * blockDim.x) {
+    double v[U];
+#pragma unroll
+    for (int u = 0; u < U; u++) v[u] = i + u * blockDim.x < n ? partial[i + u * blockDim.x] : 0.0;
+#pragma unroll
+    for (int u = 0; u < U; u++)
+      if (i + u * blockDim.x < n) acc += v[u];
+  }
   acc = block_sum(acc, red);
   if (threadIdx.x == 0) out[0] = acc;
 }
@@ -482,6 +490,37 @@ cudaError_t launch_blas1(int kind, T* z, const T* x, const T* y, T a, T b, const
     case 3: blas1_kernel<T, 3><<<grid, th, 0, st>>>(z, x, y, a, b, g, zc); break;
     default: blas1_kernel<T, 4><<<grid, th, 0, st>>>(z, x, y, a, b, g, zc); break;
   }
+  return cudaGetLastError();
+}
+
+// The ghost planes in z (and the ghost rows in y) of a brick: contiguous but for
+// the interior rows, one warp per piece.
+template <typename T>
+__global__ void __launch_bounds__(256) copy_frame_kernel(T* __restrict__ dst,
+                                                         const T* __restrict__ src, Geom g,
+                                                         int rows) {
+  const int64_t base = (int64_t)blockIdx.x * g.bstride;
+  T* d = dst + base;
+  const T* s = src + base;
+  const int ends = g.vc * g.sz;                // the ghost planes at either end
+  const int hi = (g.vc + g.nz) * g.sz;
+  for (int e = threadIdx.x; e < ends; e += blockDim.x) {
+    d[e] = s[e];
+    d[hi + e] = s[hi + e];
+  }
+  if (!rows) return;
+  const int n = g.vc * g.sy, up = (g.vc + g.ny) * g.sy;
+  for (int z = g.vc + (threadIdx.x >> 5); z < g.vc + g.nz; z += blockDim.x >> 5)
+    for (int e = threadIdx.x & 31; e < n; e += 32) {
+      d[z * g.sz + e] = s[z * g.sz + e];
+      d[z * g.sz + up + e] = s[z * g.sz + up + e];
+    }
+}
+
+template <typename T>
+cudaError_t launch_copy_frame(T* dst, const T* src, const Geom& g, bool rows, cudaStream_t st) {
+  if (g.nb == 0) return cudaSuccess;
+  copy_frame_kernel<T><<<g.nb, 256, 0, st>>>(dst, src, g, rows ? 1 : 0);
   return cudaGetLastError();
 }
 
@@ -653,6 +692,7 @@ cudaError_t launch_accumulate_f32_into_f64(double* x, const float* d, const Geom
 }
 
 #define INST(T)                                                                              \
+  template cudaError_t launch_copy_frame<T>(T*, const T*, const Geom&, bool, cudaStream_t); \
   template cudaError_t launch_recip<T>(T*, const T*, const Geom&, cudaStream_t);            \
   template cudaError_t launch_jacobi<T>(T*, const T*, const T*, Op<T>, const Geom&, T,      \
                                         cudaStream_t);                                      \
