@@ -1160,12 +1160,12 @@ static long sor_key(int dtype, int n, int vc, int form) {
 }
 
 // Kernel shape for a fused SOR sweep: forced, tuned, or the default -- the
-// pull form one CTA per block (7) where it applies, else the staged-source
+// pull form one CTA per block (7) where it applies (no face fed in part), else the staged-source
 // tile (1).  Push-only
 // contexts (bcmg_set_ghost_form) never get the pull form.
 static int sor_variant(bcmg_ctx c, const Field& f, int form) {
   const bool cubic = c->nx == c->ny && c->ny == c->nz;
-  const bool pull_ok = c->ghost_form != BCMG_GHOST_PUSH && cubic && sor_pull_ok((int)dsize(f.dtype), c->nx, f.vc, form);
+  const bool pull_ok = c->ghost_form != BCMG_GHOST_PUSH && cubic && c->whole_faces && sor_pull_ok((int)dsize(f.dtype), c->nx, f.vc, form);
   int v = c->sor_fixed;
   if (!v) {
     auto it = c->sor_tuned.find(sor_key(f.dtype, c->nx, f.vc, form));
@@ -1745,7 +1745,9 @@ static int converged(double rr, double bb, double eps, double* res) {
 enum { kJacPush = 1, kJacPullTile = 2, kJacPullPipe = 3 };
 static long jacobi_key(int dtype, int n, int vc) { return ((long)dtype * 64 + n) * 8 + vc; }
 static int jacobi_choice(bcmg_ctx c, const Field& x) {
-  if (c->nx == 32) return kJacPush;  // the only fused form of 32^3 blocks
+  // the only fused form of 32^3 blocks, and of faces fed in part: a side-buffer
+  // slot has no values for the quarters that no finer block feeds
+  if (c->nx == 32 || !c->whole_faces) return kJacPush;
   if (c->jacobi_force) return c->jacobi_force;
   if (c->ghost_form == BCMG_GHOST_PUSH) return kJacPush;
   if (c->jacobi_shape) return c->jacobi_shape == kJacobiPipe ? kJacPullPipe : kJacPullTile;

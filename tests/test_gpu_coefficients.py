@@ -106,3 +106,46 @@ def test_bicgstab_f64_agrees(gpu_ok, n, vc, cells):
     inner = (slice(None),) + (slice(vc, -vc),) * 3
     g, r = X.download()[inner], ref[inner]
     assert np.linalg.norm(g - r) <= 1e-12 * np.linalg.norm(r), cells
+
+
+def with_a_hole():
+    """Two levels with one fine leaf left out: a coarse face fed by three of
+    its four quarters, whose other ghosts no launch writes."""
+    full = small_octree(periodic=(False, False, False), level=2, radius=0.3)
+    ld, nid, _, _ = full.neighbors()
+    b, f = np.argwhere(ld == 1)[0]
+    peds = np.delete(full.pedigrees, nid[b, f, 2])
+    return bg.Octree.from_pedigrees(full.rootgrid, peds)
+
+
+@pytest.mark.parametrize("dt", ["f32", "f64"])
+@pytest.mark.parametrize("n,vc", [(8, 2), (16, 1), (32, 1)])
+@pytest.mark.parametrize("iters", [1, 2, 5])
+@pytest.mark.parametrize("push", [True, False])
+def test_jacobi_run_with_a_face_fed_in_part(gpu_ok, dt, n, vc, iters, push):
+    tree = with_a_hole()
+    bm = bg.BlockManager(0)
+    bm.register_octree(tree, n)
+    ld, nid, sf, outer = tree.neighbors()
+    assert ((nid[ld == 1] < 0).any(axis=1) & (nid[ld == 1] >= 0).any(axis=1)).any()
+    m = po.OracleMesh(ld, nid, sf, n, vc)
+    bct, bcv = outer_dirichlet(tree, 0.25)
+    bm.set_boundary(bct, bcv, bg.DIRICHLET_SOR)
+    bm.set_ghost_form(push=push)
+    x, b = bm.setDataClass(dt, vc), bm.setDataClass(dt, vc)
+    rng = np.random.default_rng(8)
+    a0 = rng.uniform(-1, 1, size=x.shape).astype(x.dtype)
+    ab = np.zeros_like(a0)
+    inner = (slice(None),) + (slice(vc, -vc),) * 3
+    ab[inner] = rng.uniform(-1, 1, size=ab[inner].shape)
+    x.upload(a0)
+    b.upload(ab)
+    cc = bg.laplace_coef(tree.cell_sizes(n))
+    bm.jacobi_run(bm.op_const(cc), x, b, 0.9, iters)
+    ref, x1 = a0.copy(), np.zeros_like(a0)
+    for _ in range(iters):
+        m.jacobi(x1, ref, ab, 0.9, cc=cc)
+        ref[inner] = x1[inner]
+        m.vc_update(ref)
+        m.dirichlet(ref, bct, bcv, 0)
+    assert_bitexact(x.download(), ref, face_mask(n, vc), f"partly fed {dt} {n} {iters}")
