@@ -1226,12 +1226,24 @@ BCMG_API int bcmg_sor_run(bcmg_ctx c, int fid, int sid, const double* coef, doub
   // Fused ping-pong path: one launch per outer iteration writes the next
   // iterate with every ghost updated.  It needs the block's Dirichlet ghosts
   // to be the only writers of their cells (no Dirichlet face with a
-  // neighbour), at least one inner pass, and a brick that fits shared memory.
-  const bool fused = n_inner >= 1 && !c->bc_conflict && smem <= kSorMaxSmem && !c->no_fusion;
+  // neighbour), at least one inner pass, and a brick that fits shared memory
+  // or, with one inner pass, planes that stream through it.
+  const bool streams = smem > kSorMaxSmem && sor_streams(g, form == 2, n_inner, es);
+  bool fused = n_inner >= 1 && !c->bc_conflict && (smem <= kSorMaxSmem || streams) && !c->no_fusion;
   int rc = BCMG_SUCCESS;
+  int wid, pid = -1;
+  if (fused && n_outer > 0 && (rc = work_field(c, f->dtype, f->vc, 30, &wid))) {
+    // no room for a second buffer: a streamed shape is swept in place
+    if (!(streams && rc == BCMG_MEMORY)) {
+      cudaFreeAsync(d_coef, stream);
+      return rc;
+    }
+    fused = false;
+    rc = BCMG_SUCCESS;
+    f = get_field(c, fid);
+    s = form == 2 ? get_field(c, sid) : nullptr;
+  }
   if (fused && n_outer > 0) {
-    int wid, pid = -1;
-    if ((rc = work_field(c, f->dtype, f->vc, 30, &wid))) { cudaFreeAsync(d_coef, stream); return rc; }
     // Runs of the pull-form kernels with a source term and enough iterations
     // read the source packed N^3 per block in sweep order (no padding, one
     // bulk copy per block): packed once here, it saves the padding's bytes
@@ -1265,9 +1277,12 @@ BCMG_API int bcmg_sor_run(bcmg_ctx c, int fid, int sid, const double* coef, doub
     }
     // Cells no kernel writes (edges, corners, ghosts without a source) must
     // agree between the two buffers: start from a copy of them, which for the
-    // pull form are the ghost rows and planes (43 us for the whole field and 17
-    // for those on 4432 blocks of 16^3, FP32, vc = 2).
-    if (pulled) {
+    // pull form, and for the push form where every ghost layer is written, are
+    // in the ghost rows and planes (43 us for the whole field and 17 for those
+    // on 4432 blocks of 16^3, FP32, vc = 2).
+    const bool all_layers = !c->open_faces && c->whole_faces &&
+                            (f->vc == 1 || (f->vc == 2 && c->bcform == BCMG_DIRICHLET_BCX));
+    if (pulled || all_layers) {
       if ((rc = copy_frame(c, *w, *f, true, stream))) {
         cudaFreeAsync(d_coef, stream);
         return rc;

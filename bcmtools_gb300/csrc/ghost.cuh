@@ -212,18 +212,29 @@ __device__ __forceinline__ void task_apply(const VcTask& t, T* __restrict__ dst,
   const Box B = task_box(t, g);
   const int cnt = B.b[0] * B.b[1] * B.b[2];
   const int bxy = B.b[0] * B.b[1];
+  // cell `lane` of the box, and the step to the worker's next cell: one
+  // division each, not one a cell (box extents are any even numbers)
+  int i, j, k, di, dj, dk, rem;
+  divmod(lane, bxy, k, rem);
+  divmod(rem, B.b[0], j, i);
+  divmod(nl, bxy, dk, rem);
+  divmod(rem, B.b[0], dj, di);
+  const auto step = [&] {
+    i += di;
+    j += dj;
+    k += dk;
+    if (i >= B.b[0]) { i -= B.b[0]; j++; }
+    if (j >= B.b[1]) { j -= B.b[1]; k++; }
+  };
   for (int e0 = lane; e0 < cnt; e0 += U * nl) {
     T vals[U], second[U];
     int at[U], at2[U];
 #pragma unroll
-    for (int q = 0; q < U; q++) {
+    for (int q = 0; q < U; q++, step()) {
       const int e = e0 + q * nl;
       at[q] = -1;
       at2[q] = -1;
       if (e >= cnt) continue;
-      int k, r, j, i;
-      divmod(e, bxy, k, r);
-      divmod(r, B.b[0], j, i);
       at[q] = TOBUF ? e : g.at(B.d[0] + i, B.d[1] + j, B.d[2] + k);
       if (t.kind == VC_COPY) {
         vals[q] = *src.at(B.o[0] + i, B.o[1] + j, B.o[2] + k);

@@ -9,6 +9,19 @@
 
 namespace bcmg {
 
+// log2 of the lanes that share one face-table entry in the kernels for any block
+// shape: a warp, or for small blocks the power of two that holds the largest
+// ghost box (vc cells by the largest face), so that a warp takes several
+// entries.  With a warp each, 2^3 blocks left 28 of 32 lanes idle in every FP64
+// instruction (8.0 us an iteration of 456 such blocks).
+__host__ __device__ inline int entry_shift(const Geom& g) {
+  const int xy = g.nx * g.ny, yz = g.ny * g.nz, xz = g.nx * g.nz;
+  const int most = g.vc * (xy > yz ? (xy > xz ? xy : xz) : (yz > xz ? yz : xz));
+  int l = 5;
+  while (l > 0 && (1 << (l - 1)) >= most) l--;
+  return l;
+}
+
 // Up to 12 contiguous slices of the face table (4 kinds x 3 axes) selected
 // by one launch; prefix[q] is the first warp of slice q.
 struct VcRanges {
@@ -83,11 +96,53 @@ constexpr size_t kSorMaxSmem = 200 * 1024;
 // Dynamic shared memory one CTA may use (227 KB on sm_100-class GPUs).
 constexpr size_t kPipeMaxSmem = 227 * 1024;
 
+// Ring of the streamed red-black SOR pass (sor_stream.cuh): one unit holds rows
+// [-1, ny] of a plane and, with a source, the source's rows [0, ny), each
+// widened to 16-byte bounds.
+struct SorRing {
+  int xlo, xbytes;  // first byte and bytes of the rows of a brick plane
+  int slo, sbytes;
+  int slot, slots;  // bytes of a unit, units in shared memory
+  int threads;      // of the CTA
+  static SorRing make(const Geom& g, bool src, size_t es) {
+    SorRing r;
+    const int row = g.sy * (int)es;
+    r.xlo = (g.vc - 1) * row / 16 * 16;
+    r.xbytes = ((g.vc + g.ny + 1) * row + 15) / 16 * 16 - r.xlo;
+    r.slo = g.vc * row / 16 * 16;
+    r.sbytes = src ? ((g.vc + g.ny) * row + 15) / 16 * 16 - r.slo : 0;
+    r.slot = r.xbytes + r.sbytes;
+    // Planes of at most 128 cell pairs take 128 threads and a ring of eight per
+    // SM, larger ones 256 and four per SM; six slots at least (one in flight)
+    r.threads = g.nx / 2 * g.ny <= 128 ? 128 : 256;
+    const int fit = (r.threads == 128 ? 27 : 55) * 1024 / r.slot;
+    r.slots = fit < 6 ? 6 : fit > 16 ? 16 : fit;
+    if (r.slots > g.nz + 2 && g.nz + 2 >= 6) r.slots = g.nz + 2;
+    return r;
+  }
+  size_t bytes() const { return 128 + (size_t)slots * slot; }
+};
+// Whether that pass covers a run: one inner pass, whole 16-byte planes, a ring
+// within shared memory.  FP64 blocks of up to 256 cells stay staged whole (575
+// blocks of 4^3: 17.9 us an iteration, streamed 20.1), and bricks too large for
+// that are swept in place unless the rounds of 256 threads over a plane are
+// nearly full (28^3: 410 us in place, 462 streamed at 77 %; 32^3: 617 and 478).
+inline bool sor_streams(const Geom& g, bool src, int n_inner, size_t es) {
+  const SorRing r = SorRing::make(g, src, es);
+  if (n_inner != 1 || (g.sz * es) % 16 != 0 || r.bytes() > kSorMaxSmem) return false;
+  if (es == 4) return true;
+  const int np = g.nx / 2 * g.ny, rounds = (np + r.threads - 1) / r.threads;
+  const size_t whole = (size_t)(g.nx + 2) * (g.ny + 2) * (g.nz + 2) * es;
+  return g.nx * g.ny * g.nz > 256 &&
+         (whole <= kSorMaxSmem || 10 * np >= 9 * rounds * r.threads);
+}
+
 // Kernel shapes of the fused sweep, chosen per (dtype, N, VC, scheme) by the
 // autotuner (bcmg_autotune_sor) or fixed with bcmg_set_sor_variant.
 enum SorVariant : int {
   SV_AUTO = 0,       // tuned choice if any, else SV_TILE_SS_256
   SV_TILE_SS_256 = 1,  // one CTA per block, source staged in shared memory
+                       // (32^3: the planes streamed through it, sor_stream.cuh)
   SV_TILE_GS_256 = 2,  // one CTA per block, source read from global (L1)
   SV_TILE_SS_512 = 3,
   SV_TILE_GS_512 = 4,

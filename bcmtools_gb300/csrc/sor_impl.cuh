@@ -60,6 +60,16 @@ template <typename T, int N>
 cudaError_t launch_sor_tile(const T* A, T* B, const T* s, const Geom& g, const SorArgs& a,
                             bool push, int variant, cudaStream_t st);
 
+__device__ __forceinline__ unsigned dirichlet_mask(const SorArgs& a, int b) {
+  unsigned m = 0;
+  if (a.bc.type) {
+#pragma unroll
+    for (int fc = 0; fc < 6; fc++)
+      if (a.bc.type[b * 6 + fc] == kBcDirichlet) m |= 1u << fc;
+  }
+  return m;
+}
+
 // SMEM: stage (n+2)^3 in shared memory; otherwise sweep in place in global
 // memory (bricks too large for shared memory).  PUSH requires SMEM.
 template <typename T, int FORM, bool SMEM, bool PUSH>
@@ -73,6 +83,23 @@ __global__ void __launch_bounds__(512) sor_kernel(const T* A, T* Bf,
   const T* __restrict__ sbk = (FORM == 2) ? s + (int64_t)b * g.bstride : nullptr;
   const int nx = g.nx, ny = g.ny, nz = g.nz;
   const int lx = nx + 2, ly = ny + 2, lz = nz + 2;
+  // block constants, loaded before the staging is waited for
+  SorCell<T, FORM> cell;
+  cell.init(a, b);
+  const unsigned dmask = dirichlet_mask(a, b);
+  const bool anyd = dmask != 0;
+  bool dir[6];
+  double dv[6];
+#pragma unroll
+  for (int fc = 0; fc < 6; fc++) {
+    dir[fc] = (dmask >> fc) & 1;
+    dv[fc] = a.bc.value[b * 6 + fc];
+    if (a.bc.bcx) dv[fc] = (double)(T)dv[fc];
+  }
+  const int es = PUSH ? entry_shift(g) : 5;
+  const int p0 = PUSH ? a.push.ptr[b] + (tid >> es) : 0, p1 = PUSH ? a.push.ptr[b + 1] : 0;
+  VcTask first{};  // this thread's first ghost entry
+  if (p0 < p1) first = a.push.tasks[p0];
   T* base;
   int sy, sz, o;
   if (SMEM) {
@@ -88,19 +115,6 @@ __global__ void __launch_bounds__(512) sor_kernel(const T* A, T* Bf,
     __syncthreads();
   } else {
     base = fb; sy = g.sy; sz = g.sz; o = g.off0;
-  }
-  SorCell<T, FORM> cell;
-  cell.init(a, b);
-
-  bool dir[6];
-  double dv[6];
-  bool anyd = false;
-  for (int fc = 0; fc < 6; fc++) {
-    dir[fc] = a.bc.type && a.bc.type[b * 6 + fc] == kBcDirichlet;
-    double v = dir[fc] ? a.bc.value[b * 6 + fc] : 0.0;
-    if (a.bc.bcx) v = (double)(T)v;
-    dv[fc] = v;
-    anyd |= dir[fc];
   }
 
   // Fixed per-thread (i2, j, k0) when a whole number of k-slices fits the CTA.
@@ -210,10 +224,10 @@ __global__ void __launch_bounds__(512) sor_kernel(const T* A, T* Bf,
   if (PUSH) {
     // Ghost values this block's interior feeds, straight from shared memory.
     const Acc<T> src{base, sy, sz, o};
-    const int p0 = a.push.ptr[b], p1 = a.push.ptr[b + 1];
-    for (int q = p0 + warp; q < p1; q += nw) {
-      const VcTask t = a.push.tasks[q];
-      task_apply<T>(t, Bf + (int64_t)t.dst * g.bstride, g, src, 0.0, lane, 32);
+    for (int q = p0; q < p1; q += nt >> es) {
+      const VcTask t = q == p0 ? first : a.push.tasks[q];
+      task_apply<T>(t, Bf + (int64_t)t.dst * g.bstride, g, src, 0.0, tid & ((1 << es) - 1),
+                    1 << es);
     }
   }
 }
@@ -268,16 +282,6 @@ __device__ __forceinline__ void emit_block(const T* sf, T* fb, T* Bf, const Geom
       push_dispatch<T, N, VC>(t, Bf + (int64_t)t.dst * g.bstride, g, sf, lane);
     }
   }
-}
-
-__device__ __forceinline__ unsigned dirichlet_mask(const SorArgs& a, int b) {
-  unsigned m = 0;
-  if (a.bc.type) {
-#pragma unroll
-    for (int fc = 0; fc < 6; fc++)
-      if (a.bc.type[b * 6 + fc] == kBcDirichlet) m |= 1u << fc;
-  }
-  return m;
 }
 
 // One CTA per block: staging with vector loads, then sweep and emit.
@@ -529,6 +533,10 @@ static bool tile_ok(const Geom& g) {
   return f <= kSorMaxSmem;
 }
 
+}  // namespace bcmg
+#include "sor_stream.cuh"
+namespace bcmg {
+
 static int sor_threads(const Geom& g) {
   const int slice = (g.nx / 2) * g.ny;
   if (slice <= 256) return 256;
@@ -580,6 +588,13 @@ cudaError_t launch_sor_impl(const T* A, T* B, const T* s, const Geom& g, const d
                       : launch_sor_pull<T, 8>(A, B, sp, g, a, stages, st);
   }
   if (variant == SV_PULL || variant == SV_PULL_TILE) variant = SV_AUTO;
+  // 32^3 blocks (their default and staged-source shape) and blocks of no
+  // special shape
+  const bool staged = variant == SV_AUTO || variant == SV_TILE_SS_256;
+  if (fused && (!tile_ok<T>(g) || (g.nx == 32 && staged)) &&
+      sor_stream_ok<T>(g, A, form == 2 ? s : nullptr, n_inner))
+    return form == 1 ? launch_sor_stream<T, 1>(A, B, s, g, a, st)
+                     : launch_sor_stream<T, 2>(A, B, s, g, a, st);
   if (tile_ok<T>(g)) {
     const T* sp = form == 2 ? s : nullptr;
     if (g.nx == 16) return launch_sor_tile<T, 16>(A, B, sp, g, a, fused, variant, st);

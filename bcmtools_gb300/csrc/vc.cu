@@ -8,8 +8,9 @@
 // SolverTest/bcx.f90:18-76).  Every read is an interior cell and every write a
 // ghost cell, so entries are independent and run concurrently.
 //
-// Work decomposition: one warp per face-table entry, lanes walking the entry's
-// ghost box x-fastest (coalesced along rows for Y and Z faces).
+// Work decomposition: one warp per face-table entry (small blocks: a part of
+// one, entry_shift), lanes walking the entry's ghost box x-fastest (coalesced
+// along rows for Y and Z faces).
 #include "ghost.cuh"
 #include "kernels.h"
 #include "tile.cuh"
@@ -19,8 +20,9 @@ namespace bcmg {
 template <typename T>
 __global__ void __launch_bounds__(256) vc_gather_kernel(T* __restrict__ data, Geom g,
                                                         VcTable tab, VcRanges rg) {
-  const int w = (int)((blockIdx.x * (unsigned)blockDim.x + threadIdx.x) >> 5);
-  const int lane = threadIdx.x & 31;
+  const int es = entry_shift(g);
+  const int w = (int)((blockIdx.x * (unsigned)blockDim.x + threadIdx.x) >> es);
+  const int lane = threadIdx.x & ((1 << es) - 1);
   if (w >= rg.prefix[rg.n]) return;
   int q = 0;
   while (w >= rg.prefix[q + 1]) q++;
@@ -29,7 +31,7 @@ __global__ void __launch_bounds__(256) vc_gather_kernel(T* __restrict__ data, Ge
   const int sb = t.kind == VC_DIRICHLET ? t.dst : t.src;
   const Acc<T> src{data + (int64_t)sb * g.bstride, g.sy, g.sz, g.off0};
   const double bcv = t.kind == VC_DIRICHLET ? tab.bcval[t.dst * 6 + t.face] : 0.0;
-  task_apply<T>(t, dst, g, src, bcv, lane, 32);
+  task_apply<T>(t, dst, g, src, bcv, lane, 1 << es);
 }
 
 // Cubic 8^3 / 16^3 / 32^3 blocks with vc <= 2: the same entries with the
@@ -86,7 +88,11 @@ cudaError_t launch_vc_gather(T* data, const Geom& g, const VcTable& tab, const V
     case 16 * 4 + 2: vc_gather_cubic_kernel<T, 16, 2><<<grid, 256, 0, st>>>(data, g, tab, rg); break;
     case 32 * 4 + 1: vc_gather_cubic_kernel<T, 32, 1><<<grid, 256, 0, st>>>(data, g, tab, rg); break;
     case 32 * 4 + 2: vc_gather_cubic_kernel<T, 32, 2><<<grid, 256, 0, st>>>(data, g, tab, rg); break;
-    default: vc_gather_kernel<T><<<grid, 32 * warps_per_cta, 0, st>>>(data, g, tab, rg); break;
+    default: {
+      const int per = 256 >> entry_shift(g);
+      vc_gather_kernel<T><<<(nw + per - 1) / per, 256, 0, st>>>(data, g, tab, rg);
+      break;
+    }
   }
   return cudaGetLastError();
 }
