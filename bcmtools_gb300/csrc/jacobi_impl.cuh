@@ -492,6 +492,7 @@ __global__ void __launch_bounds__(N * N, (N == 8 ? 12 : sizeof(T) == 4 ? (VC == 
       if (PRE == kPreP) r = xadd(r, xmul(s_beta, xadd(pv[u], xmul(s_ng, qv[u]))));  // kr_p
       if (PRE == kPreS) r = xadd(xmul(s_na, qv[u]), r);                             // kr_s
       if (PRE != kPreNone) bp[(k0 + u) * LXY] = r;
+      if (PRE == kPreS || PRE == kPreCopy) row_ends(bp + (k0 + u) * LXY, tid % N, N, VC);
       const T v = positive_zero(xmul(om, sweep_div(r, c0, rc0)));
       xp[(k0 + u) * LXY] = v;
       x1s[(k0 + u) * NT + tid] = v;
@@ -784,6 +785,7 @@ __global__ void __launch_bounds__(NT_, (JacStream<T, N, VC, S, RES, ZERO, NT_, P
     else if (PRE == kPreS)  // kr_s: s = r - alpha q
       r = xadd(xmul(s_na, ring.cp(m, NB - 1)[q]), r);
     if (PRE != 0) bout[q] = r;  // kPreCopy, the first iteration: p = r
+    if (PRE == kPreS || PRE == kPreCopy) row_ends(bout + q, i0, N, VC);
     return r;
   };
   bool ok;
@@ -864,9 +866,11 @@ __global__ void __launch_bounds__(NT_, (JacStream<T, N, VC, S, RES, ZERO, NT_, P
           } else if (PRE == kPreS) {  // kr_s: s = r - alpha q
             r = xadd(xmul(s_na, ring.cp(m, NB - 1)[q]), bp[q]);
             bout[q] = r;
+            row_ends(bout + q, i0, N, VC);
           } else if (PRE == kPreCopy) {  // the first iteration: p = r
             r = bp[q];
             bout[q] = r;
+            row_ends(bout + q, i0, N, VC);
           } else {
             r = bp[q];
           }

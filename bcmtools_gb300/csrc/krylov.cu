@@ -4,7 +4,7 @@
 // (i, j) column each, the k walk unrolled so that a thread has several
 // planes' loads in flight; other block shapes loop over the columns.
 // Inner products: FP64 multiply-add per element along the column, then the
-// CTA's fixed-order tree (kr_block_sum); partial sums per block go to
+// CTA's fixed-order tree (kr_block_sums); partial sums per block go to
 // partial[slot * nb + b] and kr_scalar reduces them per segment.
 #include <cfloat>
 #include <type_traits>
@@ -86,7 +86,7 @@ template <typename T, int N, bool CC, int NDOT>
 __global__ void __launch_bounds__(kr_nt<N>(), (CC ? kr_minb<T, N, true>() : 768 / kr_nt<N>())) kr_ax_kernel(
     T* __restrict__ out, const T* __restrict__ x, const T* __restrict__ cf8, Op<T> op,
     const T* __restrict__ y0, Geom g, KSegs S, double* __restrict__ partial) {
-  __shared__ double red[32];
+  __shared__ double red[NDOT * kr_nt<N>()];
   const int b = blockIdx.x;
   if (S.seg[kseg_of(S, b)].status != kRunning) return;
   T c[7];
@@ -131,8 +131,8 @@ __global__ void __launch_bounds__(kr_nt<N>(), (CC ? kr_minb<T, N, true>() : 768 
       if (NDOT == 2) a1.add(a, a);
     }
   });
-  const double v0 = kr_block_sum(a0.value(), red);
-  const double v1 = NDOT == 2 ? kr_block_sum(a1.value(), red) : 0.0;
+  double v0 = a0.value(), v1 = NDOT == 2 ? a1.value() : 0.0;
+  kr_block_sums<NDOT>(v0, v1, red);
   if (threadIdx.x == 0) {
     partial[b] = v0;
     if (NDOT == 2) partial[g.nb + b] = v1;
@@ -160,8 +160,8 @@ __device__ __forceinline__ void kr_ax_finish(bool ok, const DotAcc<T>& a0, const
                                              double* red, double* __restrict__ partial, int b,
                                              int nb) {
   const double nan = __longlong_as_double(0x7ff8000000000000ll);
-  const double v0 = kr_block_sum(ok ? a0.value() : nan, red);
-  const double v1 = NDOT == 2 ? kr_block_sum(ok ? a1.value() : nan, red) : 0.0;
+  double v0 = ok ? a0.value() : nan, v1 = NDOT == 2 && ok ? a1.value() : nan;
+  kr_block_sums<NDOT>(v0, v1, red);
   if (threadIdx.x == 0) {
     partial[b] = v0;
     if (NDOT == 2) partial[nb + b] = v1;
@@ -177,7 +177,8 @@ __global__ void __launch_bounds__(NT_, (AxStream<T, N, VC, S, NT_>::MINB)) kr_ax
   constexpr int NT = AS::NT, CPT = N * N / NT, LX = R::LX, LXY = R::LXY;
   static_assert(N * N % NT == 0, "whole planes per CTA");
   extern __shared__ __align__(128) unsigned char smraw[];
-  __shared__ double red[32];
+  double* red = reinterpret_cast<double*>(smraw + R::BAR_BYTES);  // the ring, after the walk
+  static_assert(AS::SMEM >= R::BAR_BYTES + 2 * NT * sizeof(double), "room for the sums");
   const int b = blockIdx.x, tid = threadIdx.x;
   if (S_.seg[kseg_of(S_, b)].status != kRunning) return;
   const int64_t base = (int64_t)b * g.bstride;
@@ -303,7 +304,8 @@ __global__ void __launch_bounds__(256, (XrStream<T, N, VC, S>::MINB)) kr_xr_stre
   using R = typename XS::R;
   constexpr int NT = XS::NT, CPT = N * N / NT, LXY = R::LXY;
   extern __shared__ __align__(128) unsigned char smraw[];
-  __shared__ double red[32];
+  double* red = reinterpret_cast<double*>(smraw + R::BAR_BYTES);  // the ring, after the walk
+  static_assert(XS::SMEM >= R::BAR_BYTES + 2 * NT * sizeof(double), "room for the sums");
   const int b = blockIdx.x, tid = threadIdx.x;
   const KSeg& sg = S_.seg[kseg_of(S_, b)];
   if (sg.status != kRunning) return;
@@ -339,8 +341,8 @@ __global__ void __launch_bounds__(256, (XrStream<T, N, VC, S>::MINB)) kr_xr_stre
     }
   });
   const double nan = __longlong_as_double(0x7ff8000000000000ll);
-  const double v0 = kr_block_sum(ok ? a0.value() : nan, red);
-  const double v1 = kr_block_sum(ok ? a1.value() : nan, red);
+  double v0 = ok ? a0.value() : nan, v1 = ok ? a1.value() : nan;
+  kr_block_sums<2>(v0, v1, red);
   if (tid == 0) {
     partial[b] = v0;
     partial[g.nb + b] = v1;
@@ -377,7 +379,7 @@ __global__ void __launch_bounds__(kr_nt<N>(), (kr_minb<T, N, true>())) kr_xr_ker
     T* __restrict__ x, T* __restrict__ r, const T* __restrict__ p_, const T* __restrict__ s_,
     const T* __restrict__ s, const T* __restrict__ t, const T* __restrict__ r0, Geom g, KSegs S,
     double* __restrict__ partial) {
-  __shared__ double red[32];
+  __shared__ double red[2 * kr_nt<N>()];
   const int b = blockIdx.x;
   const KSeg& sg = S.seg[kseg_of(S, b)];
   if (sg.status != kRunning) return;
@@ -406,8 +408,8 @@ __global__ void __launch_bounds__(kr_nt<N>(), (kr_minb<T, N, true>())) kr_xr_ker
       a1.add(rv, r0v[v]);
     }
   });
-  const double v0 = kr_block_sum(a0.value(), red);
-  const double v1 = kr_block_sum(a1.value(), red);
+  double v0 = a0.value(), v1 = a1.value();
+  kr_block_sums<2>(v0, v1, red);
   if (threadIdx.x == 0) {
     partial[b] = v0;
     partial[g.nb + b] = v1;
@@ -420,7 +422,7 @@ template <typename T, int N>
 __global__ void __launch_bounds__(kr_nt<N>(), (kr_minb<T, N, true>())) kr_dot2_kernel(
     const T* __restrict__ x, const T* __restrict__ y, const T* __restrict__ u,
     const T* __restrict__ v, Geom g, double* __restrict__ partial) {
-  __shared__ double red[32];
+  __shared__ double red[2 * kr_nt<N>()];
   DotAcc<T> a0, a1;
   kr_walk<N, (sizeof(T) == 4 && N != 32 ? 4 : 2)>(g, [&](int64_t o0, auto vt) {
     constexpr int V = decltype(vt)::value;
@@ -439,8 +441,8 @@ __global__ void __launch_bounds__(kr_nt<N>(), (kr_minb<T, N, true>())) kr_dot2_k
       a1.add(uv[k], vv[k]);
     }
   });
-  const double v0 = kr_block_sum(a0.value(), red);
-  const double v1 = kr_block_sum(a1.value(), red);
+  double v0 = a0.value(), v1 = a1.value();
+  kr_block_sums<2>(v0, v1, red);
   if (threadIdx.x == 0) {
     partial[blockIdx.x] = v0;
     partial[g.nb + blockIdx.x] = v1;
@@ -505,6 +507,7 @@ __global__ void __launch_bounds__(256) kr_zero_pass_kernel(T* __restrict__ x1, T
         if (PRE == kPreP) r = xadd(r, xmul(beta, xadd(pv[v], xmul(ng, qv[v]))));  // kr_p
         if (PRE == kPreS) r = xadd(xmul(na, qv[v]), r);                           // kr_s
         if (PRE != kPreNone) b[o] = r;
+        if (PRE == kPreS || PRE == kPreCopy) row_ends(b + o, ij % nx, nx, g.vc);
         x1[o] = positive_zero(xmul(om, CC ? sweep_div(r, c0, rc0) : field_div(r, av[v], yv[v])));
       }
       o0 += (int64_t)V * g.sz;

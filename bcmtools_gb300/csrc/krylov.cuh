@@ -103,7 +103,16 @@ struct DotAcc<float> {
     }
   }
   __device__ __forceinline__ double value() const {
-    return __dadd_rn(__dadd_rn((double)s, (double)c), wide);
+    const double v = __dadd_rn(widen(s), widen(c));
+    return (__double_as_longlong(wide) << 1) == 0 ? v : __dadd_rn(v, wide);
+  }
+  // (double)f on the integer pipe (normal values and zeros): the conversion
+  // issues at the FP64 rate.
+  static __device__ __forceinline__ double widen(float f) {
+    const unsigned u = __float_as_uint(f), m = u & 0x7fffffffu;
+    if (m == 0) return __hiloint2double((int)u, 0);
+    if (m - 0x00800000u >= 0x7f000000u) return (double)f;
+    return __hiloint2double((int)((u & 0x80000000u) | ((m >> 3) + 0x38000000u)), (int)(m << 29));
   }
 };
 template <>
@@ -126,6 +135,62 @@ __device__ __forceinline__ double kr_block_sum(double v, double* red) {
   }
   __syncthreads();
   return v;
+}
+
+// ND sums at once (v1 unused for one), valid in thread 0: kr_block_sum's trees
+// -- lane l takes lane l + o for o = 16, 8, 4, 2, 1 within each warp, then the
+// same over the warps -- with the pairs of all warps packed into full ones,
+// since an FP64 addition costs a warp the same with one lane as with 32.  Two
+// sums of 256 threads take 19 warp additions instead of 90, which on 4432 blocks
+// of 16^3 were 30 us of the FP64 pipe in an 80 us A.x with two inner products.
+// buf: ND * blockDim doubles; begins and ends with a CTA barrier.
+template <int ND>
+__device__ __forceinline__ void kr_block_sums(double& v0, double& v1, double* buf) {
+  const int nt = blockDim.x, tid = threadIdx.x, nw = nt >> 5;
+  __syncthreads();
+  buf[tid] = v0;
+  if (ND == 2) buf[nt + tid] = v1;
+  __syncthreads();
+  const int rows = ND * nw;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    for (int e = tid; e < rows * o; e += nt) {
+      double* p = buf + (e / o) * 32 + e % o;
+      p[0] = __dadd_rn(p[0], p[o]);
+    }
+    if (rows * o > 32) __syncthreads();
+    else __syncwarp();
+  }
+  // lane 0 of every warp is at buf[32 w]; nw is at most 16
+  for (int o = 8; o > 0; o >>= 1) {
+    for (int e = tid; e < ND * o; e += nt) {
+      const int d = e / o, w = e % o;
+      if (w + o < nw) {
+        double* p = buf + d * nt + 32 * w;
+        p[0] = __dadd_rn(p[0], p[32 * o]);
+      }
+    }
+    __syncwarp();
+  }
+  if (tid == 0) {
+    v0 = buf[0];
+    if (ND == 2) v1 = buf[nt];
+  }
+  __syncthreads();
+}
+
+// The x ghosts of an interior row, by the threads of its first and last cell,
+// where a preconditioner's first pass writes s (or p) without reading it: whole
+// rows leave no 32-byte sector half written, which L2 fills from memory before
+// it writes it back (102 -> 97 us on 4432 blocks of 16^3; A.x and the x/r update
+// ran 6 to 8 us longer with these stores).  Nothing reads those ghosts; they are
+// zero.
+template <typename T>
+__device__ __forceinline__ void row_ends(T* p, int i, int n, int vc) {
+  if (i == 0)
+    for (int q = 1; q <= vc; q++) p[-q] = T(0);
+  if (i == n - 1)
+    for (int q = 1; q <= vc; q++) p[q] = T(0);
 }
 
 // Threads of one CTA: one per column up to 16^3 blocks (64, 256), 512 for

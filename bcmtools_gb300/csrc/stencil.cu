@@ -348,7 +348,7 @@ __global__ void __launch_bounds__(256) dot_partial_kernel(const T* __restrict__ 
                                                           const T* __restrict__ y, Geom g,
                                                           double* __restrict__ partial) {
   constexpr int U = 8;
-  __shared__ double red[32];
+  __shared__ double red[256];
   const int b = blockIdx.x;
   const int64_t base = (int64_t)b * g.bstride;
   const int nx = g.nx, ny = g.ny, nz = g.nz;
@@ -404,7 +404,8 @@ __global__ void __launch_bounds__(256) dot_partial_kernel(const T* __restrict__ 
       for (; k < nz; k++, p += g.sz) acc += (double)x[p] * (double)y[p];
     }
   }
-  acc = block_sum(acc, red);
+  double none = 0.0;
+  kr_block_sums<1>(acc, none, red);
   if (threadIdx.x == 0) partial[b] = acc;
 }
 
@@ -412,7 +413,9 @@ template <typename T>
 cudaError_t launch_dot_partial(const T* x, const T* y, const Geom& g, double* partial,
                                cudaStream_t st) {
   if (g.nb == 0) return cudaSuccess;
-  dot_partial_kernel<T><<<g.nb, min(256, g.nx * g.ny), 0, st>>>(x, y, g, partial);
+  // whole warps: kr_block_sums
+  const int nt = (min(256, g.nx * g.ny) + 31) / 32 * 32;
+  dot_partial_kernel<T><<<g.nb, nt, 0, st>>>(x, y, g, partial);
   return cudaGetLastError();
 }
 
