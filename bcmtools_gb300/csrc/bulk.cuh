@@ -9,6 +9,7 @@
 // so a lost completion can never hang the GPU.
 #pragma once
 #include <cstdint>
+#include <cuda_runtime.h>
 
 namespace bcmg {
 
@@ -86,6 +87,25 @@ __device__ __forceinline__ void griddep_wait() {
 }
 __device__ __forceinline__ void griddep_launch_dependents() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
+// Host: a launch that may begin while the kernel before it in the stream ends
+// (programmatic dependent launch); the kernel calls griddep_wait before it
+// touches what that one writes.
+template <class... P, class... A>
+inline cudaError_t launch_dependent(void (*kern)(P...), dim3 grid, dim3 block, size_t smem,
+                                    cudaStream_t st, bool pdl, A&&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = pdl ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);
 }
 
 __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, unsigned parity) {

@@ -1784,7 +1784,7 @@ struct PreArgs {
 static int jacobi_fused(bcmg_ctx c, const OpRec& o, const Field& x0, const Field& x1,
                         const Field& b, double omega, bool homogeneous, bool res, int seq,
                         int choice, cudaStream_t st, bool zero_x0 = false,
-                        const PreArgs* pre = nullptr, bool close = false) {
+                        const PreArgs* pre = nullptr, bool close = false, bool pdl = false) {
   Geom g = geom_of(c, x0);
   BlockBc bc{c->bctype.empty() ? nullptr : c->d_bctype,
              homogeneous ? c->d_bczero : c->d_bcval, c->bcform == BCMG_DIRICHLET_BCX ? 1 : 0,
@@ -1806,7 +1806,7 @@ static int jacobi_fused(bcmg_ctx c, const OpRec& o, const Field& x0, const Field
     LAUNCH(c, K_JACOBI, st, launch_jacobi_fused<double>((const double*)x0.d, (double*)x1.d,
                                                          (const double*)b.d, g, o.d_jc64, omega,
                                                          bc, push, mode, shape, part, c->d_err,
-                                                         pre ? &jp : nullptr, st));
+                                                         pre ? &jp : nullptr, st, pdl));
   } else {
     JacPre<float> jp{pre ? pre->kind : kPreNone, pre ? (const float*)pre->r->d : nullptr,
                      pre && pre->q ? (const float*)pre->q->d : nullptr,
@@ -1814,7 +1814,7 @@ static int jacobi_fused(bcmg_ctx c, const OpRec& o, const Field& x0, const Field
     LAUNCH(c, K_JACOBI, st, launch_jacobi_fused<float>((const float*)x0.d, (float*)x1.d,
                                                         (const float*)b.d, g, o.d_jc32,
                                                         (float)omega, bc, push, mode, shape, part,
-                                                        c->d_err, pre ? &jp : nullptr, st));
+                                                        c->d_err, pre ? &jp : nullptr, st, pdl));
   }
   return BCMG_SUCCESS;
 }
@@ -2134,7 +2134,8 @@ static int jacobi_pre(bcmg_ctx c, int op, Field& x, Field& x0, Field& b, double 
     int rc;
     if (fused) {
       rc = jacobi_fused(c, c->ops[op], x, x0, b, omega, true, false, 0, kJacPush, st,
-                        zero_pass && k == 0, k == 0 ? pre : nullptr);
+                        zero_pass && k == 0, k == 0 ? pre : nullptr, false,
+                        kr_dependent(dsize(x.dtype), geom_of(c, x)));
       if (rc) return rc;
       std::swap(x.d, x0.d);
       continue;
@@ -2209,16 +2210,19 @@ static int kr_iteration(bcmg_ctx c, int op, const KrVecs& v, const Op<T>& o, KSe
                        recip)))
     return rc;
   LAUNCH(c, K_RESIDUAL, st, launch_kr_ax<T>(d(v.q_), d(v.p_), o, d(v.r0), 1, g, S, part, c->d_err, st));
-  LAUNCH(c, K_DOT, st, launch_kr_scalar(part, c->nb, S, KS_ALPHA, max_iter, eps2, keep_best, st));
+  LAUNCH(c, K_DOT, st, launch_kr_scalar(part, c->nb, S, KS_ALPHA, max_iter, eps2, keep_best,
+                                     kr_dependent(sizeof(T), g), st));
   if (!fuse) LAUNCH(c, K_BLAS1, st, launch_kr_s<T>(d(v.s), d(v.r), d(v.q_), g, S, st));
   if ((rc = jacobi_pre(c, op, *v.s_, *v.x0, *v.s, omega, n_pre, st, true, fuse ? &pre_s : nullptr,
                        recip)))
     return rc;
   LAUNCH(c, K_RESIDUAL, st, launch_kr_ax<T>(d(v.t_), d(v.s_), o, d(v.s), 2, g, S, part, c->d_err, st));
-  LAUNCH(c, K_DOT, st, launch_kr_scalar(part, c->nb, S, KS_GAMMA, max_iter, eps2, keep_best, st));
+  LAUNCH(c, K_DOT, st, launch_kr_scalar(part, c->nb, S, KS_GAMMA, max_iter, eps2, keep_best,
+                                     kr_dependent(sizeof(T), g), st));
   LAUNCH(c, K_BLAS1, st, launch_kr_xr<T>(d(v.x), d(v.r), d(v.p_), d(v.s_), d(v.s), d(v.t_),
                                          d(v.r0), g, S, part, c->d_err, st));
-  LAUNCH(c, K_DOT, st, launch_kr_scalar(part, c->nb, S, KS_R, max_iter, eps2, keep_best, st));
+  LAUNCH(c, K_DOT, st, launch_kr_scalar(part, c->nb, S, KS_R, max_iter, eps2, keep_best,
+                                     kr_dependent(sizeof(T), g), st));
   if (keep_best) LAUNCH(c, K_BLAS1, st, launch_kr_best<T>(d(v.xbest), d(v.x), g, S, st));
   return BCMG_SUCCESS;
 }
@@ -2279,7 +2283,7 @@ static int bicgstab_dev(bcmg_ctx c, int op, KrVecs v, double omega, int n_pre, i
   LAUNCH(c, K_DOT, st, launch_kr_dot2<T>((T*)v.b->d, (T*)v.b->d, (T*)v.r->d, (T*)v.r0->d, g,
                                          c->d_kpart, st));
   LAUNCH(c, K_DOT, st, launch_kr_scalar(c->d_kpart, c->nb, S, KS_INIT, max_iter, eps2,
-                                        keep_best ? 1 : 0, st));
+                                        keep_best ? 1 : 0, false, st));
   auto read_back = [&]() -> int {
     CUDA_TRY(c, cudaMemcpyAsync(c->h_kseg, c->d_kseg, (size_t)nseg * sizeof(KSeg),
                                 cudaMemcpyDeviceToHost, st));

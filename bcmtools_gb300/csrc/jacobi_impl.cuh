@@ -36,7 +36,8 @@ struct JacArgs {
   double* partial;   // [nb] sum of squared residuals of x0 (or null)
   int* err;          // device error word (bounded-wait timeouts)
   int zero_x0;       // 32^3 push form: x0 is zero everywhere and is not read
-  JacPre<T> pre;     // 32^3 streamed zero-start pass: b made in the same pass
+  JacPre<T> pre;     // zero-start pass: b made in the same pass
+  bool pdl;          // launched as a dependent of the kernel before (launch_dependent)
 };
 
 // Index of the out-of-range coordinate u in [0, 2VC): -VC..-1, then N..N+VC-1.
@@ -58,6 +59,8 @@ __global__ void __launch_bounds__(N * N, (BrickStage<T, N, VC, true>::MIN_BLOCKS
   __shared__ double red[NW];
   __shared__ VcTask outs[PULL ? kMaxOutEntries : 1];
   __shared__ float dv2f[8];
+  griddep_launch_dependents();
+  griddep_wait();
   uint64_t* bar = reinterpret_cast<uint64_t*>(smraw);
   T* xs = reinterpret_cast<T*>(smraw + L::X_OFF);
   T* bs = reinterpret_cast<T*>(smraw + L::B_OFF);
@@ -457,6 +460,8 @@ __global__ void __launch_bounds__(N * N, (N == 8 ? 12 : sizeof(T) == 4 ? (VC == 
   using BL = BrickTile<T, N, VC>;
   constexpr int NT = N * N, LXY = BL::LXY, U = 4;
   __shared__ T x1s[N * N * N];
+  griddep_launch_dependents();
+  griddep_wait();
   const int b = blockIdx.x, tid = threadIdx.x;
   T s_beta = T(0), s_ng = T(0), s_na = T(0);
   if (PRE != kPreNone) {
@@ -506,12 +511,11 @@ template <typename T, int N, int VC>
 static cudaError_t jacobi_zero_push_launch(T* x1, T* b, const Geom& g, const JacArgs<T>& a,
                                            cudaStream_t st) {
   switch (a.pre.kind) {
-    case kPreP: jacobi_zero_push_kernel<T, N, VC, kPreP><<<g.nb, N * N, 0, st>>>(x1, b, g, a); break;
-    case kPreS: jacobi_zero_push_kernel<T, N, VC, kPreS><<<g.nb, N * N, 0, st>>>(x1, b, g, a); break;
-    case kPreCopy: jacobi_zero_push_kernel<T, N, VC, kPreCopy><<<g.nb, N * N, 0, st>>>(x1, b, g, a); break;
-    default: jacobi_zero_push_kernel<T, N, VC, kPreNone><<<g.nb, N * N, 0, st>>>(x1, b, g, a); break;
+    case kPreP: return launch_dependent(jacobi_zero_push_kernel<T, N, VC, kPreP>, g.nb, N * N, 0, st, a.pdl, x1, b, g, a);
+    case kPreS: return launch_dependent(jacobi_zero_push_kernel<T, N, VC, kPreS>, g.nb, N * N, 0, st, a.pdl, x1, b, g, a);
+    case kPreCopy: return launch_dependent(jacobi_zero_push_kernel<T, N, VC, kPreCopy>, g.nb, N * N, 0, st, a.pdl, x1, b, g, a);
+    default: return launch_dependent(jacobi_zero_push_kernel<T, N, VC, kPreNone>, g.nb, N * N, 0, st, a.pdl, x1, b, g, a);
   }
-  return cudaGetLastError();
 }
 
 // Push-form fused Jacobi on 32^3 blocks (too large to stage in shared
@@ -641,6 +645,8 @@ __global__ void __launch_bounds__(NT_, (JacStream<T, N, VC, S, RES, ZERO, NT_, P
   __shared__ float xface[XW ? 2 * 3 * N * 2 : 1];
   __shared__ VcTask xle[XW ? kXle : 1];
   __shared__ int nxle;
+  griddep_launch_dependents();
+  griddep_wait();
   const int b = blockIdx.x, tid = threadIdx.x, w = tid >> 5, lane = tid & 31;
   const int64_t base = (int64_t)b * g.bstride;
   // the update's scalars; a finished segment's blocks change nothing (their
@@ -930,8 +936,7 @@ static cudaError_t jacobi_stream_launch_one(const T* x0, T* x1, const T* b, cons
     if (e != cudaSuccess) return e;
     attr_set = true;
   }
-  kern<<<g.nb, JS::NT, JS::SMEM, st>>>(x0, x1, b, g, a);
-  return cudaGetLastError();
+  return launch_dependent(kern, g.nb, JS::NT, JS::SMEM, st, a.pdl, x0, x1, b, g, a);
 }
 
 // Ring depths of the streamed Jacobi (74 KB of shared memory, 3 CTAs per
@@ -993,8 +998,7 @@ static cudaError_t jacobi_tile_launch(const T* x0, T* x1, const T* b, const Geom
     if (e != cudaSuccess) return e;
     attr_set[ki] = true;
   }
-  kern<<<g.nb, L::NT, L::SMEM, st>>>(x0, x1, b, g, a);
-  return cudaGetLastError();
+  return launch_dependent(kern, g.nb, L::NT, L::SMEM, st, a.pdl, x0, x1, b, g, a);
 }
 
 template <typename T, int N, int VC>
@@ -1020,13 +1024,13 @@ template <typename T>
 cudaError_t launch_jacobi_fused_impl(const T* x0, T* x1, const T* b, const Geom& g, const T* cf,
                                      T omega, BlockBc bc, PushTable push, int ghost_mode,
                                      int shape, double* partial, int* err, const JacPre<T>* pre,
-                                     cudaStream_t st) {
+                                     cudaStream_t st, bool pdl) {
   if (g.nb == 0) return cudaSuccess;
   if (g.nx == 32 && g.ny == 32 && g.nz == 32 && (g.vc == 1 || g.vc == 2)) {
     // 32^3: push form only
     if (ghost_mode != kGhostPush && ghost_mode != kGhostPushZero) return cudaErrorInvalidValue;
     JacArgs<T> a{0, cf, omega, bc, push, partial, err, ghost_mode == kGhostPushZero ? 1 : 0,
-                 pre ? *pre : JacPre<T>{kPreNone, nullptr, nullptr, KSegs{}}};
+                 pre ? *pre : JacPre<T>{kPreNone, nullptr, nullptr, KSegs{}}, pdl};
     const bool streamed = plane_stream_enabled() && stream_aligned<T>(g, x0, b) &&
                           (!pre || (stream_aligned<T>(g, pre->r, pre->q ? pre->q : pre->r)));
     if (a.pre.kind != kPreNone && !streamed) return cudaErrorNotSupported;
@@ -1040,7 +1044,7 @@ cudaError_t launch_jacobi_fused_impl(const T* x0, T* x1, const T* b, const Geom&
   if (ghost_mode == kGhostPushZero) {
     if (partial) return cudaErrorInvalidValue;
     JacArgs<T> a{0, cf, omega, bc, push, nullptr, err, 1,
-                 pre ? *pre : JacPre<T>{kPreNone, nullptr, nullptr, KSegs{}}};
+                 pre ? *pre : JacPre<T>{kPreNone, nullptr, nullptr, KSegs{}}, pdl};
     T* bw = const_cast<T*>(b);  // written only where pre makes it
     if (g.nx == 16)
       return g.vc == 1 ? jacobi_zero_push_launch<T, 16, 1>(x1, bw, g, a, st)
@@ -1063,7 +1067,8 @@ cudaError_t launch_jacobi_fused_impl(const T* x0, T* x1, const T* b, const Geom&
   }
   const bool pl = ghost_mode != kGhostPush;
   const bool close = ghost_mode == kGhostPullClose || ghost_mode == kGhostAsIsClose;
-  JacArgs<T> a{ghost_mode == kGhostPull || ghost_mode == kGhostPullClose ? 1 : 0, cf, omega, bc, push, partial, err};
+  JacArgs<T> a{ghost_mode == kGhostPull || ghost_mode == kGhostPullClose ? 1 : 0, cf, omega, bc, push, partial, err, 0,
+               JacPre<T>{kPreNone, nullptr, nullptr, KSegs{}}, pdl};
   if (g.nx == 16)
     return g.vc == 1 ? jacobi_tile_launch<T, 16, 1>(x0, x1, b, g, a, pl, close, st)
                      : jacobi_tile_launch<T, 16, 2>(x0, x1, b, g, a, pl, close, st);

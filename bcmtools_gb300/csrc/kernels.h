@@ -218,7 +218,8 @@ cudaError_t launch_jacobi(T* x1, const T* x0, const T* b, Op<T> op, const Geom& 
 // corners, ghost layers no neighbour or Dirichlet condition writes) takes
 // x0's value.  partial[b] = sum of squared residuals of x0 when partial !=
 // null.  cudaErrorInvalidValue for shapes it does not cover (cubic 8/16
-// blocks, vc <= 2, tiles within shared memory).
+// blocks, vc <= 2, tiles within shared memory).  pdl: launched as a dependent of
+// the kernel before (launch_dependent, bulk.cuh), which the push forms allow.
 // Ghost modes of the fused sweeps.  kGhostPush: x0's ghosts are read as
 // they are and the launch writes every ghost x1 feeds (x1 leaves with all
 // ghosts updated).  kGhostPull: the launch first fills x0's first ghost
@@ -253,7 +254,7 @@ template <typename T>
 cudaError_t launch_jacobi_fused(const T* x0, T* x1, const T* b, const Geom& g, const T* cf,
                                 T omega, BlockBc bc, PushTable push, int ghost_mode, int shape,
                                 double* partial, int* err, const JacPre<T>* pre,
-                                cudaStream_t st);
+                                cudaStream_t st, bool pdl = false);
 // mode 0: ax = A x;  mode 1: r = b - A x;  mode 2: partial[b] = sum r^2 (no store)
 template <typename T>
 cudaError_t launch_residual(T* out, const T* x, const T* b, Op<T> op, const Geom& g, int mode,
@@ -290,6 +291,16 @@ template <typename T>
 cudaError_t launch_xch(T* data, const Geom& g, const VcTask* ents, const int64_t* off, int n,
                        T* buf, bool pack, cudaStream_t st);
 
+// Whether the BiCGSTAB iteration's kernels are launched as dependents of one
+// another (launch_dependent, bulk.cuh): FP32, where the gap between two launches
+// is some per cent of a kernel (six solves of 1001 blocks of 16^3: 62.7 -> 59.3
+// ms).  Not where a kernel's blocks fill less than two waves of three CTAs per SM:
+// the next one's CTAs then take the free slots unevenly (FP64, 342 blocks of
+// 32^3: 38.6 -> 40.7 ms).
+inline bool kr_dependent(size_t es, const Geom& g) {
+  return es == 4 && (g.nx * g.ny * g.nz <= 4096 || g.nb >= 2 * 3 * 152);
+}
+
 // Device-resident BiCGSTAB iteration (krylov.cu): see krylov.cuh.
 template <typename T>
 cudaError_t launch_kr_p(T* p, const T* r, const T* q, const Geom& g, KSegs S, cudaStream_t st);
@@ -312,7 +323,7 @@ cudaError_t launch_kr_dot2(const T* x, const T* y, const T* u, const T* v, const
 template <typename T>
 cudaError_t launch_kr_best(T* xbest, const T* x, const Geom& g, KSegs S, cudaStream_t st);
 cudaError_t launch_kr_scalar(const double* partial, int nb, KSegs S, int stage, int max_iter,
-                             double eps2, int keep_best, cudaStream_t st);
+                             double eps2, int keep_best, bool dependent, cudaStream_t st);
 cudaError_t launch_kr_segsum(const double* partial, int nb, KSegs S, double* out,
                              cudaStream_t st);
 template <typename T>

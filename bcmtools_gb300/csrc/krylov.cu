@@ -6,10 +6,14 @@
 // Inner products: FP64 multiply-add per element along the column, then the
 // CTA's fixed-order tree (kr_block_sums); partial sums per block go to
 // partial[slot * nb + b] and kr_scalar reduces them per segment.
+// The iteration's kernels may be launched as dependents of one another
+// (kr_dependent): each starts as the one before drains, and waits for it before
+// its first access.
 #include <cfloat>
 #include <type_traits>
 
 #include "bcmg.h"
+#include "bulk.cuh"
 #include "cells.cuh"
 #include "kernels.h"
 #include "krylov.cuh"
@@ -87,6 +91,8 @@ __global__ void __launch_bounds__(kr_nt<N>(), (CC ? kr_minb<T, N, true>() : 768 
     T* __restrict__ out, const T* __restrict__ x, const T* __restrict__ cf8, Op<T> op,
     const T* __restrict__ y0, Geom g, KSegs S, double* __restrict__ partial) {
   __shared__ double red[NDOT * kr_nt<N>()];
+  griddep_launch_dependents();
+  griddep_wait();
   const int b = blockIdx.x;
   if (S.seg[kseg_of(S, b)].status != kRunning) return;
   T c[7];
@@ -179,6 +185,8 @@ __global__ void __launch_bounds__(NT_, (AxStream<T, N, VC, S, NT_>::MINB)) kr_ax
   extern __shared__ __align__(128) unsigned char smraw[];
   double* red = reinterpret_cast<double*>(smraw + R::BAR_BYTES);  // the ring, after the walk
   static_assert(AS::SMEM >= R::BAR_BYTES + 2 * NT * sizeof(double), "room for the sums");
+  griddep_launch_dependents();
+  griddep_wait();
   const int b = blockIdx.x, tid = threadIdx.x;
   if (S_.seg[kseg_of(S_, b)].status != kRunning) return;
   const int64_t base = (int64_t)b * g.bstride;
@@ -266,8 +274,7 @@ static cudaError_t kr_ax_stream_one(T* out, const T* x, const T* cf8, const T* y
     if (e != cudaSuccess) return e;
     attr_set = true;
   }
-  kern<<<g.nb, AS::NT, AS::SMEM, st>>>(out, x, cf8, y0, g, S_, partial, err);
-  return cudaGetLastError();
+  return launch_dependent(kern, g.nb, AS::NT, AS::SMEM, st, kr_dependent(sizeof(T), g), out, x, cf8, y0, g, S_, partial, err);
 }
 
 // Ring depths: 32^3 4 slots (FP32: 6 CTAs per SM, FP64: 3); 16^3 8 (FP32)
@@ -306,6 +313,8 @@ __global__ void __launch_bounds__(256, (XrStream<T, N, VC, S>::MINB)) kr_xr_stre
   extern __shared__ __align__(128) unsigned char smraw[];
   double* red = reinterpret_cast<double*>(smraw + R::BAR_BYTES);  // the ring, after the walk
   static_assert(XS::SMEM >= R::BAR_BYTES + 2 * NT * sizeof(double), "room for the sums");
+  griddep_launch_dependents();
+  griddep_wait();
   const int b = blockIdx.x, tid = threadIdx.x;
   const KSeg& sg = S_.seg[kseg_of(S_, b)];
   if (sg.status != kRunning) return;
@@ -367,8 +376,8 @@ static cudaError_t kr_xr_stream(T* x, T* r, const T* p_, const T* s_, const T* s
     if (e != cudaSuccess) return e;
     attr_set = true;
   }
-  kern<<<g.nb, XS::NT, XS::SMEM, st>>>(x, r, p_, s_, s, t, r0, g, S_, partial, err);
-  return cudaGetLastError();
+  return launch_dependent(kern, g.nb, XS::NT, XS::SMEM, st, kr_dependent(sizeof(T), g), x, r, p_, s_, s, t, r0, g, S_,
+                          partial, err);
 }
 
 // x = alpha p^ + gamma s^ + x (AXPBYPZ, ILS3D.h:783, blas.f90:345-377) and
@@ -380,6 +389,8 @@ __global__ void __launch_bounds__(kr_nt<N>(), (kr_minb<T, N, true>())) kr_xr_ker
     const T* __restrict__ s, const T* __restrict__ t, const T* __restrict__ r0, Geom g, KSegs S,
     double* __restrict__ partial) {
   __shared__ double red[2 * kr_nt<N>()];
+  griddep_launch_dependents();
+  griddep_wait();
   const int b = blockIdx.x;
   const KSeg& sg = S.seg[kseg_of(S, b)];
   if (sg.status != kRunning) return;
@@ -461,6 +472,8 @@ template <typename T, bool CC, int PRE>
 __global__ void __launch_bounds__(256) kr_zero_pass_kernel(T* __restrict__ x1, T* __restrict__ b,
                                                            JacPre<T> pre, Op<T> op, Geom g,
                                                            T omega, int zc) {
+  griddep_launch_dependents();
+  griddep_wait();
   const int blk = blockIdx.x;
   T beta = T(0), ng = T(0), na = T(0);
   if (PRE != kPreNone) {
@@ -526,9 +539,9 @@ cudaError_t launch_kr_zero_pass(T* x1, T* b, const JacPre<T>& pre, const Op<T>& 
   const dim3 grid(g.nb, (g.nz + zc - 1) / zc);
 #define Z_(PRE)                                                                            \
   if (op.cc)                                                                               \
-    kr_zero_pass_kernel<T, true, PRE><<<grid, nt, 0, st>>>(x1, b, pre, op, g, omega, zc);   \
+    return launch_dependent(kr_zero_pass_kernel<T, true, PRE>, grid, nt, 0, st, kr_dependent(sizeof(T), g), x1, b, pre, op, g, omega, zc);   \
   else                                                                                     \
-    kr_zero_pass_kernel<T, false, PRE><<<grid, nt, 0, st>>>(x1, b, pre, op, g, omega, zc)
+    return launch_dependent(kr_zero_pass_kernel<T, false, PRE>, grid, nt, 0, st, kr_dependent(sizeof(T), g), x1, b, pre, op, g, omega, zc)
   switch (pre.kind) {
     case kPreP: Z_(kPreP); break;
     case kPreS: Z_(kPreS); break;
@@ -545,6 +558,8 @@ template <typename T>
 __global__ void __launch_bounds__(256) kr_best_kernel(T* __restrict__ xbest,
                                                       const T* __restrict__ x, Geom g,
                                                       KSegs S) {
+  griddep_launch_dependents();
+  griddep_wait();
   const int b = blockIdx.x;
   if (!S.seg[kseg_of(S, b)].improved) return;
   const int64_t base = (int64_t)b * g.bstride;
@@ -629,6 +644,8 @@ __device__ __forceinline__ void kr_segment_sums(const double* __restrict__ parti
 __global__ void __launch_bounds__(256) kr_scalar_kernel(const double* __restrict__ partial, int nb,
                                                         KSegs S, int stage, int max_iter,
                                                         double eps2, int keep_best) {
+  griddep_launch_dependents();
+  griddep_wait();
   __shared__ double red[32];
   const int sgi = blockIdx.x;
   KSeg& sg = S.seg[sgi];
@@ -789,17 +806,13 @@ cudaError_t launch_kr_ax(T* out, const T* x, Op<T> op, const T* y0, int ndot, co
   }
 #define C_(N)                                                                                     \
   if (cc && ndot == 2)                                                                            \
-    kr_ax_kernel<T, N, true, 2><<<g.nb, kr_threads<N>(g), 0, st>>>(out, x, op.cf8, op, y0, g, S,  \
-                                                                   partial);                      \
+    return launch_dependent(kr_ax_kernel<T, N, true, 2>, g.nb, kr_threads<N>(g), 0, st, kr_dependent(sizeof(T), g), out, x, op.cf8, op, y0, g, S, partial);                      \
   else if (cc)                                                                                    \
-    kr_ax_kernel<T, N, true, 1><<<g.nb, kr_threads<N>(g), 0, st>>>(out, x, op.cf8, op, y0, g, S,  \
-                                                                   partial);                      \
+    return launch_dependent(kr_ax_kernel<T, N, true, 1>, g.nb, kr_threads<N>(g), 0, st, kr_dependent(sizeof(T), g), out, x, op.cf8, op, y0, g, S, partial);                      \
   else if (ndot == 2)                                                                             \
-    kr_ax_kernel<T, N, false, 2><<<g.nb, kr_threads<N>(g), 0, st>>>(out, x, op.cf8, op, y0, g, S, \
-                                                                    partial);                     \
+    return launch_dependent(kr_ax_kernel<T, N, false, 2>, g.nb, kr_threads<N>(g), 0, st, kr_dependent(sizeof(T), g), out, x, op.cf8, op, y0, g, S, partial);                     \
   else                                                                                            \
-    kr_ax_kernel<T, N, false, 1><<<g.nb, kr_threads<N>(g), 0, st>>>(out, x, op.cf8, op, y0, g, S, \
-                                                                    partial)
+    return launch_dependent(kr_ax_kernel<T, N, false, 1>, g.nb, kr_threads<N>(g), 0, st, kr_dependent(sizeof(T), g), out, x, op.cf8, op, y0, g, S, partial)
   KR_DISPATCH(C_)
 #undef C_
   return cudaGetLastError();
@@ -817,7 +830,7 @@ cudaError_t launch_kr_xr(T* x, T* r, const T* p_, const T* s_, const T* s, const
     return g.vc == 1 ? kr_xr_stream<T, 32, 1, 2>(x, r, p_, s_, s, t, r0, g, S, partial, err, st)
                      : kr_xr_stream<T, 32, 2, 2>(x, r, p_, s_, s, t, r0, g, S, partial, err, st);
 #define C_(N) \
-  kr_xr_kernel<T, N><<<g.nb, kr_threads<N>(g), 0, st>>>(x, r, p_, s_, s, t, r0, g, S, partial)
+  return launch_dependent(kr_xr_kernel<T, N>, g.nb, kr_threads<N>(g), 0, st, kr_dependent(sizeof(T), g), x, r, p_, s_, s, t, r0, g, S, partial)
   KR_DISPATCH(C_)
 #undef C_
   return cudaGetLastError();
@@ -836,14 +849,13 @@ cudaError_t launch_kr_dot2(const T* x, const T* y, const T* u, const T* v, const
 template <typename T>
 cudaError_t launch_kr_best(T* xbest, const T* x, const Geom& g, KSegs S, cudaStream_t st) {
   if (g.nb == 0) return cudaSuccess;
-  kr_best_kernel<T><<<g.nb, 256, 0, st>>>(xbest, x, g, S);
-  return cudaGetLastError();
+  return launch_dependent(kr_best_kernel<T>, g.nb, 256, 0, st, kr_dependent(sizeof(T), g), xbest, x, g, S);
 }
 
 cudaError_t launch_kr_scalar(const double* partial, int nb, KSegs S, int stage, int max_iter,
-                             double eps2, int keep_best, cudaStream_t st) {
-  kr_scalar_kernel<<<S.nseg, 256, 0, st>>>(partial, nb, S, stage, max_iter, eps2, keep_best);
-  return cudaGetLastError();
+                             double eps2, int keep_best, bool dependent, cudaStream_t st) {
+  return launch_dependent(kr_scalar_kernel, S.nseg, 256, 0, st, dependent, partial, nb, S, stage, max_iter,
+                          eps2, keep_best);
 }
 
 cudaError_t launch_kr_segsum(const double* partial, int nb, KSegs S, double* out,
