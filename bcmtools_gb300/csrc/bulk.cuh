@@ -91,20 +91,29 @@ __device__ __forceinline__ void griddep_launch_dependents() {
 
 // Host: a launch that may begin while the kernel before it in the stream ends
 // (programmatic dependent launch); the kernel calls griddep_wait before it
-// touches what that one writes.
+// touches what that one writes.  cluster > 1: in clusters of so many CTAs.
 template <class... P, class... A>
 inline cudaError_t launch_dependent(void (*kern)(P...), dim3 grid, dim3 block, size_t smem,
-                                    cudaStream_t st, bool pdl, A&&... args) {
+                                    cudaStream_t st, bool pdl, int cluster, A&&... args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
   cfg.blockDim = block;
   cfg.dynamicSmemBytes = smem;
   cfg.stream = st;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchAttribute attr[2];
+  int n = 0;
+  if (pdl) {
+    attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[n++].val.programmaticStreamSerializationAllowed = 1;
+  }
+  if (cluster > 1) {
+    attr[n].id = cudaLaunchAttributeClusterDimension;
+    attr[n].val.clusterDim.x = cluster;
+    attr[n].val.clusterDim.y = 1;
+    attr[n++].val.clusterDim.z = 1;
+  }
   cfg.attrs = attr;
-  cfg.numAttrs = pdl ? 1 : 0;
+  cfg.numAttrs = n;
   return cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);
 }
 

@@ -2149,14 +2149,14 @@ static int jacobi_pre(bcmg_ctx c, int op, Field& x, Field& x0, Field& b, double 
   return BCMG_SUCCESS;
 }
 
-// Scratch of the device-resident BiCGSTAB: two FP64 partial sums per block
+// Scratch of the device-resident BiCGSTAB: two FP64 partial sums per part of a block
 // and `nseg` scalar records (device, and a pinned host mirror).
 static int kr_scratch(bcmg_ctx c, int nseg) {
   if (c->kpart_nb < c->nb) {
     cudaFree(c->d_kpart);
     c->d_kpart = nullptr;
     c->kpart_nb = 0;
-    CUDA_TRY(c, cudaMalloc(&c->d_kpart, (size_t)2 * c->nb * sizeof(double)));
+    CUDA_TRY(c, cudaMalloc(&c->d_kpart, (size_t)2 * kKrMaxParts * c->nb * sizeof(double)));
     c->kpart_nb = c->nb;
   }
   if (c->kseg_cap < nseg) {
@@ -2188,6 +2188,11 @@ static int kr_iteration(bcmg_ctx c, int op, const KrVecs& v, const Op<T>& o, KSe
                         bool first, const double* recip, cudaStream_t st) {
   const Geom g = geom_of(c, *v.x);
   double* part = c->d_kpart;
+  // FP32 with constant coefficients keeps one sum per block
+  const bool in_parts = sizeof(T) == 8 || !o.cc;
+  const bool fixed = c->nx == c->ny && c->ny == c->nz && (c->nx == 8 || c->nx == 16 || c->nx == 32);
+  const int ax_parts = in_parts ? kr_parts(g) : 1;
+  const int xr_parts = in_parts && !(sizeof(T) == 4 && fixed) ? kr_parts(g) : 1;
   int rc;
   auto d = [](Field* f) { return (T*)f->d; };
   // p's and s's updates made by their preconditioner's first pass (one launch
@@ -2209,19 +2214,19 @@ static int kr_iteration(bcmg_ctx c, int op, const KrVecs& v, const Op<T>& o, KSe
   if ((rc = jacobi_pre(c, op, *v.p_, *v.x0, *v.p, omega, n_pre, st, true, fuse ? &pre_p : nullptr,
                        recip)))
     return rc;
-  LAUNCH(c, K_RESIDUAL, st, launch_kr_ax<T>(d(v.q_), d(v.p_), o, d(v.r0), 1, g, S, part, c->d_err, st));
-  LAUNCH(c, K_DOT, st, launch_kr_scalar(part, c->nb, S, KS_ALPHA, max_iter, eps2, keep_best,
+  LAUNCH(c, K_RESIDUAL, st, launch_kr_ax<T>(d(v.q_), d(v.p_), o, d(v.r0), 1, g, ax_parts, S, part, c->d_err, st));
+  LAUNCH(c, K_DOT, st, launch_kr_scalar(part, c->nb, ax_parts, S, KS_ALPHA, max_iter, eps2, keep_best,
                                      kr_dependent(sizeof(T), g), st));
   if (!fuse) LAUNCH(c, K_BLAS1, st, launch_kr_s<T>(d(v.s), d(v.r), d(v.q_), g, S, st));
   if ((rc = jacobi_pre(c, op, *v.s_, *v.x0, *v.s, omega, n_pre, st, true, fuse ? &pre_s : nullptr,
                        recip)))
     return rc;
-  LAUNCH(c, K_RESIDUAL, st, launch_kr_ax<T>(d(v.t_), d(v.s_), o, d(v.s), 2, g, S, part, c->d_err, st));
-  LAUNCH(c, K_DOT, st, launch_kr_scalar(part, c->nb, S, KS_GAMMA, max_iter, eps2, keep_best,
+  LAUNCH(c, K_RESIDUAL, st, launch_kr_ax<T>(d(v.t_), d(v.s_), o, d(v.s), 2, g, ax_parts, S, part, c->d_err, st));
+  LAUNCH(c, K_DOT, st, launch_kr_scalar(part, c->nb, ax_parts, S, KS_GAMMA, max_iter, eps2, keep_best,
                                      kr_dependent(sizeof(T), g), st));
   LAUNCH(c, K_BLAS1, st, launch_kr_xr<T>(d(v.x), d(v.r), d(v.p_), d(v.s_), d(v.s), d(v.t_),
-                                         d(v.r0), g, S, part, c->d_err, st));
-  LAUNCH(c, K_DOT, st, launch_kr_scalar(part, c->nb, S, KS_R, max_iter, eps2, keep_best,
+                                         d(v.r0), g, xr_parts, S, part, c->d_err, st));
+  LAUNCH(c, K_DOT, st, launch_kr_scalar(part, c->nb, xr_parts, S, KS_R, max_iter, eps2, keep_best,
                                      kr_dependent(sizeof(T), g), st));
   if (keep_best) LAUNCH(c, K_BLAS1, st, launch_kr_best<T>(d(v.xbest), d(v.x), g, S, st));
   return BCMG_SUCCESS;
@@ -2282,7 +2287,7 @@ static int bicgstab_dev(bcmg_ctx c, int op, KrVecs v, double omega, int n_pre, i
   CUDA_TRY(c, cudaMemcpyAsync(v.r0->d, v.r->d, v.r->bytes, cudaMemcpyDeviceToDevice, st));
   LAUNCH(c, K_DOT, st, launch_kr_dot2<T>((T*)v.b->d, (T*)v.b->d, (T*)v.r->d, (T*)v.r0->d, g,
                                          c->d_kpart, st));
-  LAUNCH(c, K_DOT, st, launch_kr_scalar(c->d_kpart, c->nb, S, KS_INIT, max_iter, eps2,
+  LAUNCH(c, K_DOT, st, launch_kr_scalar(c->d_kpart, c->nb, 1, S, KS_INIT, max_iter, eps2,
                                         keep_best ? 1 : 0, false, st));
   auto read_back = [&]() -> int {
     CUDA_TRY(c, cudaMemcpyAsync(c->h_kseg, c->d_kseg, (size_t)nseg * sizeof(KSeg),

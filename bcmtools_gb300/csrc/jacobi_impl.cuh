@@ -37,6 +37,7 @@ struct JacArgs {
   int* err;          // device error word (bounded-wait timeouts)
   int zero_x0;       // 32^3 push form: x0 is zero everywhere and is not read
   JacPre<T> pre;     // zero-start pass: b made in the same pass
+  int ranks;         // CTAs per block of the split streamed kernel
   bool pdl;          // launched as a dependent of the kernel before (launch_dependent)
 };
 
@@ -347,13 +348,15 @@ __global__ void __launch_bounds__(N * N, (BrickStage<T, N, VC, true>::MIN_BLOCKS
 // back from the brick.  NT threads, one warp per face-table entry, UB cells
 // in flight per lane; !COPIES: the same-level entries were written during
 // the sweep and are skipped here.
-// src: x1's interior in the layout SL (default: its brick in X1).
+// src: x1's interior in the layout SL (default: its brick in X1).  rank, ranks:
+// this CTA's share when several take the block.
 template <typename T, int N, int VC, int NT, int UB = 8, bool COPIES = true,
           class SL = BrickTile<T, N, VC>>
 __device__ __forceinline__ void jacobi_push_tail(const T* __restrict__ X0, T* __restrict__ X1,
                                                  const Geom& g, const JacArgs<T>& a, int b,
                                                  int tid, bool zero, int skip_x = 0,
-                                                 const T* src = nullptr) {
+                                                 const T* src = nullptr, int rank = 0,
+                                                 int ranks = 1) {
   using BL = BrickTile<T, N, VC>;
   constexpr int NW = NT / 32, LX = BL::LX;
   const int w = tid >> 5, lane = tid & 31;
@@ -366,7 +369,7 @@ __device__ __forceinline__ void jacobi_push_tail(const T* __restrict__ X0, T* __
     constexpr int NA = W * W * LX;  // z and y outside: whole rows
     constexpr int NE = W * N * W;   // z outside, y inside, x outside
     constexpr int NC = N * W * W;   // z inside, y and x outside
-    for (int e = tid; e < NA + NE + NC; e += NT) {
+    for (int e = tid + rank * NT; e < NA + NE + NC; e += NT * ranks) {
       int x, y, z;
       if (e < NA) {
         x = e % LX - VC;
@@ -405,7 +408,7 @@ __device__ __forceinline__ void jacobi_push_tail(const T* __restrict__ X0, T* __
       const int ax = fc >> 1;
       const bool minus = (fc & 1) == 0;
       const bool second = a.bc.bcx && VC >= 2;
-      for (int e = tid; e < VC * N * N; e += NT) {
+      for (int e = tid + rank * NT; e < VC * N * N; e += NT * ranks) {
         const int p = e % N, q = (e / N) % N, u = e / (N * N);
         const int l = minus ? -1 - u : N + u, l0 = minus ? 0 : N - 1;
         int gi, ii;
@@ -429,11 +432,12 @@ __device__ __forceinline__ void jacobi_push_tail(const T* __restrict__ X0, T* __
     // the same-level entries were written during the sweep, and so were the
     // first skip_x level-change entries of x faces; the level-change entries
     // left (about two per block) take the whole CTA each
-    int nx = 0;
+    int nx = 0, left = 0;
     for (int q = p0; q < p1; q++) {
       const VcTask t = a.push.tasks[q];
       if (t.kind == VC_COPY) continue;
       if ((t.face >> 1) == 0 && nx++ < skip_x) continue;
+      if (left++ % ranks != rank) continue;
       push_dispatch_cta<T, N, VC, SL, NT, UB>(t, X1 + (int64_t)t.dst * g.bstride, g, src, tid);
     }
   }
@@ -511,10 +515,10 @@ template <typename T, int N, int VC>
 static cudaError_t jacobi_zero_push_launch(T* x1, T* b, const Geom& g, const JacArgs<T>& a,
                                            cudaStream_t st) {
   switch (a.pre.kind) {
-    case kPreP: return launch_dependent(jacobi_zero_push_kernel<T, N, VC, kPreP>, g.nb, N * N, 0, st, a.pdl, x1, b, g, a);
-    case kPreS: return launch_dependent(jacobi_zero_push_kernel<T, N, VC, kPreS>, g.nb, N * N, 0, st, a.pdl, x1, b, g, a);
-    case kPreCopy: return launch_dependent(jacobi_zero_push_kernel<T, N, VC, kPreCopy>, g.nb, N * N, 0, st, a.pdl, x1, b, g, a);
-    default: return launch_dependent(jacobi_zero_push_kernel<T, N, VC, kPreNone>, g.nb, N * N, 0, st, a.pdl, x1, b, g, a);
+    case kPreP: return launch_dependent(jacobi_zero_push_kernel<T, N, VC, kPreP>, g.nb, N * N, 0, st, a.pdl, 1, x1, b, g, a);
+    case kPreS: return launch_dependent(jacobi_zero_push_kernel<T, N, VC, kPreS>, g.nb, N * N, 0, st, a.pdl, 1, x1, b, g, a);
+    case kPreCopy: return launch_dependent(jacobi_zero_push_kernel<T, N, VC, kPreCopy>, g.nb, N * N, 0, st, a.pdl, 1, x1, b, g, a);
+    default: return launch_dependent(jacobi_zero_push_kernel<T, N, VC, kPreNone>, g.nb, N * N, 0, st, a.pdl, 1, x1, b, g, a);
   }
 }
 
@@ -609,6 +613,13 @@ __global__ void __launch_bounds__(N * N / CPT, sizeof(T) == 4 ? (CPT >= 4 ? 4 : 
 // then does the rest (edges, unfed faces, the other level-change entries).  ZERO: x0 == 0, only b is streamed.  PRE (with ZERO): b made
 // in the same pass from the BiCGSTAB vectors streamed instead (JacPre, the
 // operations of kr_p / kr_s) and written back.
+//
+// SPLIT: a thread-block cluster of 2, 4 or 8 CTAs takes a block, each its share
+// of the planes, and after a cluster barrier (every x1 plane is then in its brick,
+// seen by the whole cluster) its share of the tail; x faces' ghosts are then all
+// pushed as computed or in the tail.  One CTA per block leaves most of the chip
+// idle for a few dozen blocks of 32^3, and for a few hundred some SMs hold one
+// block more than others (jacobi_split).
 template <int PRE>
 __host__ __device__ constexpr int jac_pre_fields() { return PRE == kPreP ? 3 : PRE == kPreS ? 2 : 1; }
 
@@ -622,7 +633,8 @@ struct JacStream {
   static constexpr int MINB = stream_minb<SMEM + 64, (NT_ == 256 ? 6 : 2048 / NT_)>();
 };
 
-template <typename T, int N, int VC, int S, bool RES, bool ZERO, int NT_ = 256, int PRE = 0>
+template <typename T, int N, int VC, int S, bool RES, bool ZERO, int NT_ = 256, int PRE = 0,
+          bool SPLIT = false>
 __global__ void __launch_bounds__(NT_, (JacStream<T, N, VC, S, RES, ZERO, NT_, PRE>::MINB))
     jacobi_stream_push_kernel(const T* __restrict__ X0, T* __restrict__ X1,
                               const T* Bv, Geom g, JacArgs<T> a) {
@@ -640,15 +652,19 @@ __global__ void __launch_bounds__(NT_, (JacStream<T, N, VC, S, RES, ZERO, NT_, P
   // for the last three planes (xface[side][plane % 3][j][column]); the tail
   // makes the rest.  Up to kXle such entries (2:1 balance gives at most 8:
   // four finer neighbours on each x face).
-  constexpr bool XW = sizeof(T) == 4 && VC == 1;
+  constexpr bool XW = sizeof(T) == 4 && VC == 1 && !SPLIT;
   constexpr int kXle = 12;
   __shared__ float xface[XW ? 2 * 3 * N * 2 : 1];
   __shared__ VcTask xle[XW ? kXle : 1];
   __shared__ int nxle;
   griddep_launch_dependents();
   griddep_wait();
-  const int b = blockIdx.x, tid = threadIdx.x, w = tid >> 5, lane = tid & 31;
-  const int64_t base = (int64_t)b * g.bstride;
+  static_assert(!SPLIT || !RES, "the residual's sum is one CTA's");
+  const int ranks = SPLIT ? a.ranks : 1, rank = SPLIT ? blockIdx.x % ranks : 0;
+  const int b = SPLIT ? blockIdx.x / ranks : blockIdx.x;
+  const int np = SPLIT ? N / ranks : N, z0 = rank * np;  // planes of this CTA
+  const int tid = threadIdx.x, w = tid >> 5, lane = tid & 31;
+  const int64_t base = (int64_t)b * g.bstride + (int64_t)z0 * LXY;
   // the update's scalars; a finished segment's blocks change nothing (their
   // x1 is never read: no face joins two segments)
   T s_beta = T(0), s_ng = T(0), s_na = T(0);
@@ -659,7 +675,7 @@ __global__ void __launch_bounds__(NT_, (JacStream<T, N, VC, S, RES, ZERO, NT_, P
     s_ng = (T)(-sg.gamma);
     s_na = (T)(-sg.alpha);
   }
-  R ring(smraw);
+  R ring(smraw, np);
   constexpr int NB = jac_pre_fields<PRE>();
   const T* C[NB];
   if (PRE == kPreP) { C[0] = a.pre.r; C[1] = Bv; C[NB - 1] = a.pre.q; }
@@ -772,6 +788,7 @@ __global__ void __launch_bounds__(NT_, (JacStream<T, N, VC, S, RES, ZERO, NT_, P
   auto put = [&](int m, int c, T v) {
     const int j = j0 + c * JSTEP;
     X1[base + (int64_t)(VC + m) * LXY + o[c]] = v;
+    if (SPLIT) m += z0;  // the block's plane
     if (XW && xcol >= 0)
       xface[((xcol >> 1) * 3 + m % 3) * 2 * N + j * 2 + (xcol & 1)] = (float)v;
     if (xdst) xdst[BL::at(xg, j, m)] = v;
@@ -848,8 +865,9 @@ __global__ void __launch_bounds__(NT_, (JacStream<T, N, VC, S, RES, ZERO, NT_, P
         const T* bp = ring.cp(ZERO ? m : m + 1, 0);
         T* out = X1 + base + (int64_t)(VC + m) * LXY;
         T* bout = const_cast<T*>(Bv) + base + (int64_t)(VC + m) * LXY;
-        const int zd = m < VC ? zlo : (m >= N - VC ? zhi : -1);
-        const int zg = m < VC ? N + m : m - N;
+        const int mz = m + z0;  // the block's plane
+        const int zd = mz < VC ? zlo : (mz >= N - VC ? zhi : -1);
+        const int zg = mz < VC ? N + mz : mz - N;
 #pragma unroll
         for (int c = 0; c < CPT; c++) {
           const int q = o[c];
@@ -895,13 +913,18 @@ __global__ void __launch_bounds__(NT_, (JacStream<T, N, VC, S, RES, ZERO, NT_, P
           const int j = j0 + c * JSTEP;
           if (XW && xcol >= 0)
             xface[((xcol >> 1) * 3 + m % 3) * 2 * N + j * 2 + (xcol & 1)] = (float)v;
-          if (xdst) xdst[BL::at(xg, j, m)] = v;
-          if (c == 0 && ylo >= 0) X1[(int64_t)ylo * g.bstride + BL::at(i0, N + j, m)] = v;
-          if (c == CPT - 1 && yhi >= 0) X1[(int64_t)yhi * g.bstride + BL::at(i0, j - N, m)] = v;
+          if (xdst) xdst[BL::at(xg, j, mz)] = v;
+          if (c == 0 && ylo >= 0) X1[(int64_t)ylo * g.bstride + BL::at(i0, N + j, mz)] = v;
+          if (c == CPT - 1 && yhi >= 0) X1[(int64_t)yhi * g.bstride + BL::at(i0, j - N, mz)] = v;
           if (zd >= 0) X1[(int64_t)zd * g.bstride + BL::at(i0, j, zg)] = v;
         }
       });
     }
+  }
+  if constexpr (SPLIT) {
+    // arrives whatever became of this CTA's copies
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;"
+                 ::: "memory");
   }
   if (!ok) return;  // a copy never arrived: the error word says so
   xlev(N);  // the walk's last barrier made planes N-2 and N-1 visible
@@ -916,14 +939,21 @@ __global__ void __launch_bounds__(NT_, (JacStream<T, N, VC, S, RES, ZERO, NT_, P
     }
   }
   // the walk's last barrier made the block's x1 interior visible to the CTA
-  jacobi_push_tail<T, N, VC, NT, 4, false>(X0, X1, g, a, b, tid, ZERO, nxl);
+  jacobi_push_tail<T, N, VC, NT, 4, false>(X0, X1, g, a, b, tid, ZERO, nxl, nullptr, rank, ranks);
 }
 
-template <typename T, int N, int VC, int S, bool RES, bool ZERO, int PRE = 0>
-static cudaError_t jacobi_stream_launch_one(const T* x0, T* x1, const T* b, const Geom& g,
-                                            const JacArgs<T>& a, cudaStream_t st) {
+// CTAs per 32^3 block of the streamed kernel.
+inline int jacobi_split(int nb) {
+  int r = 1;
+  while (r < 8 && nb * r < kSplitCtas) r *= 2;
+  return r;
+}
+
+template <typename T, int N, int VC, int S, bool RES, bool ZERO, int PRE, bool SPLIT>
+static cudaError_t jacobi_stream_launch_as(const T* x0, T* x1, const T* b, const Geom& g,
+                                           const JacArgs<T>& a, cudaStream_t st) {
   using JS = JacStream<T, N, VC, S, RES, ZERO, 256, PRE>;
-  auto kern = jacobi_stream_push_kernel<T, N, VC, S, RES, ZERO, 256, PRE>;
+  auto kern = jacobi_stream_push_kernel<T, N, VC, S, RES, ZERO, 256, PRE, SPLIT>;
   // set once per process (not a stream operation; runs before any CUDA-graph
   // capture of these launches)
   static bool attr_set = false;
@@ -936,7 +966,19 @@ static cudaError_t jacobi_stream_launch_one(const T* x0, T* x1, const T* b, cons
     if (e != cudaSuccess) return e;
     attr_set = true;
   }
-  return launch_dependent(kern, g.nb, JS::NT, JS::SMEM, st, a.pdl, x0, x1, b, g, a);
+  return launch_dependent(kern, g.nb * (SPLIT ? a.ranks : 1), JS::NT, JS::SMEM, st, a.pdl,
+                          SPLIT ? a.ranks : 1, x0, x1, b, g, a);
+}
+
+template <typename T, int N, int VC, int S, bool RES, bool ZERO, int PRE = 0>
+static cudaError_t jacobi_stream_launch_one(const T* x0, T* x1, const T* b, const Geom& g,
+                                            JacArgs<T> a, cudaStream_t st) {
+  a.ranks = RES ? 1 : jacobi_split(g.nb);
+  if constexpr (!RES) {
+    if (a.ranks > 1)
+      return jacobi_stream_launch_as<T, N, VC, S, false, ZERO, PRE, true>(x0, x1, b, g, a, st);
+  }
+  return jacobi_stream_launch_as<T, N, VC, S, RES, ZERO, PRE, false>(x0, x1, b, g, a, st);
 }
 
 // Ring depths of the streamed Jacobi (74 KB of shared memory, 3 CTAs per
@@ -998,7 +1040,7 @@ static cudaError_t jacobi_tile_launch(const T* x0, T* x1, const T* b, const Geom
     if (e != cudaSuccess) return e;
     attr_set[ki] = true;
   }
-  return launch_dependent(kern, g.nb, L::NT, L::SMEM, st, a.pdl, x0, x1, b, g, a);
+  return launch_dependent(kern, g.nb, L::NT, L::SMEM, st, a.pdl, 1, x0, x1, b, g, a);
 }
 
 template <typename T, int N, int VC>
@@ -1030,7 +1072,7 @@ cudaError_t launch_jacobi_fused_impl(const T* x0, T* x1, const T* b, const Geom&
     // 32^3: push form only
     if (ghost_mode != kGhostPush && ghost_mode != kGhostPushZero) return cudaErrorInvalidValue;
     JacArgs<T> a{0, cf, omega, bc, push, partial, err, ghost_mode == kGhostPushZero ? 1 : 0,
-                 pre ? *pre : JacPre<T>{kPreNone, nullptr, nullptr, KSegs{}}, pdl};
+                 pre ? *pre : JacPre<T>{kPreNone, nullptr, nullptr, KSegs{}}, 1, pdl};
     const bool streamed = plane_stream_enabled() && stream_aligned<T>(g, x0, b) &&
                           (!pre || (stream_aligned<T>(g, pre->r, pre->q ? pre->q : pre->r)));
     if (a.pre.kind != kPreNone && !streamed) return cudaErrorNotSupported;
@@ -1044,7 +1086,7 @@ cudaError_t launch_jacobi_fused_impl(const T* x0, T* x1, const T* b, const Geom&
   if (ghost_mode == kGhostPushZero) {
     if (partial) return cudaErrorInvalidValue;
     JacArgs<T> a{0, cf, omega, bc, push, nullptr, err, 1,
-                 pre ? *pre : JacPre<T>{kPreNone, nullptr, nullptr, KSegs{}}, pdl};
+                 pre ? *pre : JacPre<T>{kPreNone, nullptr, nullptr, KSegs{}}, 1, pdl};
     T* bw = const_cast<T*>(b);  // written only where pre makes it
     if (g.nx == 16)
       return g.vc == 1 ? jacobi_zero_push_launch<T, 16, 1>(x1, bw, g, a, st)
@@ -1068,7 +1110,7 @@ cudaError_t launch_jacobi_fused_impl(const T* x0, T* x1, const T* b, const Geom&
   const bool pl = ghost_mode != kGhostPush;
   const bool close = ghost_mode == kGhostPullClose || ghost_mode == kGhostAsIsClose;
   JacArgs<T> a{ghost_mode == kGhostPull || ghost_mode == kGhostPullClose ? 1 : 0, cf, omega, bc, push, partial, err, 0,
-               JacPre<T>{kPreNone, nullptr, nullptr, KSegs{}}, pdl};
+               JacPre<T>{kPreNone, nullptr, nullptr, KSegs{}}, 1, pdl};
   if (g.nx == 16)
     return g.vc == 1 ? jacobi_tile_launch<T, 16, 1>(x0, x1, b, g, a, pl, close, st)
                      : jacobi_tile_launch<T, 16, 2>(x0, x1, b, g, a, pl, close, st);

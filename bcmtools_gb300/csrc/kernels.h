@@ -92,6 +92,9 @@ struct PushTable {
 };
 
 
+// Fewest CTAs the streamed 32^3 kernels should have: below, a block's planes are
+// split over a cluster of them.
+constexpr int kSplitCtas = 152 * 4;
 constexpr size_t kSorMaxSmem = 200 * 1024;
 // Dynamic shared memory one CTA may use (227 KB on sm_100-class GPUs).
 constexpr size_t kPipeMaxSmem = 227 * 1024;
@@ -301,17 +304,34 @@ inline bool kr_dependent(size_t es, const Geom& g) {
   return es == 4 && (g.nx * g.ny * g.nz <= 4096 || g.nb >= 2 * 3 * 152);
 }
 
+// Parts of a block's planes that the kernels with inner products take as CTAs of
+// their own in FP64 and for coefficient fields: two thousand cells or more and
+// four planes, at most four parts.  They are bound by the FP64 pipe (or by the
+// bytes in flight), so a mesh of a few hundred blocks should not leave an SM with
+// three blocks beside one with two.  The parts' sums are added in order, and the
+// split depends on the block's shape alone: a system's sums are the same alone
+// and among others.
+inline int kr_parts(const Geom& g) {
+  const int by_cells = g.nx * g.ny * g.nz / 2048, by_planes = g.nz / 4;
+  const int n = by_cells < by_planes ? by_cells : by_planes;
+  return n < 1 ? 1 : n > 4 ? 4 : n;
+}
+constexpr int kKrMaxParts = 4;
+
 // Device-resident BiCGSTAB iteration (krylov.cu): see krylov.cuh.
 template <typename T>
 cudaError_t launch_kr_p(T* p, const T* r, const T* q, const Geom& g, KSegs S, cudaStream_t st);
 template <typename T>
 cudaError_t launch_kr_s(T* s, const T* r, const T* q, const Geom& g, KSegs S, cudaStream_t st);
+// parts: partial sums per block (1 or kr_parts), part p of block b at
+// partial[b * parts + p], the second sums nb * parts further on.
 template <typename T>
 cudaError_t launch_kr_ax(T* out, const T* x, Op<T> op, const T* y0, int ndot, const Geom& g,
-                         KSegs S, double* partial, int* err, cudaStream_t st);
+                         int parts, KSegs S, double* partial, int* err, cudaStream_t st);
 template <typename T>
 cudaError_t launch_kr_xr(T* x, T* r, const T* p_, const T* s_, const T* s, const T* t,
-                         const T* r0, const Geom& g, KSegs S, double* partial, int* err, cudaStream_t st);
+                         const T* r0, const Geom& g, int parts, KSegs S, double* partial, int* err,
+                         cudaStream_t st);
 // A preconditioner's pass from x0 = 0 on blocks of any shape or coefficient
 // fields: x1's interior from b, or from b made of the BiCGSTAB vectors (pre).
 template <typename T>
@@ -322,8 +342,9 @@ cudaError_t launch_kr_dot2(const T* x, const T* y, const T* u, const T* v, const
                            double* partial, cudaStream_t st);
 template <typename T>
 cudaError_t launch_kr_best(T* xbest, const T* x, const Geom& g, KSegs S, cudaStream_t st);
-cudaError_t launch_kr_scalar(const double* partial, int nb, KSegs S, int stage, int max_iter,
-                             double eps2, int keep_best, bool dependent, cudaStream_t st);
+cudaError_t launch_kr_scalar(const double* partial, int nb, int parts, KSegs S, int stage,
+                             int max_iter, double eps2, int keep_best, bool dependent,
+                             cudaStream_t st);
 cudaError_t launch_kr_segsum(const double* partial, int nb, KSegs S, double* out,
                              cudaStream_t st);
 template <typename T>

@@ -45,15 +45,16 @@ namespace bcmg {
 // behind it: on 4432 blocks of 16^3 the x/r update ran at 40 % of the copy
 // bandwidth with one plane at a time).  Columns and planes in the same order,
 // so sums keep their bits.
+// Planes [z0, z1).
 template <int N, int U, class F>
-__device__ __forceinline__ void kr_walk(const Geom& g, F&& f) {
+__device__ __forceinline__ void kr_walk(const Geom& g, int z0, int z1, F&& f) {
   const int64_t base = (int64_t)blockIdx.x * g.bstride;
-  const int nx = N ? N : g.nx, nc = N ? N * N : g.nx * g.ny, nz = N ? N : g.nz;
+  const int nx = N ? N : g.nx, nc = N ? N * N : g.nx * g.ny;
   for (int ij = threadIdx.x; ij < nc; ij += blockDim.x) {
-    int64_t o = base + g.at(ij % nx, ij / nx, 0);
-    int k = 0;
-    for (; k + U <= nz; k += U, o += (int64_t)U * g.sz) f(o, std::integral_constant<int, U>{});
-    for (; k < nz; k++, o += g.sz) f(o, std::integral_constant<int, 1>{});
+    int64_t o = base + g.at(ij % nx, ij / nx, z0);
+    int k = z0;
+    for (; k + U <= z1; k += U, o += (int64_t)U * g.sz) f(o, std::integral_constant<int, U>{});
+    for (; k < z1; k++, o += g.sz) f(o, std::integral_constant<int, 1>{});
   }
 }
 
@@ -89,7 +90,7 @@ __global__ void __launch_bounds__(kr_nt<N>(), (kr_minb<T, N, false>())) kr_s_ker
 template <typename T, int N, bool CC, int NDOT>
 __global__ void __launch_bounds__(kr_nt<N>(), (CC ? kr_minb<T, N, true>() : 768 / kr_nt<N>())) kr_ax_kernel(
     T* __restrict__ out, const T* __restrict__ x, const T* __restrict__ cf8, Op<T> op,
-    const T* __restrict__ y0, Geom g, KSegs S, double* __restrict__ partial) {
+    const T* __restrict__ y0, Geom g, int zc, KSegs S, double* __restrict__ partial) {
   __shared__ double red[NDOT * kr_nt<N>()];
   griddep_launch_dependents();
   griddep_wait();
@@ -103,7 +104,10 @@ __global__ void __launch_bounds__(kr_nt<N>(), (CC ? kr_minb<T, N, true>() : 768 
   const int sy = g.sy, sz = g.sz;
   DotAcc<T> a0, a1;
   constexpr int U = CC && sizeof(T) == 4 && N != 32 ? 4 : 2;
-  kr_walk<N, U>(g, [&](int64_t o0, auto vt) {
+  // all planes in FP32 with constant coefficients (zc is nz there)
+  constexpr bool PARTS = !CC || sizeof(T) == 8;
+  const int nz = N ? N : g.nz, z0 = PARTS ? blockIdx.y * zc : 0;
+  kr_walk<N, U>(g, z0, PARTS ? min(nz, z0 + zc) : nz, [&](int64_t o0, auto vt) {
     constexpr int V = decltype(vt)::value;
     T w[V], e[V], s[V], n[V], m[V], u[V], xc[V], y[V], cf[CC ? 1 : V][7];
 #pragma unroll
@@ -140,8 +144,9 @@ __global__ void __launch_bounds__(kr_nt<N>(), (CC ? kr_minb<T, N, true>() : 768 
   double v0 = a0.value(), v1 = NDOT == 2 ? a1.value() : 0.0;
   kr_block_sums<NDOT>(v0, v1, red);
   if (threadIdx.x == 0) {
-    partial[b] = v0;
-    if (NDOT == 2) partial[g.nb + b] = v1;
+    const int at = b * gridDim.y + blockIdx.y;
+    partial[at] = v0;
+    if (NDOT == 2) partial[g.nb * gridDim.y + at] = v1;
   }
 }
 
@@ -163,21 +168,21 @@ struct AxStream {
 // down instead of going on.
 template <int NDOT, typename T>
 __device__ __forceinline__ void kr_ax_finish(bool ok, const DotAcc<T>& a0, const DotAcc<T>& a1,
-                                             double* red, double* __restrict__ partial, int b,
-                                             int nb) {
+                                             double* red, double* __restrict__ partial, int at,
+                                             int n) {
   const double nan = __longlong_as_double(0x7ff8000000000000ll);
   double v0 = ok ? a0.value() : nan, v1 = NDOT == 2 && ok ? a1.value() : nan;
   kr_block_sums<NDOT>(v0, v1, red);
   if (threadIdx.x == 0) {
-    partial[b] = v0;
-    if (NDOT == 2) partial[nb + b] = v1;
+    partial[at] = v0;
+    if (NDOT == 2) partial[n + at] = v1;
   }
 }
 
 template <typename T, int N, int VC, int NDOT, int S, int NT_ = 256>
 __global__ void __launch_bounds__(NT_, (AxStream<T, N, VC, S, NT_>::MINB)) kr_ax_stream_kernel(
     T* __restrict__ out, const T* __restrict__ x, const T* __restrict__ cf8,
-    const T* __restrict__ y0, Geom g, KSegs S_, double* __restrict__ partial, int* err) {
+    const T* __restrict__ y0, Geom g, int zc, KSegs S_, double* __restrict__ partial, int* err) {
   using AS = AxStream<T, N, VC, S, NT_>;
   using R = typename AS::R;
   constexpr int NT = AS::NT, CPT = N * N / NT, LX = R::LX, LXY = R::LXY;
@@ -189,8 +194,10 @@ __global__ void __launch_bounds__(NT_, (AxStream<T, N, VC, S, NT_>::MINB)) kr_ax
   griddep_wait();
   const int b = blockIdx.x, tid = threadIdx.x;
   if (S_.seg[kseg_of(S_, b)].status != kRunning) return;
-  const int64_t base = (int64_t)b * g.bstride;
-  R ring(smraw);
+  // FP64: planes [blockIdx.y zc, + zc) of the block (zc divides N)
+  const int z0 = sizeof(T) == 8 ? blockIdx.y * zc : 0;
+  const int64_t base = (int64_t)b * g.bstride + (int64_t)z0 * LXY;
+  R ring(smraw, sizeof(T) == 8 ? zc : N);
   const T* C[1] = {y0};
   if (tid == 0) ring.start(x, C, base);
   T c[7];
@@ -229,7 +236,7 @@ __global__ void __launch_bounds__(NT_, (AxStream<T, N, VC, S, NT_>::MINB)) kr_ax
         }
         sp.shift();
       });
-      kr_ax_finish<NDOT>(ok, a0, a1, red, partial, b, g.nb);
+      kr_ax_finish<NDOT>(ok, a0, a1, red, partial, b * gridDim.y + blockIdx.y, g.nb * gridDim.y);
       return;
     }
   }
@@ -254,12 +261,13 @@ __global__ void __launch_bounds__(NT_, (AxStream<T, N, VC, S, NT_>::MINB)) kr_ax
       if (NDOT == 2) a1.add(a, a);
     }
   });
-  kr_ax_finish<NDOT>(ok, a0, a1, red, partial, b, g.nb);
+  kr_ax_finish<NDOT>(ok, a0, a1, red, partial, b * gridDim.y + blockIdx.y, g.nb * gridDim.y);
 }
 
 template <typename T, int N, int VC, int NDOT, int S>
 static cudaError_t kr_ax_stream_one(T* out, const T* x, const T* cf8, const T* y0, const Geom& g,
-                                    KSegs S_, double* partial, int* err, cudaStream_t st) {
+                                    int parts, KSegs S_, double* partial, int* err,
+                                    cudaStream_t st) {
   using AS = AxStream<T, N, VC, S>;
   auto kern = kr_ax_stream_kernel<T, N, VC, NDOT, S>;
   // set once per process (not a stream operation; runs before any CUDA-graph
@@ -274,7 +282,8 @@ static cudaError_t kr_ax_stream_one(T* out, const T* x, const T* cf8, const T* y
     if (e != cudaSuccess) return e;
     attr_set = true;
   }
-  return launch_dependent(kern, g.nb, AS::NT, AS::SMEM, st, kr_dependent(sizeof(T), g), out, x, cf8, y0, g, S_, partial, err);
+  return launch_dependent(kern, dim3(g.nb, parts), AS::NT, AS::SMEM, st, kr_dependent(sizeof(T), g), 1, out, x,
+                          cf8, y0, g, N / parts, S_, partial, err);
 }
 
 // Ring depths: 32^3 4 slots (FP32: 6 CTAs per SM, FP64: 3); 16^3 8 (FP32)
@@ -283,11 +292,11 @@ static cudaError_t kr_ax_stream_one(T* out, const T* x, const T* cf8, const T* y
 // 394 for the column walk.
 template <typename T, int N, int VC>
 static cudaError_t kr_ax_stream(T* out, const T* x, const T* cf8, const T* y0, int ndot,
-                                const Geom& g, KSegs S_, double* partial, int* err,
+                                const Geom& g, int parts, KSegs S_, double* partial, int* err,
                                 cudaStream_t st) {
   constexpr int SS = N == 32 ? 4 : (sizeof(T) == 4 ? 8 : 6);
-  return ndot == 2 ? kr_ax_stream_one<T, N, VC, 2, SS>(out, x, cf8, y0, g, S_, partial, err, st)
-                   : kr_ax_stream_one<T, N, VC, 1, SS>(out, x, cf8, y0, g, S_, partial, err, st);
+  return ndot == 2 ? kr_ax_stream_one<T, N, VC, 2, SS>(out, x, cf8, y0, g, parts, S_, partial, err, st)
+                   : kr_ax_stream_one<T, N, VC, 1, SS>(out, x, cf8, y0, g, parts, S_, partial, err, st);
 }
 
 // kr_xr for cubic 16^3 / 32^3 blocks: the six fields it reads streamed
@@ -376,7 +385,7 @@ static cudaError_t kr_xr_stream(T* x, T* r, const T* p_, const T* s_, const T* s
     if (e != cudaSuccess) return e;
     attr_set = true;
   }
-  return launch_dependent(kern, g.nb, XS::NT, XS::SMEM, st, kr_dependent(sizeof(T), g), x, r, p_, s_, s, t, r0, g, S_,
+  return launch_dependent(kern, g.nb, XS::NT, XS::SMEM, st, kr_dependent(sizeof(T), g), 1, x, r, p_, s_, s, t, r0, g, S_,
                           partial, err);
 }
 
@@ -386,7 +395,7 @@ static cudaError_t kr_xr_stream(T* x, T* r, const T* p_, const T* s_, const T* s
 template <typename T, int N>
 __global__ void __launch_bounds__(kr_nt<N>(), (kr_minb<T, N, true>())) kr_xr_kernel(
     T* __restrict__ x, T* __restrict__ r, const T* __restrict__ p_, const T* __restrict__ s_,
-    const T* __restrict__ s, const T* __restrict__ t, const T* __restrict__ r0, Geom g, KSegs S,
+    const T* __restrict__ s, const T* __restrict__ t, const T* __restrict__ r0, Geom g, int zc, KSegs S,
     double* __restrict__ partial) {
   __shared__ double red[2 * kr_nt<N>()];
   griddep_launch_dependents();
@@ -396,7 +405,9 @@ __global__ void __launch_bounds__(kr_nt<N>(), (kr_minb<T, N, true>())) kr_xr_ker
   if (sg.status != kRunning) return;
   const T al = (T)sg.alpha, gm = (T)sg.gamma, ngm = (T)(-sg.gamma);
   DotAcc<T> a0, a1;
-  kr_walk<N, (sizeof(T) == 4 && N != 32 ? 4 : 2)>(g, [&](int64_t o0, auto vt) {
+  constexpr bool PARTS = N == 0 || sizeof(T) == 8;  // else zc is nz
+  const int nz = N ? N : g.nz, z0 = PARTS ? blockIdx.y * zc : 0;
+  kr_walk<N, (sizeof(T) == 4 && N != 32 ? 4 : 2)>(g, z0, PARTS ? min(nz, z0 + zc) : nz, [&](int64_t o0, auto vt) {
     constexpr int V = decltype(vt)::value;
     T pv[V], sv_[V], xv[V], tv[V], sv[V], r0v[V];
 #pragma unroll
@@ -422,8 +433,9 @@ __global__ void __launch_bounds__(kr_nt<N>(), (kr_minb<T, N, true>())) kr_xr_ker
   double v0 = a0.value(), v1 = a1.value();
   kr_block_sums<2>(v0, v1, red);
   if (threadIdx.x == 0) {
-    partial[b] = v0;
-    partial[g.nb + b] = v1;
+    const int at = b * gridDim.y + blockIdx.y;
+    partial[at] = v0;
+    partial[g.nb * gridDim.y + at] = v1;
   }
 }
 
@@ -435,7 +447,7 @@ __global__ void __launch_bounds__(kr_nt<N>(), (kr_minb<T, N, true>())) kr_dot2_k
     const T* __restrict__ v, Geom g, double* __restrict__ partial) {
   __shared__ double red[2 * kr_nt<N>()];
   DotAcc<T> a0, a1;
-  kr_walk<N, (sizeof(T) == 4 && N != 32 ? 4 : 2)>(g, [&](int64_t o0, auto vt) {
+  kr_walk<N, (sizeof(T) == 4 && N != 32 ? 4 : 2)>(g, 0, N ? N : g.nz, [&](int64_t o0, auto vt) {
     constexpr int V = decltype(vt)::value;
     T xv[V], yv[V], uv[V], vv[V];
 #pragma unroll
@@ -539,9 +551,9 @@ cudaError_t launch_kr_zero_pass(T* x1, T* b, const JacPre<T>& pre, const Op<T>& 
   const dim3 grid(g.nb, (g.nz + zc - 1) / zc);
 #define Z_(PRE)                                                                            \
   if (op.cc)                                                                               \
-    return launch_dependent(kr_zero_pass_kernel<T, true, PRE>, grid, nt, 0, st, kr_dependent(sizeof(T), g), x1, b, pre, op, g, omega, zc);   \
+    return launch_dependent(kr_zero_pass_kernel<T, true, PRE>, grid, nt, 0, st, kr_dependent(sizeof(T), g), 1, x1, b, pre, op, g, omega, zc);   \
   else                                                                                     \
-    return launch_dependent(kr_zero_pass_kernel<T, false, PRE>, grid, nt, 0, st, kr_dependent(sizeof(T), g), x1, b, pre, op, g, omega, zc)
+    return launch_dependent(kr_zero_pass_kernel<T, false, PRE>, grid, nt, 0, st, kr_dependent(sizeof(T), g), 1, x1, b, pre, op, g, omega, zc)
   switch (pre.kind) {
     case kPreP: Z_(kPreP); break;
     case kPreS: Z_(kPreS); break;
@@ -642,7 +654,7 @@ __device__ __forceinline__ void kr_segment_sums(const double* __restrict__ parti
 // Per segment: reduce its blocks' partial sums (fixed order), then one stage
 // of the scalar recurrence of ILS3D.h:663-844 in FP64.
 __global__ void __launch_bounds__(256) kr_scalar_kernel(const double* __restrict__ partial, int nb,
-                                                        KSegs S, int stage, int max_iter,
+                                                        int parts, KSegs S, int stage, int max_iter,
                                                         double eps2, int keep_best) {
   griddep_launch_dependents();
   griddep_wait();
@@ -653,7 +665,7 @@ __global__ void __launch_bounds__(256) kr_scalar_kernel(const double* __restrict
   const int f0 = S.seg_first ? S.seg_first[sgi] : 0;
   const int f1 = S.seg_first ? S.seg_first[sgi + 1] : nb;
   double v0, v1;
-  kr_segment_sums(partial, nb, f0, f1, red, v0, v1);
+  kr_segment_sums(partial, nb * parts, f0 * parts, f1 * parts, red, v0, v1);
   if (threadIdx.x != 0) return;
   const double fmin = (double)FLT_MIN;
   if (stage == KS_INIT) {
@@ -792,27 +804,29 @@ cudaError_t launch_kr_s(T* s, const T* r, const T* q, const Geom& g, KSegs S, cu
 
 template <typename T>
 cudaError_t launch_kr_ax(T* out, const T* x, Op<T> op, const T* y0, int ndot, const Geom& g,
-                         KSegs S, double* partial, int* err, cudaStream_t st) {
+                         int parts, KSegs S, double* partial, int* err, cudaStream_t st) {
   if (g.nb == 0) return cudaSuccess;
+  const int zc = (g.nz + parts - 1) / parts;
+  const dim3 grid(g.nb, parts);
   const bool cc = op.cc && op.cf8;
   if (cc && plane_stream_enabled() && (g.vc == 1 || g.vc == 2) &&
-      (g.nx == 16 || g.nx == 32) && stream_aligned<T>(g, x, y0) &&
+      (g.nx == 16 || g.nx == 32) && g.nz % parts == 0 && stream_aligned<T>(g, x, y0) &&
       (reinterpret_cast<uintptr_t>(out) % 16) == 0) {
     if (g.nx == 32)
-      return g.vc == 1 ? kr_ax_stream<T, 32, 1>(out, x, op.cf8, y0, ndot, g, S, partial, err, st)
-                       : kr_ax_stream<T, 32, 2>(out, x, op.cf8, y0, ndot, g, S, partial, err, st);
-    return g.vc == 1 ? kr_ax_stream<T, 16, 1>(out, x, op.cf8, y0, ndot, g, S, partial, err, st)
-                     : kr_ax_stream<T, 16, 2>(out, x, op.cf8, y0, ndot, g, S, partial, err, st);
+      return g.vc == 1 ? kr_ax_stream<T, 32, 1>(out, x, op.cf8, y0, ndot, g, parts, S, partial, err, st)
+                       : kr_ax_stream<T, 32, 2>(out, x, op.cf8, y0, ndot, g, parts, S, partial, err, st);
+    return g.vc == 1 ? kr_ax_stream<T, 16, 1>(out, x, op.cf8, y0, ndot, g, parts, S, partial, err, st)
+                     : kr_ax_stream<T, 16, 2>(out, x, op.cf8, y0, ndot, g, parts, S, partial, err, st);
   }
 #define C_(N)                                                                                     \
   if (cc && ndot == 2)                                                                            \
-    return launch_dependent(kr_ax_kernel<T, N, true, 2>, g.nb, kr_threads<N>(g), 0, st, kr_dependent(sizeof(T), g), out, x, op.cf8, op, y0, g, S, partial);                      \
+    return launch_dependent(kr_ax_kernel<T, N, true, 2>, grid, kr_threads<N>(g), 0, st, kr_dependent(sizeof(T), g), 1, out, x, op.cf8, op, y0, g, zc, S, partial);                      \
   else if (cc)                                                                                    \
-    return launch_dependent(kr_ax_kernel<T, N, true, 1>, g.nb, kr_threads<N>(g), 0, st, kr_dependent(sizeof(T), g), out, x, op.cf8, op, y0, g, S, partial);                      \
+    return launch_dependent(kr_ax_kernel<T, N, true, 1>, grid, kr_threads<N>(g), 0, st, kr_dependent(sizeof(T), g), 1, out, x, op.cf8, op, y0, g, zc, S, partial);                      \
   else if (ndot == 2)                                                                             \
-    return launch_dependent(kr_ax_kernel<T, N, false, 2>, g.nb, kr_threads<N>(g), 0, st, kr_dependent(sizeof(T), g), out, x, op.cf8, op, y0, g, S, partial);                     \
+    return launch_dependent(kr_ax_kernel<T, N, false, 2>, grid, kr_threads<N>(g), 0, st, kr_dependent(sizeof(T), g), 1, out, x, op.cf8, op, y0, g, zc, S, partial);                     \
   else                                                                                            \
-    return launch_dependent(kr_ax_kernel<T, N, false, 1>, g.nb, kr_threads<N>(g), 0, st, kr_dependent(sizeof(T), g), out, x, op.cf8, op, y0, g, S, partial)
+    return launch_dependent(kr_ax_kernel<T, N, false, 1>, grid, kr_threads<N>(g), 0, st, kr_dependent(sizeof(T), g), 1, out, x, op.cf8, op, y0, g, zc, S, partial)
   KR_DISPATCH(C_)
 #undef C_
   return cudaGetLastError();
@@ -820,17 +834,19 @@ cudaError_t launch_kr_ax(T* out, const T* x, Op<T> op, const T* y0, int ndot, co
 
 template <typename T>
 cudaError_t launch_kr_xr(T* x, T* r, const T* p_, const T* s_, const T* s, const T* t,
-                         const T* r0, const Geom& g, KSegs S, double* partial, int* err,
+                         const T* r0, const Geom& g, int parts, KSegs S, double* partial, int* err,
                          cudaStream_t st) {
   if (g.nb == 0) return cudaSuccess;
+  const int zc = (g.nz + parts - 1) / parts;
+  const dim3 grid(g.nb, parts);
   // 32^3 FP32: six planes a slot, 2 slots (4 CTAs per SM)
-  if (sizeof(T) == 4 && g.nx == 32 && (g.vc == 1 || g.vc == 2) && plane_stream_enabled() &&
+  if (sizeof(T) == 4 && parts == 1 && g.nx == 32 && (g.vc == 1 || g.vc == 2) && plane_stream_enabled() &&
       stream_aligned<T>(g, x, r) && stream_aligned<T>(g, p_, s_) && stream_aligned<T>(g, s, t) &&
       stream_aligned<T>(g, r0, r0))
     return g.vc == 1 ? kr_xr_stream<T, 32, 1, 2>(x, r, p_, s_, s, t, r0, g, S, partial, err, st)
                      : kr_xr_stream<T, 32, 2, 2>(x, r, p_, s_, s, t, r0, g, S, partial, err, st);
 #define C_(N) \
-  return launch_dependent(kr_xr_kernel<T, N>, g.nb, kr_threads<N>(g), 0, st, kr_dependent(sizeof(T), g), x, r, p_, s_, s, t, r0, g, S, partial)
+  return launch_dependent(kr_xr_kernel<T, N>, grid, kr_threads<N>(g), 0, st, kr_dependent(sizeof(T), g), 1, x, r, p_, s_, s, t, r0, g, zc, S, partial)
   KR_DISPATCH(C_)
 #undef C_
   return cudaGetLastError();
@@ -849,13 +865,14 @@ cudaError_t launch_kr_dot2(const T* x, const T* y, const T* u, const T* v, const
 template <typename T>
 cudaError_t launch_kr_best(T* xbest, const T* x, const Geom& g, KSegs S, cudaStream_t st) {
   if (g.nb == 0) return cudaSuccess;
-  return launch_dependent(kr_best_kernel<T>, g.nb, 256, 0, st, kr_dependent(sizeof(T), g), xbest, x, g, S);
+  return launch_dependent(kr_best_kernel<T>, g.nb, 256, 0, st, kr_dependent(sizeof(T), g), 1, xbest, x, g, S);
 }
 
-cudaError_t launch_kr_scalar(const double* partial, int nb, KSegs S, int stage, int max_iter,
-                             double eps2, int keep_best, bool dependent, cudaStream_t st) {
-  return launch_dependent(kr_scalar_kernel, S.nseg, 256, 0, st, dependent, partial, nb, S, stage, max_iter,
-                          eps2, keep_best);
+cudaError_t launch_kr_scalar(const double* partial, int nb, int parts, KSegs S, int stage,
+                             int max_iter, double eps2, int keep_best, bool dependent,
+                             cudaStream_t st) {
+  return launch_dependent(kr_scalar_kernel, S.nseg, 256, 0, st, dependent, 1, partial, nb, parts, S, stage,
+                          max_iter, eps2, keep_best);
 }
 
 cudaError_t launch_kr_segsum(const double* partial, int nb, KSegs S, double* out,
@@ -899,10 +916,10 @@ cudaError_t launch_kr_seg_acc(double* x64, const float* d32, const Geom& g32, co
 #define INST(T)                                                                                    \
   template cudaError_t launch_kr_p<T>(T*, const T*, const T*, const Geom&, KSegs, cudaStream_t);  \
   template cudaError_t launch_kr_s<T>(T*, const T*, const T*, const Geom&, KSegs, cudaStream_t);  \
-  template cudaError_t launch_kr_ax<T>(T*, const T*, Op<T>, const T*, int, const Geom&, KSegs,    \
-                                       double*, int*, cudaStream_t);                              \
+  template cudaError_t launch_kr_ax<T>(T*, const T*, Op<T>, const T*, int, const Geom&, int,      \
+                                       KSegs, double*, int*, cudaStream_t);                       \
   template cudaError_t launch_kr_xr<T>(T*, T*, const T*, const T*, const T*, const T*, const T*,  \
-                                       const Geom&, KSegs, double*, int*, cudaStream_t);          \
+                                       const Geom&, int, KSegs, double*, int*, cudaStream_t);     \
   template cudaError_t launch_kr_dot2<T>(const T*, const T*, const T*, const T*, const Geom&,     \
                                          double*, cudaStream_t);                                  \
   template cudaError_t launch_kr_zero_pass<T>(T*, T*, const JacPre<T>&, const Op<T>&, const Geom&, T,\

@@ -64,7 +64,6 @@ struct PlaneRing {
   static constexpr unsigned ROW_LO = VC * LX * sizeof(T) / 16 * 16;
   static constexpr unsigned ROW_HI = ((VC + N) * LX * sizeof(T) + 15) / 16 * 16;
   static constexpr unsigned RB = ROW_HI - ROW_LO;
-  static constexpr int NU = HX ? N + 2 : N;  // units per block
   static constexpr unsigned SLOT = (HX ? PB : 0) + NB * PB;
   static constexpr unsigned BAR_BYTES = 128;
   static constexpr size_t SMEM = BAR_BYTES + (size_t)S * SLOT;
@@ -78,9 +77,11 @@ struct PlaneRing {
 
   uint64_t* bar;
   unsigned char* slots;
+  int np;  // interior planes walked: N, or a part of the block's (base then starts there)
+  __device__ __forceinline__ int nu() const { return HX ? np + 2 : np; }  // units
 
-  __device__ __forceinline__ PlaneRing(unsigned char* smraw)
-      : bar(reinterpret_cast<uint64_t*>(smraw)), slots(smraw + BAR_BYTES) {}
+  __device__ __forceinline__ PlaneRing(unsigned char* smraw, int planes = N)
+      : bar(reinterpret_cast<uint64_t*>(smraw)), slots(smraw + BAR_BYTES), np(planes) {}
 
   // Plane of X held by unit u; plane of cell-only field f held by unit u.
   __device__ __forceinline__ const T* xp(int u) const {
@@ -94,14 +95,14 @@ struct PlaneRing {
   __device__ __forceinline__ void start(const T* X, const T* const* C, int64_t base) {
     for (int s = 0; s < S; s++) mbar_init(&bar[s], 1);
     mbar_fence_init();
-    for (int u = 0; u < S && u < NU; u++) issue(u, X, C, base);
+    for (int u = 0; u < S && u < nu(); u++) issue(u, X, C, base);
   }
 
   // Thread 0: unit u of the block whose brick starts at element `base`.
   __device__ __forceinline__ void issue(int u, const T* X, const T* const* C, int64_t base) {
     unsigned char* dst = slots + (u % S) * SLOT;
     const int z = HX ? VC - 1 + u : VC + u;  // brick plane
-    const bool cells = !HX || (u >= 1 && u <= N);
+    const bool cells = !HX || (u >= 1 && u <= np);
     const unsigned bytes = (HX ? PB : 0) + (cells ? NB * RB : 0);
     mbar_expect_tx(&bar[u % S], bytes);
     if (HX) bulk_g2s(dst, X + base + (int64_t)z * LXY, PB, &bar[u % S]);
@@ -183,9 +184,9 @@ struct ScaledPlanes {
     for (int k = 0; k < CPT; k++) {
       xu[k] = u[o[k]];
       pu[k] = __dmul_rn(c, xu[k]);
-      if (m + 1 < N) u[o[k]] = pu[k];
+      if (m + 1 < ring.np) u[o[k]] = pu[k];
     }
-    if (m + 1 < N) rim(u, c, tid);
+    if (m + 1 < ring.np) rim(u, c, tid);
   }
   // After plane m's cells: plane m+1 becomes the centre.  The proxy fence
   // orders this thread's stores to a slot before the bulk copy that refills
@@ -225,9 +226,10 @@ __device__ __forceinline__ bool plane_walk(PlaneRing<T, N, VC, S, HX, NB>& ring,
   using R = PlaneRing<T, N, VC, S, HX, NB>;
   // unit m+2 (HX) is waited for at plane m and issued at plane m+3-S: S >= 4
   static_assert(S >= (HX ? 4 : 2), "ring too shallow for the walk");
-  int issued = S < R::NU ? S : R::NU;
+  const int nu = ring.nu();
+  int issued = S < nu ? S : nu;
   bool ok = true;
-  for (int m = 0; m < N; m++) {
+  for (int m = 0; m < ring.np; m++) {
     if (tid == 0) {
       if (HX && m == 0) ok = ring.wait(0, err) && ring.wait(1, err);
       ok = ok && ring.wait(HX ? m + 2 : m, err);
@@ -237,7 +239,7 @@ __device__ __forceinline__ bool plane_walk(PlaneRing<T, N, VC, S, HX, NB>& ring,
       __syncthreads();
       return false;
     }
-    if (tid == 0 && m > 0 && m - 1 + S < R::NU) {
+    if (tid == 0 && m > 0 && m - 1 + S < nu) {
       ring.issue(m - 1 + S, X, C, base);
       issued = m + S;
     }

@@ -149,3 +149,64 @@ def test_jacobi_run_with_a_face_fed_in_part(gpu_ok, dt, n, vc, iters, push):
         m.vc_update(ref)
         m.dirichlet(ref, bct, bcv, 0)
     assert_bitexact(x.download(), ref, face_mask(n, vc), f"partly fed {dt} {n} {iters}")
+
+
+@pytest.mark.parametrize("dt", ["f32", "f64"])
+@pytest.mark.parametrize("vc", [1, 2])
+@pytest.mark.parametrize("copies", [1, 3, 6, 12, 50])
+def test_blocks_of_32_alone_and_among_others(gpu_ok, dt, vc, copies):
+    """The streamed 32^3 sweep splits a block over 8, 4, 2 or 1 CTAs by the number
+    of blocks (15 a copy here): every copy of a mesh in one block set gets the
+    field it gets alone, bit for bit, and the oracle's; so does its BiCGSTAB."""
+    from bcmtools_gb300.batch import Batch
+    from bcmtools_gb300.workloads import Workload
+    n = 32
+    rg = bg.RootGrid(1, 1, 1, root_length=1.0)
+    tree = bg.Octree.build(rg, bg.Divider.sphere_surface((0.3, 0.3, 0.3), 0.1, 2), "Z")
+    batch = Batch([Workload("copy", tree, n, vc)] * copies)
+    bm = batch.bm
+    bct, bcv = batch.set_dirichlet(0.25)
+    op = batch.laplace_op()
+    x, b = bm.setDataClass(dt, vc), bm.setDataClass(dt, vc)
+    rng = np.random.default_rng(9)
+    shape = (15,) + x.shape[1:]
+    a0, ab = rng.uniform(-1, 1, size=shape).astype(x.dtype), np.zeros(shape, x.dtype)
+    inner = (slice(None),) + (slice(vc, -vc),) * 3
+    ab[inner] = rng.uniform(-1, 1, size=ab[inner].shape)
+    x.upload(np.tile(a0, (copies, 1, 1, 1)))
+    b.upload(np.tile(ab, (copies, 1, 1, 1)))
+    bm.jacobi_run(op, x, b, 0.9, 3)
+    got = x.download()
+    for k in range(1, copies):
+        assert_bitexact(batch.instance(got, k), batch.instance(got, 0), what=f"copy {k}")
+    ld, nid, sf, _ = tree.neighbors()
+    m = po.OracleMesh(ld, nid, sf, n, vc)
+    cc = bg.laplace_coef(tree.cell_sizes(n))
+    ref, x1 = a0.copy(), np.zeros_like(a0)
+    for _ in range(3):
+        m.jacobi(x1, ref, ab, 0.9, cc=cc)
+        ref[inner] = x1[inner]
+        m.vc_update(ref)
+        m.dirichlet(ref, bct[:15], bcv[:15], 0)
+    mask = face_mask(n, vc)
+    if dt == "f64":
+        assert_bitexact(got[:15], ref, mask, "oracle")
+    else:  # C2F ghosts of FP32 fields: one ulp
+        d = np.abs(got[:15][:, mask].astype(np.float64) - ref[:, mask])
+        assert d.max() <= 1e-6 * np.abs(ref).max()
+    batch.set_segments()
+    bm.set_boundary(bct, np.zeros_like(bcv))
+    x.fill(0.0)
+    infos = bm.bicgstab(op, x, b, omega=0.8, n_pre=2, max_iter=5, eps=1e-12)
+    infos = infos if isinstance(infos, list) else [infos]
+    sol = x.download()
+    for k in range(1, copies):
+        assert_bitexact(batch.instance(sol, k)[inner], batch.instance(sol, 0)[inner], what=f"solve {k}")
+        assert infos[k].iterations == infos[0].iterations
+    one = bg.BlockManager(0)
+    one.register_octree(tree, n)
+    one.set_boundary(bct[:15], np.zeros((15, 6)))
+    y, c = one.setDataClass(dt, vc), one.setDataClass(dt, vc)
+    c.upload(ab)
+    one.bicgstab(one.op_const(cc), y, c, omega=0.8, n_pre=2, max_iter=5, eps=1e-12)
+    assert_bitexact(y.download()[inner], sol[:15][inner], what="solve alone")
