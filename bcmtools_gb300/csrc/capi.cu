@@ -622,7 +622,7 @@ static int finish_register(bcmg_ctx c, int nx, int ny, int nz) {
   c->nseg = 1;
   c->seg_first.assign({0, nb});
   CUDA_TRY(c, cudaSetDevice(c->device));
-  CUDA_TRY(c, cudaMalloc(&c->d_partial, (size_t)nb * sizeof(double)));
+  CUDA_TRY(c, cudaMalloc(&c->d_partial, (size_t)kKrMaxParts * nb * sizeof(double)));
   CUDA_TRY(c, cudaMalloc(&c->d_bczero, (size_t)nb * 6 * sizeof(double)));
   CUDA_TRY(c, cudaMemset(c->d_bczero, 0, (size_t)nb * 6 * sizeof(double)));
   CUDA_TRY(c, cudaMalloc(&c->d_bcval, (size_t)nb * 6 * sizeof(double)));
@@ -1629,29 +1629,37 @@ BCMG_API int bcmg_jacobi_sweep(bcmg_ctx c, int op, int x1, int x0, int b, double
   return jacobi_sweep(c, op, *f1, *f0, *fb, omega, S(c, st));
 }
 
-static int residual(bcmg_ctx c, int op, Field* out, Field& x, Field* b, int mode, cudaStream_t st) {
+// nsums (mode 2): the partial sums left for finish_reduce.
+static int residual(bcmg_ctx c, int op, Field* out, Field& x, Field* b, int mode, cudaStream_t st,
+                    int* nsums = nullptr) {
   Geom g = geom_of(c, x);
+  if (nsums) *nsums = c->nb;
   if (x.dtype == BCMG_F64) {
     Op<double> o;
     int rc = make_op(c, op, x, &o);
     if (rc) return rc;
+    // bulk copies read device memory only
+    const bool streamed = !x.host && !(b && b->host) && plane_stream_enabled() &&
+                          residual_streams(sizeof(double), o.cc != nullptr, g) &&
+                          stream_aligned<double>(g, x.d, b ? b->d : x.d);
+    if (nsums && streamed) *nsums = c->nb * kr_parts(g);
     LAUNCH(c, K_RESIDUAL, st, launch_residual<double>(out ? (double*)out->d : nullptr, (const double*)x.d,
-                                      b ? (const double*)b->d : nullptr, o, g, mode,
-                                      c->d_partial, st));
+                                      b ? (const double*)b->d : nullptr, o, g, mode, streamed,
+                                      c->d_partial, c->d_err, st));
   } else {
     Op<float> o;
     int rc = make_op(c, op, x, &o);
     if (rc) return rc;
     LAUNCH(c, K_RESIDUAL, st, launch_residual<float>(out ? (float*)out->d : nullptr, (const float*)x.d,
-                                     b ? (const float*)b->d : nullptr, o, g, mode, c->d_partial,
-                                     st));
+                                     b ? (const float*)b->d : nullptr, o, g, mode, false,
+                                     c->d_partial, c->d_err, st));
   }
   return BCMG_SUCCESS;
 }
 
-// Sum the per-block partials and bring the value to the host.
-static int finish_reduce(bcmg_ctx c, double* out, cudaStream_t st) {
-  LAUNCH(c, K_DOT, st, launch_reduce_final(c->d_partial, c->nb, c->d_scalar, st));
+// Sum the partials (one per block unless said) and bring the value to the host.
+static int finish_reduce(bcmg_ctx c, double* out, cudaStream_t st, int n = 0) {
+  LAUNCH(c, K_DOT, st, launch_reduce_final(c->d_partial, n ? n : c->nb, c->d_scalar, st));
   CUDA_TRY(c, cudaMemcpyAsync(c->h_scalar, c->d_scalar, sizeof(double), cudaMemcpyDeviceToHost, st));
   CUDA_TRY(c, cudaStreamSynchronize(st));
   *out = c->h_scalar[0];
@@ -1685,9 +1693,10 @@ BCMG_API int bcmg_calc_r2(bcmg_ctx c, int op, int x, int b, double* rr, void* st
   if (!c || !rr) return BCMG_USAGE;
   Field *fx = get_field(c, x), *fb = get_field(c, b);
   if (!same_shape(fx, fb)) return fail(c, BCMG_USAGE, "field mismatch");
-  int rc = residual(c, op, nullptr, *fx, fb, 2, S(c, st));
+  int nsums;
+  int rc = residual(c, op, nullptr, *fx, fb, 2, S(c, st), &nsums);
   if (rc) return rc;
-  return finish_reduce(c, rr, S(c, st));
+  return finish_reduce(c, rr, S(c, st), nsums);
 }
 
 BCMG_API int bcmg_dot(bcmg_ctx c, int x, int y, double* out, void* st) {
@@ -2037,8 +2046,9 @@ BCMG_API int bcmg_jacobi_solve(bcmg_ctx c, int op, int x, int b, double omega, i
     if ((rc = finish_fused(c, *fx, false, choice, stream))) return rc;
     if (!done) {
       count = max_iter;
-      if ((rc = residual(c, op, nullptr, *fx, fb, 2, stream))) return rc;
-      if ((rc = finish_reduce(c, &rr, stream))) return rc;
+      int nsums;
+      if ((rc = residual(c, op, nullptr, *fx, fb, 2, stream, &nsums))) return rc;
+      if ((rc = finish_reduce(c, &rr, stream, nsums))) return rc;
       const int cv = converged(rr, bb, eps, &res);
       if (cv > 0) status = BCMG_SUCCESS;
       if (cv < 0) status = BCMG_DIVERGED;
@@ -2060,8 +2070,9 @@ BCMG_API int bcmg_jacobi_solve(bcmg_ctx c, int op, int x, int b, double omega, i
     if (rc) return rc;
     std::swap(fx->d, fw->d);  // LSSwap
     if ((rc = impose(c, *fx, false, stream))) return rc;
-    if ((rc = residual(c, op, nullptr, *fx, fb, 2, stream))) return rc;
-    if ((rc = finish_reduce(c, &rr, stream))) return rc;
+    int nsums;
+    if ((rc = residual(c, op, nullptr, *fx, fb, 2, stream, &nsums))) return rc;
+    if ((rc = finish_reduce(c, &rr, stream, nsums))) return rc;
     int cv = converged(rr, bb, eps, &res);
     if (cv > 0) { status = BCMG_SUCCESS; break; }
     if (cv < 0) { status = BCMG_DIVERGED; break; }

@@ -188,41 +188,108 @@ __global__ void __launch_bounds__(N * N, (BrickStage<T, N, VC, true>::MIN_BLOCKS
   T* bp = bs + (VC + j) * LX + VC + i;
   T* gp = X1 + (int64_t)b * g.bstride + BL::at(i, j, 0);
   SqAcc<T> acc;
-  T xm = xc_p[-LXY], xc = xc_p[0];
   static_assert(N % 4 == 0, "cells in groups of four");
+  bool iso = false;
+  if constexpr (sizeof(T) == 8) {
+    // FP64, one coefficient for all six neighbours: each product formed once
+    // (stream.cuh), over the tile's interior -- nothing reads its raw values
+    // again but this thread's, which are in registers -- and for the x and y
+    // ghosts, whose raw values the ghost cells written below need, beside it.
+    // 15 operations a cell instead of 20, the same bits; the sweep is bound by the
+    // FP64 pipe.
+    iso = one_coefficient(c1, c2, c3, c4, c5, c6);
+    if (iso) {
+      T* gs = reinterpret_cast<T*>(smraw + L::G_OFF);
+      T* own = xs + BL::at(i, j, 0);
+      T xr[N];
 #pragma unroll
-  for (int k0 = 0; k0 < N; k0 += 4) {
-    // four cells: every load before the first store into b's area, so the
-    // loads overlap
-    T xw[4], xe[4], xs_[4], xn[4], xu[4], bv[4];
+      for (int k = 0; k < N; k++) {
+        xr[k] = own[k * LXY];
+        own[k * LXY] = xmul(c1, xr[k]);
+      }
+      gs[0 * NN + tid] = xmul(c1, xs[BL::at(-1, gpp, gq)]);
+      gs[1 * NN + tid] = xmul(c1, xs[BL::at(N, gpp, gq)]);
+      gs[2 * NN + tid] = xmul(c1, xs[BL::at(gpp, -1, gq)]);
+      gs[3 * NN + tid] = xmul(c1, xs[BL::at(gpp, N, gq)]);
+      T ym = xmul(c1, own[-LXY]);
+      const T ytop = xmul(c1, own[N * LXY]);
+      __syncthreads();
+      const T* pw = i > 0 ? own - 1 : gs + j;
+      const T* pe = i < N - 1 ? own + 1 : gs + NN + j;
+      const T* ps = j > 0 ? own - LX : gs + 2 * NN + i;
+      const T* pn = j < N - 1 ? own + LX : gs + 3 * NN + i;
+      const int sw = i > 0 ? LXY : N, se = i < N - 1 ? LXY : N;
+      const int ss = j > 0 ? LXY : N, sn = j < N - 1 ? LXY : N;
+      T yc = own[0];
 #pragma unroll
-    for (int u = 0; u < 4; u++) {
-      const T* q = xc_p + (k0 + u) * LXY;
-      xw[u] = q[-1];
-      xe[u] = q[1];
-      xs_[u] = q[-LX];
-      xn[u] = q[LX];
-      xu[u] = q[LXY];
-      bv[u] = bp[(k0 + u) * LXY];
+      for (int k0 = 0; k0 < N; k0 += 4) {
+        T yw[4], ye[4], ys[4], yn[4], yu[4], bv[4];
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+          const int k = k0 + u;
+          yw[u] = pw[k * sw];
+          ye[u] = pe[k * se];
+          ys[u] = ps[k * ss];
+          yn[u] = pn[k * sn];
+          yu[u] = k + 1 < N ? own[(k + 1) * LXY] : ytop;
+          bv[u] = bp[k * LXY];
+        }
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+          const int k = k0 + u;
+          T r = xsub(bv[u], yw[u]);
+          r = xsub(r, ye[u]);
+          r = xsub(r, ys[u]);
+          r = xsub(r, yn[u]);
+          r = xsub(r, ym);
+          r = xsub(r, yu[u]);
+          if (RES) acc.add(xsub(r, xmul(c0, xr[k])));
+          const T xt = sweep_div(r, c0, rc0);
+          const T x1 = xsub(xr[k], xmul(om, xsub(xr[k], xt)));
+          bp[k * LXY] = x1;
+          gp[k * LXY] = x1;
+          ym = yc;
+          yc = yu[u];
+        }
+      }
     }
+  }
+  if (!iso) {
+    T xm = xc_p[-LXY], xc = xc_p[0];
 #pragma unroll
-    for (int u = 0; u < 4; u++) {
-      const int k = k0 + u;
-      const T xp = xu[u];
-      T r = bv[u];  // b
-      r = xsub(r, xmul(c1, xw[u]));
-      r = xsub(r, xmul(c2, xe[u]));
-      r = xsub(r, xmul(c3, xs_[u]));
-      r = xsub(r, xmul(c4, xn[u]));
-      r = xsub(r, xmul(c5, xm));
-      r = xsub(r, xmul(c6, xp));
-      if (RES) acc.add(xsub(r, xmul(c0, xc)));
-      const T xt = sweep_div(r, c0, rc0);
-      const T x1 = xsub(xc, xmul(om, xsub(xc, xt)));
-      bp[k * LXY] = x1;
-      gp[k * LXY] = x1;
-      xm = xc;
-      xc = xp;
+    for (int k0 = 0; k0 < N; k0 += 4) {
+      // four cells: every load before the first store into b's area, so the
+      // loads overlap
+      T xw[4], xe[4], xs_[4], xn[4], xu[4], bv[4];
+#pragma unroll
+      for (int u = 0; u < 4; u++) {
+        const T* q = xc_p + (k0 + u) * LXY;
+        xw[u] = q[-1];
+        xe[u] = q[1];
+        xs_[u] = q[-LX];
+        xn[u] = q[LX];
+        xu[u] = q[LXY];
+        bv[u] = bp[(k0 + u) * LXY];
+      }
+#pragma unroll
+      for (int u = 0; u < 4; u++) {
+        const int k = k0 + u;
+        const T xp = xu[u];
+        T r = bv[u];  // b
+        r = xsub(r, xmul(c1, xw[u]));
+        r = xsub(r, xmul(c2, xe[u]));
+        r = xsub(r, xmul(c3, xs_[u]));
+        r = xsub(r, xmul(c4, xn[u]));
+        r = xsub(r, xmul(c5, xm));
+        r = xsub(r, xmul(c6, xp));
+        if (RES) acc.add(xsub(r, xmul(c0, xc)));
+        const T xt = sweep_div(r, c0, rc0);
+        const T x1 = xsub(xc, xmul(om, xsub(xc, xt)));
+        bp[k * LXY] = x1;
+        gp[k * LXY] = x1;
+        xm = xc;
+        xc = xp;
+      }
     }
   }
   if (RES) {

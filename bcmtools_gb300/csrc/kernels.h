@@ -258,10 +258,12 @@ cudaError_t launch_jacobi_fused(const T* x0, T* x1, const T* b, const Geom& g, c
                                 T omega, BlockBc bc, PushTable push, int ghost_mode, int shape,
                                 double* partial, int* err, const JacPre<T>* pre,
                                 cudaStream_t st, bool pdl = false);
-// mode 0: ax = A x;  mode 1: r = b - A x;  mode 2: partial[b] = sum r^2 (no store)
+// mode 0: ax = A x;  mode 1: r = b - A x;  mode 2: partial[b] = sum r^2 (no store).
+// streamed (residual_streams, device memory aligned to 16 bytes): the FP64 planes
+// stream through shared memory, and mode 2 leaves kr_parts sums per block.
 template <typename T>
 cudaError_t launch_residual(T* out, const T* x, const T* b, Op<T> op, const Geom& g, int mode,
-                            double* partial, cudaStream_t st);
+                            bool streamed, double* partial, int* err, cudaStream_t st);
 // Per-block FP64 partial sums of x.y (interiors).
 template <typename T>
 cudaError_t launch_dot_partial(const T* x, const T* y, const Geom& g, double* partial,
@@ -317,6 +319,10 @@ inline int kr_parts(const Geom& g) {
   return n < 1 ? 1 : n > 4 ? 4 : n;
 }
 constexpr int kKrMaxParts = 4;
+inline bool residual_streams(size_t es, bool constant_op, const Geom& g) {
+  return es == 8 && constant_op && g.nx == g.ny && g.ny == g.nz && (g.nx == 16 || g.nx == 32) &&
+         (g.vc == 1 || g.vc == 2);
+}
 
 // Device-resident BiCGSTAB iteration (krylov.cu): see krylov.cuh.
 template <typename T>

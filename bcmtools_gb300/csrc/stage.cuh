@@ -20,7 +20,10 @@ struct BrickStage {
   static constexpr unsigned B_BYTES = SRC ? N * PB : 0;
   static constexpr unsigned X_OFF = 16;
   static constexpr unsigned B_OFF = X_OFF + X_BYTES;
-  static constexpr size_t SMEM = B_OFF + B_BYTES;
+  // FP64: the four x and y ghost faces times the neighbours' one coefficient
+  static constexpr unsigned G_OFF = B_OFF + B_BYTES;
+  static constexpr unsigned G_BYTES = SRC && sizeof(T) == 8 ? 4 * N * N * sizeof(T) : 0;
+  static constexpr size_t SMEM = G_OFF + G_BYTES;
   static_assert(X_BYTES % 16 == 0 && PB % 16 == 0, "bulk copies need 16-byte sizes and offsets");
   // Rows j and j+D share a warp (N = 16): D*LX = 16 (mod 32) puts the two
   // half-warps of a float access on disjoint banks.

@@ -16,6 +16,7 @@
 #include "cells.cuh"
 #include "common.cuh"
 #include "kernels.h"
+#include "stream.cuh"
 #include "tile.cuh"
 
 namespace bcmg {
@@ -48,6 +49,10 @@ __device__ __forceinline__ double block_sum(double v, double* red) {
 // bytes a thread has in flight (4432 blocks of 16^3: 210 us with one plane's).
 // Chunks of planes (sweep_chunk) let a mesh of few blocks fill the chip: 328
 // blocks of 24x20x12 leave some SMs three blocks and others two.
+// (double)v without a conversion instruction, which issues at the FP64 rate.
+__device__ __forceinline__ double to_wide(float v) { return DotAcc<float>::widen(v); }
+__device__ __forceinline__ double to_wide(double v) { return v; }
+
 template <typename T, bool CC, int MODE, int V>
 struct SweepCells {
   T w[V], e[V], s[V], n[V], up[V], bv[V], c[CC ? 1 : V][7], rc[V];
@@ -120,7 +125,10 @@ __global__ void __launch_bounds__(256) sweep_kernel(T* __restrict__ out, const T
           } else {
             r = xsub(r, xmul(c[0], xc));
             if (MODE == 1) ob[q] = r;
-            else acc = __fma_rn((double)r, (double)r, acc);
+            else {
+              const double v = to_wide(r);
+              acc = __fma_rn(v, v, acc);
+            }
           }
         }
         xm = xc;
@@ -327,10 +335,138 @@ static void residual_cubic(T* out, const T* x, const T* b, const Op<T>& op, cons
   }
 }
 
+// calc_ax / calc_r / calc_r2 of FP64 fields on 16^3 / 32^3 blocks with a constant
+// operator: planes streamed through shared memory, each product formed once where
+// the six neighbours have one coefficient (stream.cuh).  CTA (b, y): planes [y zc,
+// + zc) of block b; calc_r2's partial sum at partial[b * gridDim.y + y].  One
+// thread per column took 398 us for calc_r on 342 blocks of 32^3: 14 FP64
+// operations a cell, and one block of 1024 threads per SM at a time.
+template <int N, int VC, int MODE, int S>
+struct ResStream {
+  using R = PlaneRing<double, N, VC, S, true, (MODE == 0 ? 0 : 1)>;
+  static constexpr int NT = 256;
+  static constexpr size_t SMEM = R::SMEM;
+  static constexpr int MINB = stream_minb<SMEM + 64, 4>();
+};
+
+template <int N, int VC, int MODE, int S>
+__global__ void __launch_bounds__(256, (ResStream<N, VC, MODE, S>::MINB)) residual_stream_kernel(
+    double* __restrict__ out, const double* __restrict__ x, const double* __restrict__ bb,
+    const double* __restrict__ cf8, Geom g, int zc, double* __restrict__ partial, int* err) {
+  using R = typename ResStream<N, VC, MODE, S>::R;
+  constexpr int NT = 256, CPT = N * N / NT, LX = R::LX, LXY = R::LXY;
+  extern __shared__ __align__(128) unsigned char smraw[];
+  const int b = blockIdx.x, tid = threadIdx.x;
+  const int64_t base = (int64_t)b * g.bstride + (int64_t)blockIdx.y * zc * LXY;
+  R ring(smraw, zc);
+  const double* C[1] = {bb};
+  if (tid == 0) ring.start(x, C, base);
+  double c[7];
+#pragma unroll
+  for (int q = 0; q < 7; q++) c[q] = cf8[(int64_t)b * 8 + q];
+  int o[CPT];
+#pragma unroll
+  for (int k = 0; k < CPT; k++) {
+    const int e = tid + k * NT;
+    o[k] = R::at(e % N, e / N);
+  }
+  double acc = 0.0, none = 0.0;
+  // products of the six neighbours and the cell's own -> its result
+  auto finish = [&](int m, int q, const double* p, double centre) {
+    if (MODE == 0) {
+      double a = xadd(p[0], p[1]);
+#pragma unroll
+      for (int k = 2; k < 6; k++) a = xadd(a, p[k]);
+      out[base + (int64_t)(VC + m) * LXY + q] = xadd(a, centre);
+    } else {
+      double r = ring.cp(m + 1, 0)[q];
+#pragma unroll
+      for (int k = 0; k < 6; k++) r = xsub(r, p[k]);
+      r = xsub(r, centre);
+      if (MODE == 1) out[base + (int64_t)(VC + m) * LXY + q] = r;
+      else acc = __fma_rn(r, r, acc);
+    }
+  };
+  __syncthreads();  // the ring's barriers are initialised
+  bool ok;
+  if (one_coefficient(c[1], c[2], c[3], c[4], c[5], c[6])) {
+    ScaledPlanes<N, VC, NT, R> sp;
+    ok = plane_walk(ring, x, C, base, err, tid, [&](int m) {
+      if (m == 0) sp.begin(ring, c[1], o, tid);
+      sp.take(ring, c[1], o, m, tid);
+      const double* pc = ring.xp(m + 1);
+#pragma unroll
+      for (int k = 0; k < CPT; k++) {
+        const int q = o[k];
+        const double p[6] = {pc[q - 1], pc[q + 1], pc[q - LX], pc[q + LX], sp.pm[k], sp.pu[k]};
+        finish(m, q, p, xmul(c[0], sp.xc[k]));
+      }
+      sp.shift();
+    });
+  } else {
+    ok = plane_walk(ring, x, C, base, err, tid, [&](int m) {
+      const double *xm = ring.xp(m), *xc = ring.xp(m + 1), *xu = ring.xp(m + 2);
+#pragma unroll
+      for (int k = 0; k < CPT; k++) {
+        const int q = o[k];
+        const double p[6] = {xmul(c[1], xc[q - 1]),  xmul(c[2], xc[q + 1]), xmul(c[3], xc[q - LX]),
+                             xmul(c[4], xc[q + LX]), xmul(c[5], xm[q]),     xmul(c[6], xu[q])};
+        finish(m, q, p, xmul(c[0], xc[q]));
+      }
+    });
+  }
+  if (MODE == 2) {
+    // a copy that never arrived makes the sum NaN
+    if (!ok) acc = __longlong_as_double(0x7ff8000000000000ll);
+    kr_block_sums<1>(acc, none, reinterpret_cast<double*>(smraw + R::BAR_BYTES));
+    if (tid == 0) partial[b * gridDim.y + blockIdx.y] = acc;
+  }
+}
+
+template <int N, int VC, int MODE>
+static cudaError_t residual_stream(double* out, const double* x, const double* b,
+                                   const double* cf8, const Geom& g, double* partial, int* err,
+                                   cudaStream_t st) {
+  constexpr int S = N == 32 ? 4 : 6;
+  using RS = ResStream<N, VC, MODE, S>;
+  auto kern = residual_stream_kernel<N, VC, MODE, S>;
+  static bool attr_set = false;  // once per process, not a stream operation
+  if (!attr_set) {
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)RS::SMEM);
+    if (e == cudaSuccess)
+      e = cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout,
+                               (int)cudaSharedmemCarveoutMaxShared);
+    if (e != cudaSuccess) return e;
+    attr_set = true;
+  }
+  const int parts = kr_parts(g);
+  kern<<<dim3(g.nb, parts), RS::NT, RS::SMEM, st>>>(out, x, b, cf8, g, N / parts, partial, err);
+  return cudaGetLastError();
+}
+
+template <int MODE>
+static cudaError_t residual_stream_mode(double* out, const double* x, const double* b,
+                                        const double* cf8, const Geom& g, double* partial,
+                                        int* err, cudaStream_t st) {
+  if (g.nx == 32)
+    return g.vc == 1 ? residual_stream<32, 1, MODE>(out, x, b, cf8, g, partial, err, st)
+                     : residual_stream<32, 2, MODE>(out, x, b, cf8, g, partial, err, st);
+  return g.vc == 1 ? residual_stream<16, 1, MODE>(out, x, b, cf8, g, partial, err, st)
+                   : residual_stream<16, 2, MODE>(out, x, b, cf8, g, partial, err, st);
+}
+
 template <typename T>
 cudaError_t launch_residual(T* out, const T* x, const T* b, Op<T> op, const Geom& g, int mode,
-                            double* partial, cudaStream_t st) {
+                            bool streamed, double* partial, int* err, cudaStream_t st) {
   if (g.nb == 0) return cudaSuccess;
+  if constexpr (sizeof(T) == 8) {
+    if (streamed) {
+      if (mode == 0) return residual_stream_mode<0>(out, x, b, op.cf8, g, partial, err, st);
+      if (mode == 1) return residual_stream_mode<1>(out, x, b, op.cf8, g, partial, err, st);
+      return residual_stream_mode<2>(out, x, b, op.cf8, g, partial, err, st);
+    }
+  }
   if (cubic_fast(op, g)) {
     if (mode == 0) residual_cubic<T, 0>(out, x, b, op, g, partial, st);
     else if (mode == 1) residual_cubic<T, 1>(out, x, b, op, g, partial, st);
@@ -699,8 +835,8 @@ cudaError_t launch_accumulate_f32_into_f64(double* x, const float* d, const Geom
   template cudaError_t launch_recip<T>(T*, const T*, const Geom&, cudaStream_t);            \
   template cudaError_t launch_jacobi<T>(T*, const T*, const T*, Op<T>, const Geom&, T,      \
                                         cudaStream_t);                                      \
-  template cudaError_t launch_residual<T>(T*, const T*, const T*, Op<T>, const Geom&, int,  \
-                                          double*, cudaStream_t);                           \
+  template cudaError_t launch_residual<T>(T*, const T*, const T*, Op<T>, const Geom&, int, bool, \
+                                          double*, int*, cudaStream_t);                           \
   template cudaError_t launch_dot_partial<T>(const T*, const T*, const Geom&, double*,      \
                                              cudaStream_t);                                 \
   template cudaError_t launch_blas1<T>(int, T*, const T*, const T*, T, T, const Geom&,      \
