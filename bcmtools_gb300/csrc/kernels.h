@@ -107,8 +107,10 @@ struct SorRing {
   int slo, sbytes;
   int slot, slots;  // bytes of a unit, units in shared memory
   int threads;      // of the CTA
+  int ranks;        // CTAs per block (a cluster)
   static SorRing make(const Geom& g, bool src, size_t es) {
     SorRing r;
+    r.ranks = 1;
     const int row = g.sy * (int)es;
     r.xlo = (g.vc - 1) * row / 16 * 16;
     r.xbytes = ((g.vc + g.ny + 1) * row + 15) / 16 * 16 - r.xlo;
@@ -127,16 +129,18 @@ struct SorRing {
 };
 // Whether that pass covers a run: one inner pass, whole 16-byte planes, a ring
 // within shared memory.  FP64 blocks of up to 256 cells stay staged whole (575
-// blocks of 4^3: 17.9 us an iteration, streamed 20.1), and bricks too large for
-// that are swept in place unless the rounds of 256 threads over a plane are
-// nearly full (28^3: 410 us in place, 462 streamed at 77 %; 32^3: 617 and 478).
+// blocks of 4^3: 17.9 us an iteration, streamed 20.1), so do many with planes of
+// less than 40 cell pairs (8x6x24, 2491 blocks: 181 and 197; 575: 64 and 62), and
+// bricks too large for that are swept in place unless the rounds of 256 threads
+// over a plane are nearly full (28^3: 410 us in place, 462 streamed at 77 %;
+// 32^3: 617 and 478).
 inline bool sor_streams(const Geom& g, bool src, int n_inner, size_t es) {
   const SorRing r = SorRing::make(g, src, es);
   if (n_inner != 1 || (g.sz * es) % 16 != 0 || r.bytes() > kSorMaxSmem) return false;
   if (es == 4) return true;
   const int np = g.nx / 2 * g.ny, rounds = (np + r.threads - 1) / r.threads;
   const size_t whole = (size_t)(g.nx + 2) * (g.ny + 2) * (g.nz + 2) * es;
-  return g.nx * g.ny * g.nz > 256 &&
+  return g.nx * g.ny * g.nz > 256 && (np >= 40 || g.nb < 1024) &&
          (whole <= kSorMaxSmem || 10 * np >= 9 * rounds * r.threads);
 }
 

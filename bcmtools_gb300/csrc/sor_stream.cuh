@@ -9,11 +9,17 @@
 // does both with one CTA barrier before it.  (sor1/Solver.cpp:132-153,
 // sor2/Solver.cpp:136-160: ghosts are read as they were before the pass.)
 //
-// Unit u of the ring is brick plane VC-1+u, rows [-1, ny] (and, for the nz
-// interior planes, the source's rows [0, ny)), one bulk copy each, widened to
+// Unit u of the ring is plane u - 1 of the block, rows [-1, ny] (and, for interior
+// planes, the source's rows [0, ny)), one bulk copy each, widened to
 // 16-byte bounds: a brick plane is a multiple of 16 bytes for every even block
 // shape.  Unit t-3 is last read in phase t-1; its slot then takes unit t-3+S.
 // Waits are bounded as in stream.cuh.
+//
+// A block may be split over a cluster of 2, 4 or 8 CTAs (fewer than two
+// blocks per SM leave it half idle, sor_split): each makes colour 1 of its
+// planes [k0, k1) and colour 0 of those and one more on either side -- the colour
+// its neighbour makes of the same values of A -- writes its planes, and after a
+// cluster barrier its share of the ghosts.
 //
 // Bound: HBM in FP32, the FP64 pipe in FP64.  The brick staged whole left one
 // CTA of 256 threads per SM for 32^3 (170 us an iteration on 18.8 M cells, FP32)
@@ -33,7 +39,8 @@ __global__ void __launch_bounds__(256, (sizeof(T) == 4 ? 4 : 2))
     sor_stream_kernel(const T* __restrict__ A, T* Bf, const T* __restrict__ S, Geom g, SorArgs a,
                       SorRing r) {
   extern __shared__ __align__(128) unsigned char smraw[];
-  const int b = blockIdx.x, tid = threadIdx.x, nt = blockDim.x;
+  const int rank = blockIdx.x % r.ranks, b = blockIdx.x / r.ranks;
+  const int tid = threadIdx.x, nt = blockDim.x;
   const int nx = N ? N : g.nx, ny = N ? N : g.ny, nz = N ? N : g.nz, vc = N ? VC : g.vc;
   const int sy = N ? N + 2 * VC : g.sy, sz = N ? (N + 2 * VC) * (N + 2 * VC) : g.sz;
   uint64_t* bar = reinterpret_cast<uint64_t*>(smraw);
@@ -42,11 +49,15 @@ __global__ void __launch_bounds__(256, (sizeof(T) == 4 ? 4 : 2))
   const unsigned char* Ab = reinterpret_cast<const unsigned char*>(A + base);
   const unsigned char* Sb = FORM == 2 ? reinterpret_cast<const unsigned char*>(S + base) : nullptr;
   T* fb = Bf + base;
-  const int nu = nz + 2;
+  // this CTA's planes, and the planes [c0, c0 + n0) of which it makes colour 0;
+  // unit u is plane c0 - 1 + u
+  const int zc = (nz + r.ranks - 1) / r.ranks, k0 = rank * zc, k1 = min(nz, k0 + zc);
+  const int c0 = max(0, k0 - 1), n0 = min(nz, k1 + 1) - c0;
+  const int nu = n0 + 2;
   auto issue = [&](int u, int s) {
-    const bool cells = FORM == 2 && u >= 1 && u <= nz;
+    const bool cells = FORM == 2 && u >= 1 && u <= n0;
     unsigned char* d = ring + (size_t)s * r.slot;
-    const size_t plane = (size_t)(vc - 1 + u) * sz * sizeof(T);
+    const size_t plane = (size_t)(vc - 1 + c0 + u) * sz * sizeof(T);
     mbar_expect_tx(&bar[s], r.xbytes + (cells ? r.sbytes : 0));
     bulk_g2s(d, Ab + plane + r.xlo, r.xbytes, &bar[s]);
     if (cells) bulk_g2s(d + r.xbytes, Sb + plane + r.slo, r.sbytes, &bar[s]);
@@ -77,8 +88,8 @@ __global__ void __launch_bounds__(256, (sizeof(T) == 4 ? 4 : 2))
     // ring slots of units t-2 .. t+2
     int s_2 = 0, s_1 = 0, s0 = 0, s1 = 1, s2 = 2;
     unsigned ph = 0;  // phase parity of unit t+2
-    for (int t = 0; t < nz + 2; t++) {
-      if (tid == 0 && t < nz) {
+    for (int t = 0; t < n0 + 2; t++) {
+      if (tid == 0 && t < n0) {
         if (t == 0) ok = mbar_wait_quiet(&bar[0], 0, a.err) && mbar_wait_quiet(&bar[1], 0, a.err);
         ok = ok && mbar_wait_quiet(&bar[s2], ph, a.err);
       }
@@ -93,13 +104,13 @@ __global__ void __launch_bounds__(256, (sizeof(T) == 4 ? 4 : 2))
         issue(t - 3 + r.slots, s);
         issued = t - 2 + r.slots;
       }
-      if (t < nz) {  // colour 0 of plane t
+      if (t < n0) {  // colour 0 of plane c0 + t
         const T* xm = xplane(s0);
         T* xc = xplane(s1);
         const T* xu = xplane(s2);
         const T* sp = splane(s1);
         for (int e = tid, j = j0, i2 = i0; e < np; e += nt) {
-          const int q = j * sy + 2 * i2 + ((j + t) & 1);
+          const int q = j * sy + 2 * i2 + ((j + c0 + t) & 1);
           const T sw = xadd(xc[q - 1], xc[q + 1]);
           const T ss = xadd(xc[q - sy], xc[q + sy]);
           const T sb = xadd(xm[q], xu[q]);
@@ -109,8 +120,8 @@ __global__ void __launch_bounds__(256, (sizeof(T) == 4 ? 4 : 2))
           if (i2 >= hx) { i2 -= hx; j++; }
         }
       }
-      if (t >= 2) {  // colour 1 of plane t-2, and its rows to B
-        const int k = t - 2;
+      const int k = c0 + t - 2;
+      if (k >= k0 && k < k1) {  // colour 1 of plane k, and its rows to B
         const T* xm = xplane(s_2);
         const T* xc = xplane(s_1);
         const T* xu = xplane(s0);
@@ -157,25 +168,30 @@ __global__ void __launch_bounds__(256, (sizeof(T) == 4 ? 4 : 2))
         if (u >= 0) mbar_wait_quiet(&bar[s], (unsigned)(u / r.slots) & 1u, nullptr);
       }
     __syncthreads();
-    return;
   }
-  __syncthreads();  // the block's new interior is in its brick, seen by the CTA
+  // the block's new interior is in its brick, seen by the CTA, or the cluster
+  if (r.ranks > 1)
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;"
+                 ::: "memory");
+  else
+    __syncthreads();
+  if (!ok) return;
   // Dirichlet ghosts: g = 2v - f, and the second layer of the bcx form
   if (dmask) {
     const double* dval = a.bc.value + b * 6;
     for (int fc = 0; fc < 6; fc++) {
       if (!((dmask >> fc) & 1)) continue;
       const int ax = fc >> 1, minus = (fc & 1) == 0;
-      const int n0 = ax == 0 ? ny : nx, n1 = ax == 2 ? ny : nz, nn = ax == 0 ? nx : ax == 1 ? ny : nz;
+      const int d0 = ax == 0 ? ny : nx, d1 = ax == 2 ? ny : nz, nn = ax == 0 ? nx : ax == 1 ? ny : nz;
       double v = dval[fc];
       if (a.bc.bcx) v = (double)(T)v;
       const double v2 = xmul(2.0, v);
       const int st0 = ax == 0 ? sy : 1, st1 = ax == 2 ? sy : sz, stn = ax == 0 ? 1 : ax == 1 ? sy : sz;
       const int in = minus ? 0 : nn - 1, gh = minus ? -1 : nn, g2 = minus ? -2 : nn + 1;
       const int o = vc * (1 + sy + sz);
-      for (int e = tid; e < n0 * n1; e += nt) {
+      for (int e = tid + rank * nt; e < d0 * d1; e += nt * r.ranks) {
         int q1, q0;
-        divmod(e, n0, q1, q0);
+        divmod(e, d0, q1, q0);
         const int at = o + q0 * st0 + q1 * st1;
         fb[at + gh * stn] = to_t<T>(xsub(v2, (double)fb[at + in * stn]));
         if (a.bc.bcx && vc >= 2) fb[at + g2 * stn] = (T)v;
@@ -183,7 +199,7 @@ __global__ void __launch_bounds__(256, (sizeof(T) == 4 ? 4 : 2))
     }
   }
   if constexpr (N > 0) {
-    for (int q = p0 + (tid >> 5); q < p1; q += nt >> 5) {
+    for (int q = p0 + ((tid + rank * nt) >> 5); q < p1; q += (nt >> 5) * r.ranks) {
       const VcTask t = a.push.tasks[q];
       push_dispatch<T, N, VC, BrickTile<T, N, VC>, 4>(t, Bf + (int64_t)t.dst * g.bstride, g, fb,
                                                       tid & 31);
@@ -191,7 +207,7 @@ __global__ void __launch_bounds__(256, (sizeof(T) == 4 ? 4 : 2))
   } else {
     const Acc<T> src{fb, g.sy, g.sz, g.off0};
     const int es = entry_shift(g);
-    for (int q = p0 + (tid >> es); q < p1; q += nt >> es) {
+    for (int q = p0 + ((tid + rank * nt) >> es); q < p1; q += (nt >> es) * r.ranks) {
       const VcTask t = a.push.tasks[q];
       task_apply<T>(t, Bf + (int64_t)t.dst * g.bstride, g, src, 0.0, tid & ((1 << es) - 1),
                     1 << es);
@@ -206,6 +222,18 @@ static bool sor_stream_ok(const Geom& g, const T* A, const T* s, int n_inner) {
   return sor_streams(g, s != nullptr, n_inner, sizeof(T)) &&
          ((size_t)g.bstride * sizeof(T)) % 16 == 0 &&
          reinterpret_cast<uintptr_t>(A) % 16 == 0 && reinterpret_cast<uintptr_t>(s) % 16 == 0;
+}
+
+// CTAs per block: two, four or eight until there are three per SM in FP64 and for
+// 128-thread planes, two in FP32, each with six planes or more (it makes colour 0
+// of two planes more than its own).  342 blocks split in two: FP64 24^3 287 -> 233
+// us an iteration, 32^3 443 -> 394, FP32 8x6x24 36 -> 26 but 28^3 78 -> 85; 575
+// blocks: FP64 24^3 302 -> 334, FP32 69 -> 83.
+inline int sor_split(const Geom& g, const SorRing& ring, size_t es) {
+  const int want = (es == 8 || ring.threads == 128 ? 3 : 2) * 152;
+  int r = 1;
+  while (r < 8 && g.nb * r < want && g.nz >= 2 * r * 6) r *= 2;
+  return r;
 }
 
 template <typename T, int FORM, int N, int VC>
@@ -223,9 +251,10 @@ static cudaError_t sor_stream_one(const T* A, T* B, const T* s, const Geom& g, c
     if (e != cudaSuccess) return e;
     attr_set = true;
   }
-  const SorRing r = SorRing::make(g, FORM == 2, sizeof(T));
-  kern<<<g.nb, r.threads, r.bytes(), st>>>(A, B, s, g, a, r);
-  return cudaGetLastError();
+  SorRing r = SorRing::make(g, FORM == 2, sizeof(T));
+  r.ranks = sor_split(g, r, sizeof(T));
+  return launch_dependent(kern, g.nb * r.ranks, r.threads, r.bytes(), st, false, r.ranks, A, B, s,
+                          g, a, r);
 }
 
 template <typename T, int FORM>
