@@ -120,7 +120,6 @@ struct bcmg_ctx_s {
   std::map<long, int> work;  // cached solver work fields: key (dtype, vc, slot)
 
   double* d_partial = nullptr;
-  double* d_scalar = nullptr;
   // device-resident BiCGSTAB: two partial sums per block, the segments'
   // scalar records and their pinned host mirror
   double* d_kpart = nullptr;
@@ -483,7 +482,6 @@ BCMG_API int bcmg_ctx_create(bcmg_ctx* out, int device) {
   c->device = device;
   if (cudaSetDevice(device) != cudaSuccess ||
       cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking) != cudaSuccess ||
-      cudaMalloc(&c->d_scalar, 64 * sizeof(double)) != cudaSuccess ||
       cudaMalloc(&c->d_err, sizeof(int)) != cudaSuccess ||
       cudaMemset(c->d_err, 0, sizeof(int)) != cudaSuccess ||
       cudaMallocHost(&c->h_scalar, 64 * sizeof(double)) != cudaSuccess) {
@@ -525,7 +523,6 @@ BCMG_API void bcmg_ctx_destroy(bcmg_ctx c) {
   cudaFree(c->d_bcv2f);
   cudaFree(c->d_bczero2f);
   cudaFree(c->d_partial);
-  cudaFree(c->d_scalar);
   cudaFree(c->d_kpart);
   cudaFree(c->d_kseg);
   cudaFreeHost(c->h_kseg);
@@ -1593,7 +1590,7 @@ static const double* op_recip(bcmg_ctx c, int op, int vc, cudaStream_t st) {
   if (work_field(c, BCMG_F64, vc, 35, &id)) return nullptr;
   double* out = (double*)get_field(c, id)->d;
   prof_mark(c, K_OTHER, st, true);
-  const cudaError_t e = launch_recip<double>(out, (const double*)a0->d, geom_of(c, *a0), st);
+  const cudaError_t e = launch_recip(out, (const double*)a0->d, geom_of(c, *a0), st);
   prof_mark(c, K_OTHER, st, false);
   c->launches++;
   return e == cudaSuccess ? out : nullptr;
@@ -1659,8 +1656,9 @@ static int residual(bcmg_ctx c, int op, Field* out, Field& x, Field* b, int mode
 
 // Sum the partials (one per block unless said) and bring the value to the host.
 static int finish_reduce(bcmg_ctx c, double* out, cudaStream_t st, int n = 0) {
-  LAUNCH(c, K_DOT, st, launch_reduce_final(c->d_partial, n ? n : c->nb, c->d_scalar, st));
-  CUDA_TRY(c, cudaMemcpyAsync(c->h_scalar, c->d_scalar, sizeof(double), cudaMemcpyDeviceToHost, st));
+  // straight to pinned host memory (one address under unified addressing): no copy
+  // between the kernel and the wait
+  LAUNCH(c, K_DOT, st, launch_reduce_final(c->d_partial, n ? n : c->nb, c->h_scalar, st));
   CUDA_TRY(c, cudaStreamSynchronize(st));
   *out = c->h_scalar[0];
   return BCMG_SUCCESS;

@@ -213,8 +213,7 @@ inline int sweep_chunk(const Geom& g) {
 
 // RN(1/Ap) of every interior cell of a coefficient field, 0 where the FP64
 // sweeps' division by it does not apply.
-template <typename T>
-cudaError_t launch_recip(T* out, const T* a, const Geom& g, cudaStream_t st);
+cudaError_t launch_recip(double* out, const double* a, const Geom& g, cudaStream_t st);
 
 template <typename T>
 cudaError_t launch_jacobi(T* x1, const T* x0, const T* b, Op<T> op, const Geom& g, T omega,

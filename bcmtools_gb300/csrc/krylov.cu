@@ -632,20 +632,22 @@ __device__ __forceinline__ void kr_segment_sums(const double* __restrict__ parti
   const int bd = blockDim.x;
   v0 = v1 = 0.0;
   int q = f0 + threadIdx.x;
-  for (; q < f1; q += U * bd) {
+  for (; q + (U - 1) * bd < f1; q += U * bd) {
     double a[U], b[U];
 #pragma unroll
     for (int u = 0; u < U; u++) {
-      const bool in = q + u * bd < f1;
-      a[u] = in ? partial[q + u * bd] : 0.0;
-      b[u] = in ? partial[nb + q + u * bd] : 0.0;
+      a[u] = partial[q + u * bd];
+      b[u] = partial[nb + q + u * bd];
     }
 #pragma unroll
     for (int u = 0; u < U; u++) {
-      if (q + u * bd >= f1) break;
       v0 = __dadd_rn(v0, a[u]);
       v1 = __dadd_rn(v1, b[u]);
     }
+  }
+  for (; q < f1; q += bd) {
+    v0 = __dadd_rn(v0, partial[q]);
+    v1 = __dadd_rn(v1, partial[nb + q]);
   }
   v0 = kr_block_sum(v0, red);
   v1 = kr_block_sum(v1, red);

@@ -49,10 +49,6 @@ __device__ __forceinline__ double block_sum(double v, double* red) {
 // bytes a thread has in flight (4432 blocks of 16^3: 210 us with one plane's).
 // Chunks of planes (sweep_chunk) let a mesh of few blocks fill the chip: 328
 // blocks of 24x20x12 leave some SMs three blocks and others two.
-// (double)v without a conversion instruction, which issues at the FP64 rate.
-__device__ __forceinline__ double to_wide(float v) { return DotAcc<float>::widen(v); }
-__device__ __forceinline__ double to_wide(double v) { return v; }
-
 template <typename T, bool CC, int MODE, int V>
 struct SweepCells {
   T w[V], e[V], s[V], n[V], up[V], bv[V], c[CC ? 1 : V][7], rc[V];
@@ -125,10 +121,7 @@ __global__ void __launch_bounds__(256) sweep_kernel(T* __restrict__ out, const T
           } else {
             r = xsub(r, xmul(c[0], xc));
             if (MODE == 1) ob[q] = r;
-            else {
-              const double v = to_wide(r);
-              acc = __fma_rn(v, v, acc);
-            }
+            else acc = __fma_rn((double)r, (double)r, acc);
           }
         }
         xm = xc;
@@ -161,25 +154,29 @@ static cudaError_t launch_sweep(T* out, const T* x, const T* b, const Op<T>& op,
 }
 
 // RN(1/Ap) of every interior cell, 0 where the two-FMA division does not cover
-// Ap (div_pre, cells.cuh): made once for the sweeps of a run or solve.
-template <typename T>
-__global__ void __launch_bounds__(256) recip_kernel(T* __restrict__ out, const T* __restrict__ a,
-                                                    Geom g) {
+// Ap (div_pre, cells.cuh): made once for the FP64 sweeps of a run or solve.
+// Bound by the FP64 pipe: a reciprocal and an integer test of the exponent (a
+// division and two compares took 318 us on 18.2 M cells).
+__global__ void __launch_bounds__(256) recip_kernel(double* __restrict__ out,
+                                                    const double* __restrict__ a, Geom g, int zc) {
   const int64_t base = (int64_t)blockIdx.x * g.bstride;
   const int ncol = g.nx * g.ny;
+  const int z0 = blockIdx.y * zc, z1 = min(g.nz, z0 + zc);
   for (int ij = threadIdx.x; ij < ncol; ij += blockDim.x) {
-    int64_t o = base + g.at(ij % g.nx, ij / g.nx, 0);
-    for (int k = 0; k < g.nz; k++, o += g.sz) {
-      const T v = a[o], m = v < T(0) ? -v : v;
-      out[o] = (m >= T(0x1p-60) && m <= T(0x1p+60)) ? xdiv(T(1), v) : T(0);
+    int64_t o = base + g.at(ij % g.nx, ij / g.nx, z0);
+#pragma unroll 4
+    for (int k = z0; k < z1; k++, o += g.sz) {
+      const double v = a[o];
+      const unsigned e = ((unsigned)__double2hiint(v) >> 20) & 0x7ffu;
+      out[o] = e - (1023u - 60u) < 120u ? __drcp_rn(v) : 0.0;
     }
   }
 }
 
-template <typename T>
-cudaError_t launch_recip(T* out, const T* a, const Geom& g, cudaStream_t st) {
+cudaError_t launch_recip(double* out, const double* a, const Geom& g, cudaStream_t st) {
   if (g.nb == 0) return cudaSuccess;
-  recip_kernel<T><<<g.nb, column_threads(g), 0, st>>>(out, a, g);
+  const int zc = sweep_chunk(g);
+  recip_kernel<<<dim3(g.nb, (g.nz + zc - 1) / zc), column_threads(g), 0, st>>>(out, a, g, zc);
   return cudaGetLastError();
 }
 
@@ -559,15 +556,17 @@ __global__ void __launch_bounds__(1024) reduce_final_kernel(const double* __rest
                                                             int n, double* __restrict__ out) {
   __shared__ double red[32];
   constexpr int U = 8;  // loads of eight rounds before the first addition
+  const int bd = blockDim.x;
   double acc = 0.0;
-  for (int i = threadIdx.x; i < n; i += U * blockDim.x) {
+  int i = threadIdx.x;
+  for (; i + (U - 1) * bd < n; i += U * bd) {
     double v[U];
 #pragma unroll
-    for (int u = 0; u < U; u++) v[u] = i + u * blockDim.x < n ? partial[i + u * blockDim.x] : 0.0;
+    for (int u = 0; u < U; u++) v[u] = partial[i + u * bd];
 #pragma unroll
-    for (int u = 0; u < U; u++)
-      if (i + u * blockDim.x < n) acc += v[u];
+    for (int u = 0; u < U; u++) acc += v[u];
   }
+  for (; i < n; i += bd) acc += partial[i];
   acc = block_sum(acc, red);
   if (threadIdx.x == 0) out[0] = acc;
 }
@@ -832,7 +831,6 @@ cudaError_t launch_accumulate_f32_into_f64(double* x, const float* d, const Geom
 
 #define INST(T)                                                                              \
   template cudaError_t launch_copy_frame<T>(T*, const T*, const Geom&, bool, cudaStream_t); \
-  template cudaError_t launch_recip<T>(T*, const T*, const Geom&, cudaStream_t);            \
   template cudaError_t launch_jacobi<T>(T*, const T*, const T*, Op<T>, const Geom&, T,      \
                                         cudaStream_t);                                      \
   template cudaError_t launch_residual<T>(T*, const T*, const T*, Op<T>, const Geom&, int, bool, \

@@ -109,7 +109,8 @@ __device__ __forceinline__ void push_entry(const VcTask& t, T* __restrict__ dst,
       if (AX == 2) {
         a = e % TN; c = (e / TN) % TN; u = e / (TN * TN);
       } else if (AX == 0) {
-        a = e % TN; u = (e / TN) % NL; c = e / (TN * NL);
+        // the ghost layers of a row side by side: two lanes a 32-byte sector
+        u = e % NL; a = (e / NL) % TN; c = e / (TN * NL);
       } else {
         c = e % TN; u = (e / TN) % NL; a = e / (TN * NL);
       }

@@ -34,6 +34,43 @@ __global__ void __launch_bounds__(256) vc_gather_kernel(T* __restrict__ data, Ge
   task_apply<T>(t, dst, g, src, bcv, lane, 1 << es);
 }
 
+// Boundary ghosts of one outer face of a cubic block (task_apply's values).
+template <typename T, int N, int VC>
+__device__ __forceinline__ void boundary_entry(const VcTask& t, T* __restrict__ brick, double v,
+                                               int lane) {
+  using BL = BrickTile<T, N, VC>;
+  const int ax = t.face >> 1;
+  const bool minus = (t.face & 1) == 0, neumann = t.flags & kTaskNeumann;
+  const int sp = ax == 0 ? BL::LX : 1, sq = ax == 2 ? BL::LX : BL::LXY;
+  const int sn = (ax == 0 ? 1 : ax == 1 ? BL::LX : BL::LXY) * (minus ? -1 : 1);  // outwards
+  T* face = brick + BL::O + (minus ? 0 : (N - 1) * sn);  // cell (0, 0) of the interior layer
+  if ((t.flags & 1) && !neumann) v = (double)(T)v;
+  const T xc = (T)v;
+  const double v2 = xmul(2.0, neumann ? (double)xc : v);
+  constexpr int U = N * N / 32 < 8 ? N * N / 32 : 8;
+  for (int e0 = lane; e0 < N * N; e0 += 32 * U) {
+    T in[U];
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+      const int e = e0 + 32 * u;
+      in[u] = face[e % N * sp + e / N * sq];
+    }
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+      const int e = e0 + 32 * u;
+      T* p = face + e % N * sp + e / N * sq + sn;
+      if (neumann) {
+        *p = minus ? xsub(in[u], xc) : xadd(in[u], xc);
+        if (VC >= 2)
+          p[sn] = to_t<T>(minus ? xsub((double)in[u], v2) : xadd((double)in[u], v2));
+      } else {
+        *p = to_t<T>(xsub(v2, (double)in[u]));
+        if ((t.flags & 1) && VC >= 2) p[sn] = xc;
+      }
+    }
+  }
+}
+
 // Cubic 8^3 / 16^3 / 32^3 blocks with vc <= 2: the same entries with the
 // entry's kind, axis, block edge and ghost width fixed at compile time,
 // reading the source brick in place (push_entry over the brick layout).
@@ -52,8 +89,7 @@ __global__ void __launch_bounds__(256)
   const VcTask t = tab.tasks[rg.start[q] + (w - rg.prefix[q])];
   T* dst = data + (int64_t)t.dst * g.bstride;
   if (t.kind == VC_DIRICHLET) {
-    const Acc<T> src{dst, g.sy, g.sz, g.off0};
-    task_apply<T>(t, dst, g, src, tab.bcval[t.dst * 6 + t.face], lane, 32);
+    boundary_entry<T, N, VC>(t, dst, tab.bcval[t.dst * 6 + t.face], lane);
     return;
   }
   const T* src = data + (int64_t)t.src * g.bstride;
