@@ -451,6 +451,28 @@ static int create_field(bcmg_ctx c, int dtype, int vc, int* out, bool host = fal
   return BCMG_SUCCESS;
 }
 
+// Work fields that a call can do without, kept from earlier ones: the reciprocals
+// of a coefficient operator (op_recip) and, unless `second` is false, the second
+// buffer of the fused SOR sweep.  Given back when another field finds no room.
+enum { kSlotSorSecond = 30, kSlotRecip = 35 };
+static bool drop_spare(bcmg_ctx c, bool second) {
+  bool any = false;
+  for (auto it = c->work.begin(); it != c->work.end();) {
+    const int slot = (int)(it->first % 64);
+    auto f = c->fields.find(it->second);
+    if (f == c->fields.end() || !(slot == kSlotRecip || (second && slot == kSlotSorSecond))) {
+      ++it;
+      continue;
+    }
+    dev_free(c, f->second.d, f->second.bytes);  // waits for the device
+    if (f->second.ev) cudaEventDestroy(f->second.ev);
+    c->fields.erase(f);
+    it = c->work.erase(it);
+    any = true;
+  }
+  return any;
+}
+
 static int work_field(bcmg_ctx c, int dtype, int vc, int slot, int* out) {
   const long key = ((long)dtype * 64 + vc) * 64 + slot;
   auto it = c->work.find(key);
@@ -459,6 +481,10 @@ static int work_field(bcmg_ctx c, int dtype, int vc, int slot, int* out) {
     return BCMG_SUCCESS;
   }
   int rc = create_field(c, dtype, vc, out);
+  // the SOR run and its tuner hold the second buffer while they ask for these
+  const bool sor = slot == kSlotSorSecond || slot == 31 || slot == 34;
+  if (rc == BCMG_MEMORY && slot != kSlotRecip && drop_spare(c, !sor))
+    rc = create_field(c, dtype, vc, out);
   if (rc) return rc;
   c->work[key] = *out;
   return BCMG_SUCCESS;
@@ -979,7 +1005,9 @@ BCMG_API int bcmg_set_boundary(bcmg_ctx c, const int* bc_type, const double* bc_
 
 BCMG_API int bcmg_field_create(bcmg_ctx c, int dtype, int vc, int* field) {
   if (!c || !field) return BCMG_USAGE;
-  return create_field(c, dtype, vc, field);
+  int rc = create_field(c, dtype, vc, field);
+  if (rc == BCMG_MEMORY && drop_spare(c, true)) rc = create_field(c, dtype, vc, field);
+  return rc;
 }
 
 BCMG_API int bcmg_field_create_host(bcmg_ctx c, int dtype, int vc, int* field) {
@@ -1229,7 +1257,7 @@ BCMG_API int bcmg_sor_run(bcmg_ctx c, int fid, int sid, const double* coef, doub
   bool fused = n_inner >= 1 && !c->bc_conflict && (smem <= kSorMaxSmem || streams) && !c->no_fusion;
   int rc = BCMG_SUCCESS;
   int wid, pid = -1;
-  if (fused && n_outer > 0 && (rc = work_field(c, f->dtype, f->vc, 30, &wid))) {
+  if (fused && n_outer > 0 && (rc = work_field(c, f->dtype, f->vc, kSlotSorSecond, &wid))) {
     // no room for a second buffer: a streamed shape is swept in place
     if (!(streams && rc == BCMG_MEMORY)) {
       cudaFreeAsync(d_coef, stream);
@@ -1587,7 +1615,7 @@ static const double* op_recip(bcmg_ctx c, int op, int vc, cudaStream_t st) {
   const Field* a0 = get_field(c, it->second.fields[0]);
   if (!a0 || a0->dtype != BCMG_F64 || a0->vc != vc) return nullptr;
   int id;
-  if (work_field(c, BCMG_F64, vc, 35, &id)) return nullptr;
+  if (work_field(c, BCMG_F64, vc, kSlotRecip, &id)) return nullptr;
   double* out = (double*)get_field(c, id)->d;
   prof_mark(c, K_OTHER, st, true);
   const cudaError_t e = launch_recip(out, (const double*)a0->d, geom_of(c, *a0), st);

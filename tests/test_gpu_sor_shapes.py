@@ -72,3 +72,45 @@ def test_no_room_for_a_second_buffer(gpu_ok):
     buffer of the streamed pass the blocks are swept in place."""
     got, ref, _ = run("f64", (32, 32, 32), 1, 2, bg.DIRICHLET_SOR, True, budget=1)
     assert_bitexact(got, ref, brick_mask((32, 32, 32), 1), "in place")
+
+
+def test_spare_work_fields_are_given_back(gpu_ok):
+    """The reciprocals a run with coefficient fields keeps, and the second buffer
+    of the streamed SOR pass, do not stand in the way of a later field."""
+    tree = small_octree(periodic=(False, False, False), level=1, radius=0.3)
+    n, vc = 8, 1
+    bm = bg.BlockManager(0)
+    bm.register_octree(tree, n)
+    bct, bcv = outer_dirichlet(tree, 0.25)
+    bm.set_boundary(bct, bcv, bg.DIRICHLET_SOR)
+    x, b = bm.setDataClass("f64", vc), bm.setDataClass("f64", vc)
+    one = bm.memory_in_use() // 2
+    fs = [bm.setDataClass("f64", vc) for _ in range(7)]
+    rng = np.random.default_rng(2)
+    for k, f in enumerate(fs):
+        f.upload(rng.uniform(0.5, 1.0, size=f.shape) - (7.0 if k == 0 else 0.0))
+    x.upload(rng.uniform(-1, 1, size=x.shape))
+    b.upload(rng.uniform(-1, 1, size=x.shape))
+    op = bm.op_fields(fs)
+    a0 = x.download()
+    bm.set_memory_budget(bm.memory_in_use() + 2 * one)  # the work copy and one more
+    bm.jacobi_run(op, x, b, 0.8, 5)
+    with_recip = x.download()
+    extra = bm.setDataClass("f64", vc)  # takes the reciprocals' place
+    with pytest.raises(bg.BcmgError):
+        bm.setDataClass("f64", vc)
+    x.upload(a0)
+    bm.jacobi_run(op, x, b, 0.8, 5)  # no room for them: divides
+    assert_bitexact(x.download(), with_recip, what="with and without the reciprocals")
+    bm.destroy(extra)
+
+    bm = bg.BlockManager(0)
+    bm.register_octree(tree, 32)
+    bm.set_boundary(bct, bcv, bg.DIRICHLET_SOR)
+    f = bm.setDataClass("f64", vc)
+    bm.set_memory_budget(2 * bm.memory_in_use())
+    coef = bg.sor1_coef(tree.cell_sizes(32), 1.3)
+    bm.sor_run(f, coef, 1.3, form=1, n_inner=1, n_outer=2)
+    bm.setDataClass("f64", vc)
+    bm.sor_run(f, coef, 1.3, form=1, n_inner=1, n_outer=2)
+    bm.sync()
