@@ -300,13 +300,15 @@ cudaError_t launch_xch(T* data, const Geom& g, const VcTask* ents, const int64_t
                        T* buf, bool pack, cudaStream_t st);
 
 // Whether the BiCGSTAB iteration's kernels are launched as dependents of one
-// another (launch_dependent, bulk.cuh): FP32, where the gap between two launches
-// is some per cent of a kernel (six solves of 1001 blocks of 16^3: 62.7 -> 59.3
-// ms).  Not where a kernel's blocks fill less than two waves of three CTAs per SM:
-// the next one's CTAs then take the free slots unevenly (FP64, 342 blocks of
-// 32^3: 38.6 -> 40.7 ms).
+// another (launch_dependent, bulk.cuh): FP32 on blocks of at most 16^3, up to 1216
+// of them, where the gap between two launches is some per cent of a kernel (six
+// solves of 1001 blocks in all: 62.7 ms without, 60.0 with).  Not on larger meshes:
+// 1427 blocks 276 us an iteration without, 281 with; 2549 blocks 419 and 447; and
+// a dependent's waiting CTAs hold slots that other streams' kernels would take (200
+// served requests on four streams: median latency 8 s without, 12 s with, 5.88 and
+// 5.82 solves a second).  Nor in FP64 (342 blocks of 32^3: 38.6 ms without, 40.7).
 inline bool kr_dependent(size_t es, const Geom& g) {
-  return es == 4 && (g.nx * g.ny * g.nz <= 4096 || g.nb >= 2 * 3 * 152);
+  return es == 4 && g.nx * g.ny * g.nz <= 4096 && g.nb <= 8 * 152;
 }
 
 // Parts of a block's planes that the kernels with inner products take as CTAs of
