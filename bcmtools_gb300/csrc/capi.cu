@@ -318,9 +318,12 @@ static VcRanges select_ranges(bcmg_ctx c, int axis_mask, int ld_mask, bool vc, b
     r.prefix[r.n + 1] = r.prefix[r.n] + c->cat_count[q];
     r.n++;
   };
-  // F2C first, then same level, then C2F (the SeparateLevelDiff order,
-  // LocalScalar3D.h:214-224); the order is immaterial on one rank.
-  const int ldbits[3] = {2, 1, 0};
+  // C2F first, then F2C, then same level: the order is immaterial on one rank
+  // (the reference's SeparateLevelDiff order is LocalScalar3D.h:214-224), and an
+  // interpolated entry takes the longest, so it must not start last (575 blocks of
+  // 32^3, FP64, vc = 2, a whole update: 171 us with C2F last, 108 with C2F first;
+  // 1427 of 16^3, FP32, 25.7 and 21.0).
+  const int ldbits[3] = {0, 2, 1};
   if (vc)
     for (int li = 0; li < 3; li++) {
       const int lb = ldbits[li];
