@@ -1349,9 +1349,10 @@ BCMG_API int bcmg_sor_run(bcmg_ctx c, int fid, int sid, const double* coef, doub
     return rc;
   }
   // In-place path: SOR pass, then the gather.  The SOR kernel leaves the
-  // block's Dirichlet ghosts final, so after it only the VC update remains
-  // (unless a Dirichlet face also has a neighbour).
-  const VcRanges after = select_ranges(c, 7, 7, true, n_inner == 0 || c->bc_conflict);
+  // block's Dirichlet ghosts final, so after it only the VC update remains.  A
+  // Dirichlet face that has a neighbour too gets its ghosts from both: the VC
+  // update first, then the boundary condition in a launch of its own.
+  const VcRanges after = select_ranges(c, 7, 7, true, n_inner == 0);
   for (int it = 0; it < n_outer && rc == BCMG_SUCCESS; it++) {
     cudaError_t e;
     prof_mark(c, K_SOR, stream, true);
@@ -1367,7 +1368,7 @@ BCMG_API int bcmg_sor_run(bcmg_ctx c, int fid, int sid, const double* coef, doub
       rc = fail(c, BCMG_CUDA_ERROR, "SOR launch: %s", cudaGetErrorString(e));
       break;
     }
-    rc = gather(c, *f, after, false, stream);
+    rc = c->bc_conflict ? impose(c, *f, false, stream) : gather(c, *f, after, false, stream);
   }
   cudaFreeAsync(d_coef, stream);
   return rc;
