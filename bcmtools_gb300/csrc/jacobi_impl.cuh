@@ -19,6 +19,7 @@
 #pragma once
 #include <type_traits>
 
+#include "attr.h"
 #include "cells.cuh"
 #include "pipe.cuh"
 #include "stage.cuh"
@@ -1021,18 +1022,8 @@ static cudaError_t jacobi_stream_launch_as(const T* x0, T* x1, const T* b, const
                                            const JacArgs<T>& a, cudaStream_t st) {
   using JS = JacStream<T, N, VC, S, RES, ZERO, 256, PRE>;
   auto kern = jacobi_stream_push_kernel<T, N, VC, S, RES, ZERO, 256, PRE, SPLIT>;
-  // set once per process (not a stream operation; runs before any CUDA-graph
-  // capture of these launches)
-  static bool attr_set = false;
-  if (!attr_set) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)JS::SMEM);
-    if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout,
-                               (int)cudaSharedmemCarveoutMaxShared);
-    if (e != cudaSuccess) return e;
-    attr_set = true;
-  }
+  static SharedMemory shared;
+  if (cudaError_t e = shared.allow(kern, JS::SMEM)) return e;
   return launch_dependent(kern, g.nb * (SPLIT ? a.ranks : 1), JS::NT, JS::SMEM, st, a.pdl,
                           SPLIT ? a.ranks : 1, x0, x1, b, g, a);
 }
@@ -1096,17 +1087,8 @@ static cudaError_t jacobi_tile_launch(const T* x0, T* x1, const T* b, const Geom
               : ki == 2 ? jacobi_tile_kernel<T, N, VC, false, true>
               : ki == 3 ? jacobi_tile_kernel<T, N, VC, true, true>
                         : jacobi_tile_kernel<T, N, VC, false, true, true>;
-  // set once per process (not a stream operation, allowed during a capture)
-  static bool attr_set[5] = {};
-  if (!attr_set[ki]) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)L::SMEM);
-    if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout,
-                               (int)cudaSharedmemCarveoutMaxShared);
-    if (e != cudaSuccess) return e;
-    attr_set[ki] = true;
-  }
+  static SharedMemory shared[5];
+  if (cudaError_t e = shared[ki].allow(kern, L::SMEM)) return e;
   return launch_dependent(kern, g.nb, L::NT, L::SMEM, st, a.pdl, 1, x0, x1, b, g, a);
 }
 

@@ -12,6 +12,7 @@
 #include <cfloat>
 #include <type_traits>
 
+#include "attr.h"
 #include "bcmg.h"
 #include "bulk.cuh"
 #include "cells.cuh"
@@ -270,18 +271,8 @@ static cudaError_t kr_ax_stream_one(T* out, const T* x, const T* cf8, const T* y
                                     cudaStream_t st) {
   using AS = AxStream<T, N, VC, S>;
   auto kern = kr_ax_stream_kernel<T, N, VC, NDOT, S>;
-  // set once per process (not a stream operation; runs before any CUDA-graph
-  // capture of these launches)
-  static bool attr_set = false;
-  if (!attr_set) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)AS::SMEM);
-    if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout,
-                               (int)cudaSharedmemCarveoutMaxShared);
-    if (e != cudaSuccess) return e;
-    attr_set = true;
-  }
+  static SharedMemory shared;
+  if (cudaError_t e = shared.allow(kern, AS::SMEM)) return e;
   return launch_dependent(kern, dim3(g.nb, parts), AS::NT, AS::SMEM, st, kr_dependent(sizeof(T), g), 1, out, x,
                           cf8, y0, g, N / parts, S_, partial, err);
 }
@@ -373,18 +364,8 @@ static cudaError_t kr_xr_stream(T* x, T* r, const T* p_, const T* s_, const T* s
                                 cudaStream_t st) {
   using XS = XrStream<T, N, VC, S>;
   auto kern = kr_xr_stream_kernel<T, N, VC, S>;
-  // set once per process (not a stream operation; runs before any CUDA-graph
-  // capture of these launches)
-  static bool attr_set = false;
-  if (!attr_set) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)XS::SMEM);
-    if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout,
-                               (int)cudaSharedmemCarveoutMaxShared);
-    if (e != cudaSuccess) return e;
-    attr_set = true;
-  }
+  static SharedMemory shared;
+  if (cudaError_t e = shared.allow(kern, XS::SMEM)) return e;
   return launch_dependent(kern, g.nb, XS::NT, XS::SMEM, st, kr_dependent(sizeof(T), g), 1, x, r, p_, s_, s, t, r0, g, S_,
                           partial, err);
 }

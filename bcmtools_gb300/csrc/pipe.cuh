@@ -32,6 +32,7 @@
 #pragma once
 #include <algorithm>
 
+#include "attr.h"
 #include "bulk.cuh"
 #include "cells.cuh"
 #include "ghost.cuh"
@@ -569,24 +570,12 @@ cudaError_t pipe_launch(const T* A, T* B, const T* S, const Geom& g, const PipeA
   constexpr size_t SMEM = STAGES * (size_t)PS::STAGE;
   if (SMEM > kPipeMaxSmem) return cudaErrorInvalidValue;
   auto kern = sweep_pipe_kernel<T, N, VC, OP, RES, STAGES>;
-  // attributes and residency: once per process (not stream operations; the
-  // first launch of every caller runs before any CUDA-graph capture)
-  static int per_sm = 0, sms = 0;
-  if (per_sm == 0) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)SMEM);
-    if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout,
-                               (int)cudaSharedmemCarveoutMaxShared);
-    int dev = 0;
-    if (e == cudaSuccess) e = cudaGetDevice(&dev);
-    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    if (e == cudaSuccess)
-      e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, PS::NT, SMEM);
-    if (e != cudaSuccess) return e;
-    if (per_sm < 1) return cudaErrorInvalidConfiguration;
-  }
-  const int grid = STAGES == 1 ? g.nb : std::max(1, std::min(g.nb, sms * per_sm));
+  static SharedMemory shared;
+  static Resident resident;
+  if (cudaError_t e = shared.allow(kern, SMEM)) return e;
+  int fit = 0;  // CTAs the device holds at once
+  if (cudaError_t e = resident.ctas(kern, PS::NT, SMEM, &fit)) return e;
+  const int grid = STAGES == 1 ? g.nb : std::max(1, std::min(g.nb, fit));
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(grid);
   cfg.blockDim = dim3(PS::NT);

@@ -26,6 +26,7 @@
 // and the general kernel walked cells with a division each (124 us on 7.9 M
 // cells of 24^3 blocks).
 #pragma once
+#include "attr.h"
 #include "bulk.cuh"
 #include "cells.cuh"
 #include "tile.cuh"
@@ -240,17 +241,8 @@ template <typename T, int FORM, int N, int VC>
 static cudaError_t sor_stream_one(const T* A, T* B, const T* s, const Geom& g, const SorArgs& a,
                                   cudaStream_t st) {
   auto kern = sor_stream_kernel<T, FORM, N, VC>;
-  // set once per process, to the most a ring may take
-  static bool attr_set = false;
-  if (!attr_set) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)kSorMaxSmem);
-    if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout,
-                               (int)cudaSharedmemCarveoutMaxShared);
-    if (e != cudaSuccess) return e;
-    attr_set = true;
-  }
+  static SharedMemory shared;
+  if (cudaError_t e = shared.allow(kern, kSorMaxSmem)) return e;
   SorRing r = SorRing::make(g, FORM == 2, sizeof(T));
   r.ranks = sor_split(g, r, sizeof(T));
   return launch_dependent(kern, g.nb * r.ranks, r.threads, r.bytes(), st, false, r.ranks, A, B, s,

@@ -13,6 +13,7 @@
 // Decomposition: one CTA per block; sweeps march each (i,j) column along k.
 #include <type_traits>
 
+#include "attr.h"
 #include "cells.cuh"
 #include "common.cuh"
 #include "kernels.h"
@@ -427,16 +428,8 @@ static cudaError_t residual_stream(double* out, const double* x, const double* b
   constexpr int S = N == 32 ? 4 : 6;
   using RS = ResStream<N, VC, MODE, S>;
   auto kern = residual_stream_kernel<N, VC, MODE, S>;
-  static bool attr_set = false;  // once per process, not a stream operation
-  if (!attr_set) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)RS::SMEM);
-    if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout,
-                               (int)cudaSharedmemCarveoutMaxShared);
-    if (e != cudaSuccess) return e;
-    attr_set = true;
-  }
+  static SharedMemory shared;
+  if (cudaError_t e = shared.allow(kern, RS::SMEM)) return e;
   const int parts = kr_parts(g);
   kern<<<dim3(g.nb, parts), RS::NT, RS::SMEM, st>>>(out, x, b, cf8, g, N / parts, partial, err);
   return cudaGetLastError();
