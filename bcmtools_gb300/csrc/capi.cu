@@ -412,7 +412,9 @@ static int impose(bcmg_ctx c, Field& f, bool homogeneous, cudaStream_t st) {
   return gather(c, f, select_ranges(c, 7, 7, false, true), homogeneous, st);
 }
 
-static int create_field(bcmg_ctx c, int dtype, int vc, int* out, bool host = false) {
+// st: the stream that zeroes a device field.
+static int create_field(bcmg_ctx c, int dtype, int vc, int* out, cudaStream_t st,
+                        bool host = false) {
   if (!c->registered) return fail(c, BCMG_USAGE, "no blocks registered");
   if (dtype != BCMG_F32 && dtype != BCMG_F64) return fail(c, BCMG_USAGE, "bad dtype %d", dtype);
   if (vc < 1 || c->nx / 2 < vc || c->ny / 2 < vc || c->nz / 2 < vc)
@@ -445,7 +447,7 @@ static int create_field(bcmg_ctx c, int dtype, int vc, int* out, bool host = fal
   } else {
     int rc = dev_alloc(c, &f.d, f.bytes);
     if (rc) return rc;
-    CUDA_TRY(c, cudaMemsetAsync(f.d, 0, f.bytes, c->stream));
+    CUDA_TRY(c, cudaMemsetAsync(f.d, 0, f.bytes, st));
   }
   CUDA_TRY(c, cudaEventCreateWithFlags(&f.ev, cudaEventDisableTiming));
   const int h = c->next_field++;
@@ -476,18 +478,20 @@ static bool drop_spare(bcmg_ctx c, bool second) {
   return any;
 }
 
-static int work_field(bcmg_ctx c, int dtype, int vc, int slot, int* out) {
+// A new one is zeroed on the caller's stream, where its first use follows: on the
+// context's own stream the zeros could land on what the call has already written.
+static int work_field(bcmg_ctx c, int dtype, int vc, int slot, int* out, cudaStream_t st) {
   const long key = ((long)dtype * 64 + vc) * 64 + slot;
   auto it = c->work.find(key);
   if (it != c->work.end() && c->fields.count(it->second)) {
     *out = it->second;
     return BCMG_SUCCESS;
   }
-  int rc = create_field(c, dtype, vc, out);
+  int rc = create_field(c, dtype, vc, out, st);
   // the SOR run and its tuner hold the second buffer while they ask for these
   const bool sor = slot == kSlotSorSecond || slot == 31 || slot == 34;
   if (rc == BCMG_MEMORY && slot != kSlotRecip && drop_spare(c, !sor))
-    rc = create_field(c, dtype, vc, out);
+    rc = create_field(c, dtype, vc, out, st);
   if (rc) return rc;
   c->work[key] = *out;
   return BCMG_SUCCESS;
@@ -1008,14 +1012,14 @@ BCMG_API int bcmg_set_boundary(bcmg_ctx c, const int* bc_type, const double* bc_
 
 BCMG_API int bcmg_field_create(bcmg_ctx c, int dtype, int vc, int* field) {
   if (!c || !field) return BCMG_USAGE;
-  int rc = create_field(c, dtype, vc, field);
-  if (rc == BCMG_MEMORY && drop_spare(c, true)) rc = create_field(c, dtype, vc, field);
+  int rc = create_field(c, dtype, vc, field, c->stream);
+  if (rc == BCMG_MEMORY && drop_spare(c, true)) rc = create_field(c, dtype, vc, field, c->stream);
   return rc;
 }
 
 BCMG_API int bcmg_field_create_host(bcmg_ctx c, int dtype, int vc, int* field) {
   if (!c || !field) return BCMG_USAGE;
-  return create_field(c, dtype, vc, field, true);
+  return create_field(c, dtype, vc, field, c->stream, true);
 }
 
 // Fields in host memory serve host code that sweeps its own bricks and
@@ -1260,7 +1264,7 @@ BCMG_API int bcmg_sor_run(bcmg_ctx c, int fid, int sid, const double* coef, doub
   bool fused = n_inner >= 1 && !c->bc_conflict && (smem <= kSorMaxSmem || streams) && !c->no_fusion;
   int rc = BCMG_SUCCESS;
   int wid, pid = -1;
-  if (fused && n_outer > 0 && (rc = work_field(c, f->dtype, f->vc, kSlotSorSecond, &wid))) {
+  if (fused && n_outer > 0 && (rc = work_field(c, f->dtype, f->vc, kSlotSorSecond, &wid, stream))) {
     // no room for a second buffer: a streamed shape is swept in place
     if (!(streams && rc == BCMG_MEMORY)) {
       cudaFreeAsync(d_coef, stream);
@@ -1277,7 +1281,7 @@ BCMG_API int bcmg_sor_run(bcmg_ctx c, int fid, int sid, const double* coef, doub
     // bulk copy per block): packed once here, it saves the padding's bytes
     // on every iteration.
     bool pack = pulled && form == 2 && n_outer >= kPackMinIters;
-    if (pack && (rc = work_field(c, f->dtype, f->vc, 34, &pid))) {
+    if (pack && (rc = work_field(c, f->dtype, f->vc, 34, &pid, stream))) {
       if (rc != BCMG_MEMORY) {
         cudaFreeAsync(d_coef, stream);
         return rc;
@@ -1389,7 +1393,7 @@ BCMG_API int bcmg_autotune_sor(bcmg_ctx c, int fid, int sid, const double* coef,
   if (!f) return fail(c, BCMG_USAGE, "unknown field %d", fid);
   if (iters < 1) iters = 1;
   int tid;
-  int rc = work_field(c, f->dtype, f->vc, 31, &tid);
+  int rc = work_field(c, f->dtype, f->vc, 31, &tid, c->stream);
   if (rc) return rc;
   f = get_field(c, fid);
   Field* t = get_field(c, tid);
@@ -1619,7 +1623,7 @@ static const double* op_recip(bcmg_ctx c, int op, int vc, cudaStream_t st) {
   const Field* a0 = get_field(c, it->second.fields[0]);
   if (!a0 || a0->dtype != BCMG_F64 || a0->vc != vc) return nullptr;
   int id;
-  if (work_field(c, BCMG_F64, vc, kSlotRecip, &id)) return nullptr;
+  if (work_field(c, BCMG_F64, vc, kSlotRecip, &id, st)) return nullptr;
   double* out = (double*)get_field(c, id)->d;
   prof_mark(c, K_OTHER, st, true);
   const cudaError_t e = launch_recip(out, (const double*)a0->d, geom_of(c, *a0), st);
@@ -1885,7 +1889,7 @@ BCMG_API int bcmg_jacobi_run(bcmg_ctx c, int op, int x, int b, double omega, int
   if (iters < 0) return fail(c, BCMG_USAGE, "iters < 0");
   cudaStream_t stream = S(c, st);
   int wid, rc;
-  if ((rc = work_field(c, fx->dtype, fx->vc, 32, &wid))) return rc;
+  if ((rc = work_field(c, fx->dtype, fx->vc, 32, &wid, stream))) return rc;
   fx = get_field(c, x); fb = get_field(c, b);
   Field* fw = get_field(c, wid);
   if (!jacobi_fusable(c, op, *fx)) {
@@ -1981,7 +1985,7 @@ BCMG_API int bcmg_autotune_jacobi(bcmg_ctx c, int op, int x, int b, double omega
     return BCMG_SUCCESS;  // separate launches: nothing to choose
   }
   int tid;
-  int rc = work_field(c, fx->dtype, fx->vc, 33, &tid);
+  int rc = work_field(c, fx->dtype, fx->vc, 33, &tid, c->stream);
   if (rc) return rc;
   fx = get_field(c, x);
   Field* t = get_field(c, tid);
@@ -2041,7 +2045,7 @@ BCMG_API int bcmg_jacobi_solve(bcmg_ctx c, int op, int x, int b, double omega, i
   if (!same_shape(fx, fb)) return fail(c, BCMG_USAGE, "field mismatch");
   cudaStream_t stream = S(c, st);
   int wid;
-  int rc = work_field(c, fx->dtype, fx->vc, 0, &wid);
+  int rc = work_field(c, fx->dtype, fx->vc, 0, &wid, stream);
   if (rc) return rc;
   fx = get_field(c, x); fb = get_field(c, b);
   Field* fw = get_field(c, wid);
@@ -2411,12 +2415,12 @@ static int bicgstab_core(bcmg_ctx c, int op, int x, int b, double omega, int n_p
   const int dt = fx->dtype, vc = fx->vc;
   int w[9];
   for (int k = 0; k < 9; k++) {
-    int rc = work_field(c, dt, vc, 1 + k, &w[k]);
+    int rc = work_field(c, dt, vc, 1 + k, &w[k], st);
     if (rc) return rc;
   }
   int wbest = -1;
   if (keep_best) {
-    int rc2 = work_field(c, dt, vc, 11, &wbest);
+    int rc2 = work_field(c, dt, vc, 11, &wbest, st);
     if (rc2) return rc2;
   }
   KrVecs v;
@@ -2495,14 +2499,14 @@ extern "C" BCMG_API int bcmg_bicgstab_mixed(bcmg_ctx c, int op, int x, int b, do
   const int vc = fx->vc, nseg = c->nseg;
   int wr64, wr32, wd32, wprev;
   int rc;
-  if ((rc = work_field(c, BCMG_F64, vc, 20, &wr64))) return rc;
-  if ((rc = work_field(c, BCMG_F32, vc, 21, &wr32))) return rc;
-  if ((rc = work_field(c, BCMG_F32, vc, 22, &wd32))) return rc;
-  if ((rc = work_field(c, BCMG_F64, vc, 23, &wprev))) return rc;
+  if ((rc = work_field(c, BCMG_F64, vc, 20, &wr64, st))) return rc;
+  if ((rc = work_field(c, BCMG_F32, vc, 21, &wr32, st))) return rc;
+  if ((rc = work_field(c, BCMG_F32, vc, 22, &wd32, st))) return rc;
+  if ((rc = work_field(c, BCMG_F64, vc, 23, &wprev, st))) return rc;
   int w32[10];
   for (int k = 0; k < 9; k++)
-    if ((rc = work_field(c, BCMG_F32, vc, 1 + k, &w32[k]))) return rc;
-  if ((rc = work_field(c, BCMG_F32, vc, 11, &w32[9]))) return rc;
+    if ((rc = work_field(c, BCMG_F32, vc, 1 + k, &w32[k], st))) return rc;
+  if ((rc = work_field(c, BCMG_F32, vc, 11, &w32[9], st))) return rc;
   if ((rc = seg_buffers(c, nseg))) return rc;
   fx = get_field(c, x); fb = get_field(c, b);
   Field *r64 = get_field(c, wr64), *r32 = get_field(c, wr32), *d32 = get_field(c, wd32);
@@ -2631,7 +2635,7 @@ extern "C" BCMG_API int bcmg_bicgstab_mixed(bcmg_ctx c, int op, int x, int b, do
     int w64[9];
     bool room = true;
     for (int k = 0; k < 9 && room; k++) {
-      rc = work_field(c, BCMG_F64, vc, 1 + k, &w64[k]);
+      rc = work_field(c, BCMG_F64, vc, 1 + k, &w64[k], st);
       if (rc == BCMG_MEMORY) room = false;  // the FP32-refined x stands
       else if (rc) return rc;
     }
