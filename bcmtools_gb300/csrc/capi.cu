@@ -245,6 +245,29 @@ static void dev_free(bcmg_ctx c, void* p, size_t bytes) {
   c->in_use -= bytes;
 }
 
+// The context's other allocations (tables, scratch, a call's own buffers).  Where
+// there is no room for one, the spare work fields are given back first; the calls
+// that hold one ask for nothing else meanwhile.
+static bool drop_spare(bcmg_ctx c, bool second);
+template <class Alloc>
+static cudaError_t with_room(bcmg_ctx c, Alloc&& alloc) {
+  cudaError_t e = alloc();
+  if (e != cudaErrorMemoryAllocation) return e;
+  cudaGetLastError();
+  if (!drop_spare(c, true)) return e;
+  e = alloc();
+  if (e == cudaErrorMemoryAllocation) cudaGetLastError();
+  return e;
+}
+template <class P>
+static cudaError_t dev_malloc(bcmg_ctx c, P** p, size_t bytes) {
+  return with_room(c, [&] { return cudaMalloc(p, bytes); });
+}
+template <class P>
+static cudaError_t dev_malloc_async(bcmg_ctx c, P** p, size_t bytes, cudaStream_t st) {
+  return with_room(c, [&] { return cudaMallocAsync(p, bytes, st); });
+}
+
 // Device face table: the reference's local face list (BlockManager::setFaceLists,
 // BlockManager.cpp:477-510) plus one entry per Dirichlet outer face.
 static void clear_graphs(bcmg_ctx c);
@@ -264,11 +287,11 @@ static int build_face_table(bcmg_ctx c) {
     for (int* q : {d_ld, d_id, d_sf, d_bt})
       if (q) cudaFreeAsync(q, st);
   };
-  if (cudaMallocAsync(reinterpret_cast<void**>(&d_ld), nbf * sizeof(int), st) != cudaSuccess ||
-      cudaMallocAsync(reinterpret_cast<void**>(&d_id), nbf * 4 * sizeof(int), st) != cudaSuccess ||
-      cudaMallocAsync(reinterpret_cast<void**>(&d_sf), nbf * sizeof(int), st) != cudaSuccess ||
+  if (dev_malloc_async(c, &d_ld, nbf * sizeof(int), st) != cudaSuccess ||
+      dev_malloc_async(c, &d_id, nbf * 4 * sizeof(int), st) != cudaSuccess ||
+      dev_malloc_async(c, &d_sf, nbf * sizeof(int), st) != cudaSuccess ||
       (!c->bctype.empty() &&
-       cudaMallocAsync(reinterpret_cast<void**>(&d_bt), nbf * sizeof(int), st) != cudaSuccess)) {
+       dev_malloc_async(c, &d_bt, nbf * sizeof(int), st) != cudaSuccess)) {
     release();
     return fail(c, BCMG_MEMORY, "face tables: device memory");
   }
@@ -375,7 +398,7 @@ static int ensure_side(bcmg_ctx c, size_t es) {
     c->d_side[k] = nullptr;
   }
   c->side_bytes = 0;
-  for (int k = 0; k < 2; k++) CUDA_TRY(c, cudaMalloc(&c->d_side[k], need));
+  for (int k = 0; k < 2; k++) CUDA_TRY(c, dev_malloc(c, &c->d_side[k], need));
   c->side_bytes = need;
   c->side_es = es;
   return BCMG_SUCCESS;
@@ -858,8 +881,8 @@ static int xch_run(bcmg_ctx c, int field, const bcmg_xch_entry* e, int n, void* 
   cudaStream_t st = S(c, stream);
   VcTask* d_t = nullptr;
   int64_t* d_o = nullptr;
-  CUDA_TRY(c, cudaMallocAsync(reinterpret_cast<void**>(&d_t), tasks.size() * sizeof(VcTask), st));
-  CUDA_TRY(c, cudaMallocAsync(reinterpret_cast<void**>(&d_o), off.size() * sizeof(int64_t), st));
+  CUDA_TRY(c, dev_malloc_async(c, &d_t, tasks.size() * sizeof(VcTask), st));
+  CUDA_TRY(c, dev_malloc_async(c, &d_o, off.size() * sizeof(int64_t), st));
   CUDA_TRY(c, cudaMemcpyAsync(d_t, tasks.data(), tasks.size() * sizeof(VcTask),
                               cudaMemcpyHostToDevice, st));
   CUDA_TRY(c, cudaMemcpyAsync(d_o, off.data(), off.size() * sizeof(int64_t),
@@ -926,11 +949,11 @@ static int seg_buffers(bcmg_ctx c, int nseg) {
   c->d_segsum = nullptr;
   c->h_segsum = nullptr;
   c->segbuf_cap = 0;
-  CUDA_TRY(c, cudaMalloc(&c->d_segflag, (size_t)nseg));
-  CUDA_TRY(c, cudaMalloc(&c->d_segscale, (size_t)nseg * sizeof(double)));
-  CUDA_TRY(c, cudaMalloc(&c->d_segmaxit, (size_t)nseg * sizeof(int)));
-  CUDA_TRY(c, cudaMalloc(&c->d_segeps2, (size_t)nseg * sizeof(double)));
-  CUDA_TRY(c, cudaMalloc(&c->d_segsum, (size_t)2 * nseg * sizeof(double)));
+  CUDA_TRY(c, dev_malloc(c, &c->d_segflag, (size_t)nseg));
+  CUDA_TRY(c, dev_malloc(c, &c->d_segscale, (size_t)nseg * sizeof(double)));
+  CUDA_TRY(c, dev_malloc(c, &c->d_segmaxit, (size_t)nseg * sizeof(int)));
+  CUDA_TRY(c, dev_malloc(c, &c->d_segeps2, (size_t)nseg * sizeof(double)));
+  CUDA_TRY(c, dev_malloc(c, &c->d_segsum, (size_t)2 * nseg * sizeof(double)));
   CUDA_TRY(c, cudaMallocHost(&c->h_segsum, (size_t)2 * nseg * sizeof(double)));
   c->segbuf_cap = nseg;
   return BCMG_SUCCESS;
@@ -966,8 +989,8 @@ BCMG_API int bcmg_set_segments(bcmg_ctx c, int nseg, const int* seg_first) {
   c->nseg = 1;
   c->seg_first.assign({0, c->nb});
   if (nseg > 1) {
-    CUDA_TRY(c, cudaMalloc(&c->d_seg_of, (size_t)c->nb * sizeof(int)));
-    CUDA_TRY(c, cudaMalloc(&c->d_seg_first, (size_t)(nseg + 1) * sizeof(int)));
+    CUDA_TRY(c, dev_malloc(c, &c->d_seg_of, (size_t)c->nb * sizeof(int)));
+    CUDA_TRY(c, dev_malloc(c, &c->d_seg_first, (size_t)(nseg + 1) * sizeof(int)));
     CUDA_TRY(c, cudaMemcpy(c->d_seg_of, of.data(), (size_t)c->nb * sizeof(int),
                            cudaMemcpyHostToDevice));
     CUDA_TRY(c, cudaMemcpy(c->d_seg_first, seg_first, (size_t)(nseg + 1) * sizeof(int),
@@ -1239,7 +1262,7 @@ BCMG_API int bcmg_sor_run(bcmg_ctx c, int fid, int sid, const double* coef, doub
     const float v = (float)coef[k];
     std::memcpy(hc.data() + nc * sizeof(double) + k * sizeof(float), &v, sizeof(float));
   }
-  CUDA_TRY(c, cudaMallocAsync((void**)&d_coef, cb, stream));
+  CUDA_TRY(c, dev_malloc_async(c, &d_coef, cb, stream));
   CUDA_TRY(c, cudaMemcpyAsync(d_coef, hc.data(), cb, cudaMemcpyHostToDevice, stream));
   CUDA_TRY(c, cudaStreamSynchronize(stream));  // hc is pageable and goes out of scope
   Geom g = geom_of(c, *f);
@@ -1473,9 +1496,9 @@ BCMG_API int bcmg_op_create_const(bcmg_ctx c, const double* cc, int* op) {
     j32[b * 8 + 7] = (a32 >= 0x1p-60f && a32 <= 0x1p+60f) ? 1.0f / j32[b * 8] : 0.0f;
     j64[b * 8 + 7] = (a64 >= 0x1p-60 && a64 <= 0x1p+60) ? 1.0 / j64[b * 8] : 0.0;
   }
-  CUDA_TRY(c, cudaMalloc(&r.d_cc, nb * 7 * sizeof(double)));
-  CUDA_TRY(c, cudaMalloc(&r.d_jc32, nb * 8 * sizeof(float)));
-  CUDA_TRY(c, cudaMalloc(&r.d_jc64, nb * 8 * sizeof(double)));
+  CUDA_TRY(c, dev_malloc(c, &r.d_cc, nb * 7 * sizeof(double)));
+  CUDA_TRY(c, dev_malloc(c, &r.d_jc32, nb * 8 * sizeof(float)));
+  CUDA_TRY(c, dev_malloc(c, &r.d_jc64, nb * 8 * sizeof(double)));
   CUDA_TRY(c, cudaMemcpy(r.d_cc, cc, nb * 7 * sizeof(double), cudaMemcpyHostToDevice));
   CUDA_TRY(c, cudaMemcpy(r.d_jc32, j32.data(), nb * 8 * sizeof(float), cudaMemcpyHostToDevice));
   CUDA_TRY(c, cudaMemcpy(r.d_jc64, j64.data(), nb * 8 * sizeof(double), cudaMemcpyHostToDevice));
@@ -1551,7 +1574,7 @@ BCMG_API int bcmg_op_fold_boundary(bcmg_ctx c, int op, int b, void* st) {
   if (!any) return BCMG_SUCCESS;
   cudaStream_t stream = S(c, st);
   int* d_code = nullptr;
-  CUDA_TRY(c, cudaMallocAsync((void**)&d_code, code.size() * sizeof(int), stream));
+  CUDA_TRY(c, dev_malloc_async(c, &d_code, code.size() * sizeof(int), stream));
   CUDA_TRY(c, cudaMemcpyAsync(d_code, code.data(), code.size() * sizeof(int),
                               cudaMemcpyHostToDevice, stream));
   Geom g = geom_of(c, *fb);
@@ -2201,7 +2224,7 @@ static int kr_scratch(bcmg_ctx c, int nseg) {
     cudaFree(c->d_kpart);
     c->d_kpart = nullptr;
     c->kpart_nb = 0;
-    CUDA_TRY(c, cudaMalloc(&c->d_kpart, (size_t)2 * kKrMaxParts * c->nb * sizeof(double)));
+    CUDA_TRY(c, dev_malloc(c, &c->d_kpart, (size_t)2 * kKrMaxParts * c->nb * sizeof(double)));
     c->kpart_nb = c->nb;
   }
   if (c->kseg_cap < nseg) {
@@ -2210,7 +2233,7 @@ static int kr_scratch(bcmg_ctx c, int nseg) {
     c->d_kseg = nullptr;
     c->h_kseg = nullptr;
     c->kseg_cap = 0;
-    CUDA_TRY(c, cudaMalloc(&c->d_kseg, (size_t)nseg * sizeof(KSeg)));
+    CUDA_TRY(c, dev_malloc(c, &c->d_kseg, (size_t)nseg * sizeof(KSeg)));
     CUDA_TRY(c, cudaMallocHost(&c->h_kseg, (size_t)nseg * sizeof(KSeg)));
     c->kseg_cap = nseg;
   }
