@@ -1214,13 +1214,19 @@ static long sor_key(int dtype, int n, int vc, int form) {
   return ((long)(dtype * 64 + n) * 8 + vc) * 4 + form;
 }
 
+// Whether the pull form covers a run: cubic blocks of its shapes, no face fed in
+// part (a side-buffer slot has no values for the quarters that no finer block
+// feeds), not a push-only context (bcmg_set_ghost_form).
+static bool sor_pulls(bcmg_ctx c, const Field& f, int form) {
+  return c->ghost_form != BCMG_GHOST_PUSH && c->nx == c->ny && c->ny == c->nz && c->whole_faces &&
+         sor_pull_ok((int)dsize(f.dtype), c->nx, f.vc, form);
+}
+
 // Kernel shape for a fused SOR sweep: forced, tuned, or the default -- the
-// pull form one CTA per block (7) where it applies (no face fed in part), else the staged-source
-// tile (1).  Push-only
-// contexts (bcmg_set_ghost_form) never get the pull form.
+// pull form one CTA per block (7) where it applies, else the staged-source
+// tile (1).
 static int sor_variant(bcmg_ctx c, const Field& f, int form) {
-  const bool cubic = c->nx == c->ny && c->ny == c->nz;
-  const bool pull_ok = c->ghost_form != BCMG_GHOST_PUSH && cubic && c->whole_faces && sor_pull_ok((int)dsize(f.dtype), c->nx, f.vc, form);
+  const bool pull_ok = sor_pulls(c, f, form);
   int v = c->sor_fixed;
   if (!v) {
     auto it = c->sor_tuned.find(sor_key(f.dtype, c->nx, f.vc, form));
@@ -1427,9 +1433,7 @@ BCMG_API int bcmg_autotune_sor(bcmg_ctx c, int fid, int sid, const double* coef,
   int bv = 1;
   double bt = 1e300;
   for (int v = 1; v < SV_COUNT; v++) {
-    if ((v == SV_PULL || v == SV_PULL_TILE) && (c->ghost_form == BCMG_GHOST_PUSH || !sor_pull_ok((int)dsize(f->dtype), c->nx, f->vc, form) ||
-                         c->nx != c->ny || c->ny != c->nz))
-      continue;
+    if ((v == SV_PULL || v == SV_PULL_TILE) && !sor_pulls(c, *f, form)) continue;
     CUDA_TRY(c, cudaMemcpyAsync(t->d, f->d, f->bytes, cudaMemcpyDeviceToDevice, c->stream));
     c->sor_fixed = v;
     rc = bcmg_sor_run(c, tid, sid, coef, omega, form, 1, 1, c->stream);  // warm-up
@@ -2019,7 +2023,9 @@ BCMG_API int bcmg_autotune_jacobi(bcmg_ctx c, int op, int x, int b, double omega
   CUDA_TRY(c, cudaEventCreate(&e0));
   CUDA_TRY(c, cudaEventCreate(&e1));
   CUDA_TRY(c, cudaEventCreate(&e2));
-  const bool only_push = c->nx == 32;  // 32^3 blocks have the push form alone
+  // 32^3 blocks have the push form alone, and so have faces fed in part
+  // (jacobi_choice): timing it as another would name one that never runs
+  const bool only_push = c->nx == 32 || !c->whole_faces;
   int bv = only_push ? kJacPush : kJacPullTile;
   double bt = 1e300;
   for (int v = kJacPush; v <= kJacPullPipe; v++) {
