@@ -487,6 +487,7 @@ __global__ void __launch_bounds__(256) kr_zero_pass_kernel(T* __restrict__ x1, T
     for (int q = 1; q < 7; q++) zz = xadd(zz, xmul(cf[q], T(0)));
     if (!(zz == T(0))) om = zz;
   }
+  const bool recip = !CC && sizeof(T) == 8 && op.rA0;
   constexpr int U = 4;
   const int nx = g.nx, ncol = g.nx * g.ny;
   const int z0 = blockIdx.y * zc, z1 = min(g.nz, z0 + zc);
@@ -503,7 +504,7 @@ __global__ void __launch_bounds__(256) kr_zero_pass_kernel(T* __restrict__ x1, T
         if (PRE == kPreP || PRE == kPreS) qv[v] = pre.q[o];
         if (!CC) {
           av[v] = op.A[0][o];
-          yv[v] = op.rA0 ? op.rA0[o] : T(0);
+          yv[v] = recip ? op.rA0[o] : T(0);
         }
       }
 #pragma unroll
@@ -514,7 +515,10 @@ __global__ void __launch_bounds__(256) kr_zero_pass_kernel(T* __restrict__ x1, T
         if (PRE == kPreS) r = xadd(xmul(na, qv[v]), r);                           // kr_s
         if (PRE != kPreNone) b[o] = r;
         if (PRE == kPreS || PRE == kPreCopy) row_ends(b + o, ij % nx, nx, g.vc);
-        x1[o] = positive_zero(xmul(om, CC ? sweep_div(r, c0, rc0) : field_div(r, av[v], yv[v])));
+        const T q = CC      ? sweep_div(r, c0, rc0)
+                    : recip ? field_div(r, av[v], yv[v])
+                            : xdiv(r, av[v]);
+        x1[o] = positive_zero(xmul(om, q));
       }
       o0 += (int64_t)V * g.sz;
     };

@@ -1,0 +1,95 @@
+"""GPU: sweeps with an operator of coefficient fields, the oracle's bits.  FP64 runs
+of four sweeps and more divide through stored reciprocals of Ap, shorter ones,
+single sweeps and FP32 by the division itself; a cell whose Ap is outside 2^-60 ..
+2^60, subnormal, zero or not finite has no reciprocal, and dividends may be zero,
+subnormal or not finite."""
+import numpy as np
+import pytest
+
+import bcmtools_gb300 as bg
+from oracle import pyoracle as po
+from tests.helpers import outer_dirichlet, small_octree
+
+pytestmark = pytest.mark.gpu
+
+SHAPES = [((8, 8, 8), 1), ((16, 16, 16), 2), ((4, 4, 4), 2), ((2, 2, 2), 1), ((24, 20, 12), 1), ((10, 6, 14), 3),
+          ((32, 32, 32), 1)]
+
+
+def same_bits(got, ref, mask, what):
+    """Bit for bit, any NaN equal to any."""
+    g, r = got[:, mask], ref[:, mask]
+    with np.errstate(invalid="ignore"):
+        bad = ~((np.isnan(g) & np.isnan(r)) | ((g == r) & (np.signbit(g) == np.signbit(r))))
+    assert not bad.any(), f"{what}: {bad.sum()} cells, first {g[bad][0]!r} {r[bad][0]!r}"
+
+
+def mask_of(n, vc):
+    out = [((np.arange(k + 2 * vc) < vc) | (np.arange(k + 2 * vc) >= k + vc)).astype(int) for k in n]
+    return (out[2][:, None, None] + out[1][None, :, None] + out[0][None, None, :]) <= 1
+
+
+def edge_values(rng, shape, dt):
+    """Ap at, just inside and just beyond the range of the stored reciprocals."""
+    a = rng.uniform(5.0, 8.0, size=shape)
+    top, eps = (60, np.finfo(np.float64).eps) if dt == "f64" else (60, np.finfo(np.float32).eps)
+    pool = np.array([2.0 ** -top, 2.0 ** -top * (1 - eps), 2.0 ** -top * (1 + eps), 2.0 ** top, 2.0 ** top * (1 - eps),
+                     2.0 ** top * (1 + eps), 2.0 ** (top + 1), 2.0 ** -(top + 1), 1e-310 if dt == "f64" else 1e-41,
+                     0.0, np.inf, 2.0 ** 100, 3.0, 1.0 / 3.0])
+    k = rng.random(shape) < 0.2
+    a[k] = rng.choice(pool, size=int(k.sum()))
+    return a * rng.choice([-1.0, 1.0], size=shape)
+
+
+@pytest.mark.parametrize("n,vc", SHAPES)
+@pytest.mark.parametrize("dt", ["f32", "f64"])
+@pytest.mark.parametrize("iters", [1, 3, 4, 5])
+@pytest.mark.parametrize("values", ["plain", "edges"])
+def test_jacobi_run(gpu_ok, n, vc, dt, iters, values):
+    tree = small_octree(periodic=(False, True, False), level=2 if max(n) < 16 else 1, radius=0.3)
+    bm = bg.BlockManager(0)
+    bm.register_octree(tree, n)
+    ld, nid, sf, _ = tree.neighbors()
+    m = po.OracleMesh(ld, nid, sf, n, vc)
+    bct, bcv = outer_dirichlet(tree, 0.25, periodic=(False, True, False))
+    bm.set_boundary(bct, bcv, bg.DIRICHLET_SOR)
+    rng = np.random.default_rng(5)
+    x, b, y = (bm.setDataClass(dt, vc) for _ in range(3))
+    T = x.dtype
+    with np.errstate(over="ignore"):
+        A = [rng.uniform(0.5, 1.0, size=x.shape).astype(T) for _ in range(7)]
+        A[0] = (edge_values(rng, x.shape, dt) if values == "edges" else rng.uniform(-8, -6, size=x.shape)).astype(T)
+    ax, ab = rng.uniform(-1, 1, size=x.shape).astype(T), rng.uniform(-1, 1, size=x.shape).astype(T)
+    if values == "edges":
+        # products of powers of two far apart: quotients at both ends of the range
+        ab *= 2.0 ** rng.integers(-40, 40, size=x.shape).astype(T)
+        ab[rng.random(x.shape) < 0.05] = 0.0
+        ax[rng.random(x.shape) < 0.02] = -0.0
+    fs = [bm.setDataClass(dt, vc) for _ in range(7)]
+    for f, a in zip(fs, A):
+        f.upload(a)
+    op = bm.op_fields(fs)
+    x.upload(ax)
+    b.upload(ab)
+    y.upload(ax)
+    inner = (slice(None),) + (slice(vc, -vc),) * 3
+    bm.jacobi_sweep(op, y, x, b, 0.8)
+    bm.jacobi_run(op, x, b, 0.8, iters)
+    ref, x1 = ax.copy(), np.zeros_like(ax)
+    with np.errstate(all="ignore"):
+        for k in range(iters):
+            m.jacobi(x1, ref, ab, 0.8, fields=A)
+            if k == 0:
+                same_bits(y.download()[inner].reshape(len(ax), -1), x1[inner].reshape(len(ax), -1), slice(None),
+                          f"sweep {n}")
+            ref[inner] = x1[inner]
+            m.vc_update(ref)
+            m.dirichlet(ref, bct, bcv, 0)
+    got = x.download()
+    if dt == "f64" and values == "plain":
+        same_bits(got, ref, mask_of(n, vc), f"run {n} {iters}")
+    else:
+        # C2F ghosts of FP32 fields may be an ulp off, and interpolation of values at
+        # the ends of the range need not be: the first sweep's interiors are exact
+        if iters == 1:
+            same_bits(got[inner].reshape(len(ax), -1), ref[inner].reshape(len(ax), -1), slice(None), f"run {n}")
