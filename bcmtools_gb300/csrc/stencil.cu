@@ -151,7 +151,9 @@ static cudaError_t launch_sweep(T* out, const T* x, const T* b, const Op<T>& op,
   const int zc = MODE == 2 ? g.nz : sweep_chunk(g);
   const dim3 grid(g.nb, (g.nz + zc - 1) / zc);
   const int nt = column_threads(g);
-  constexpr int UC = sizeof(T) == 4 ? 4 : 2, UF = 2;
+  // calc_r in FP32: two planes a round (1408 blocks of 28^3: 118 us, with four 162;
+  // 20^3 42 and 55; 288 blocks 15.0 and 17.2)
+  constexpr int UC = sizeof(T) == 4 && MODE != 1 ? 4 : 2, UF = 2;
   if (op.cc)
     sweep_kernel<T, true, MODE, UC><<<grid, nt, 0, st>>>(out, x, b, op, g, omega, zc, partial);
   else if (MODE == 3 && sizeof(T) == 8 && op.rA0)

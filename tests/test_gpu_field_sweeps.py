@@ -86,6 +86,10 @@ def test_jacobi_run(gpu_ok, n, vc, dt, iters, values):
             m.vc_update(ref)
             m.dirichlet(ref, bct, bcv, 0)
     got = x.download()
+    y.upload(ax)
+    for _ in range(iters):  # never through reciprocals
+        bm.jacobi_run(op, y, b, 0.8, 1)
+    same_bits(got, y.download(), mask_of(n, vc), f"run of {iters} against single sweeps {n}")
     if dt == "f64" and values == "plain":
         same_bits(got, ref, mask_of(n, vc), f"run {n} {iters}")
     else:
@@ -93,3 +97,46 @@ def test_jacobi_run(gpu_ok, n, vc, dt, iters, values):
         # the ends of the range need not be: the first sweep's interiors are exact
         if iters == 1:
             same_bits(got[inner].reshape(len(ax), -1), ref[inner].reshape(len(ax), -1), slice(None), f"run {n}")
+
+
+@pytest.mark.parametrize("n,vc", SHAPES + [((20, 20, 20), 1), ((28, 28, 28), 2), ((16, 16, 18), 1), ((12, 10, 6), 2)])
+@pytest.mark.parametrize("dt", ["f32", "f64"])
+@pytest.mark.parametrize("fields", [False, True])
+def test_residuals(gpu_ok, n, vc, dt, fields):
+    """b - A x and A x bit for bit, and |b - A x|^2: a sum of N squares in FP64 in
+    any order is within 2 N 2^-53 of their exact sum."""
+    tree = small_octree(periodic=(False, True, False), level=2 if max(n) < 16 else 1, radius=0.3)
+    bm = bg.BlockManager(0)
+    bm.register_octree(tree, n)
+    ld, nid, sf, _ = tree.neighbors()
+    m = po.OracleMesh(ld, nid, sf, n, vc)
+    rng = np.random.default_rng(6)
+    x, b, y = (bm.setDataClass(dt, vc) for _ in range(3))
+    T = x.dtype
+    ax, ab = rng.uniform(-1, 1, size=x.shape).astype(T), rng.uniform(-1, 1, size=x.shape).astype(T)
+    x.upload(ax)
+    b.upload(ab)
+    if fields:
+        A = [rng.uniform(0.5, 1.0, size=x.shape).astype(T) for _ in range(7)]
+        fs = [bm.setDataClass(dt, vc) for _ in range(7)]
+        for f, a in zip(fs, A):
+            f.upload(a)
+        op, kw = bm.op_fields(fs), dict(fields=A)
+    else:
+        cc = bg.laplace_coef(np.stack([tree.block_sizes / k for k in n], 1) * np.array([1.0, 0.75, 1.5]))
+        op, kw = bm.op_const(cc), dict(cc=cc)
+    inner = (slice(None),) + (slice(vc, -vc),) * 3
+    ref = np.zeros_like(ax)
+    m.calc_ax(ref, ax, **kw)
+    bm.calc_ax(op, y, x)
+    assert np.array_equal(y.download()[inner], ref[inner])
+    m.calc_r(ref, ax, ab, **kw)
+    bm.calc_r(op, y, x, b)
+    assert np.array_equal(y.download()[inner], ref[inner])
+    r = ref[inner].astype(np.longdouble).ravel()
+    exact = (r * r).sum()
+    rr = bm.calc_r2(op, x, b)
+    assert rr == bm.calc_r2(op, x, b)
+    assert abs(rr - exact) <= 2 * r.size * 2.0 ** -53 * exact
+    bm.calc_r(op, b, x, b)  # in place
+    assert np.array_equal(b.download()[inner], ref[inner])
