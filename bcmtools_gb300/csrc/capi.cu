@@ -1689,11 +1689,16 @@ BCMG_API int bcmg_jacobi_sweep(bcmg_ctx c, int op, int x1, int x0, int b, double
   return jacobi_sweep(c, op, *f1, *f0, *fb, omega, S(c, st));
 }
 
+// Partial sums per block that launch_residual leaves in mode 2.
+static int residual_sums(const double* cc, const Geom& g, size_t es, bool streamed) {
+  if (streamed) return kr_parts(g);
+  return cubic_residuals(cc != nullptr, g) ? 1 : sum_parts(g, es);
+}
+
 // nsums (mode 2): the partial sums left for finish_reduce.
 static int residual(bcmg_ctx c, int op, Field* out, Field& x, Field* b, int mode, cudaStream_t st,
                     int* nsums = nullptr) {
   Geom g = geom_of(c, x);
-  if (nsums) *nsums = c->nb;
   if (x.dtype == BCMG_F64) {
     Op<double> o;
     int rc = make_op(c, op, x, &o);
@@ -1702,7 +1707,7 @@ static int residual(bcmg_ctx c, int op, Field* out, Field& x, Field* b, int mode
     const bool streamed = !x.host && !(b && b->host) && plane_stream_enabled() &&
                           residual_streams(sizeof(double), o.cc != nullptr, g) &&
                           stream_aligned<double>(g, x.d, b ? b->d : x.d);
-    if (nsums && streamed) *nsums = c->nb * kr_parts(g);
+    if (nsums) *nsums = c->nb * residual_sums(o.cc, g, sizeof(double), streamed);
     LAUNCH(c, K_RESIDUAL, st, launch_residual<double>(out ? (double*)out->d : nullptr, (const double*)x.d,
                                       b ? (const double*)b->d : nullptr, o, g, mode, streamed,
                                       c->d_partial, c->d_err, st));
@@ -1710,6 +1715,7 @@ static int residual(bcmg_ctx c, int op, Field* out, Field& x, Field* b, int mode
     Op<float> o;
     int rc = make_op(c, op, x, &o);
     if (rc) return rc;
+    if (nsums) *nsums = c->nb * residual_sums(o.cc, g, sizeof(float), false);
     LAUNCH(c, K_RESIDUAL, st, launch_residual<float>(out ? (float*)out->d : nullptr, (const float*)x.d,
                                      b ? (const float*)b->d : nullptr, o, g, mode, false,
                                      c->d_partial, c->d_err, st));

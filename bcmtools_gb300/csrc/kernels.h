@@ -263,7 +263,8 @@ cudaError_t launch_jacobi_fused(const T* x0, T* x1, const T* b, const Geom& g, c
                                 cudaStream_t st, bool pdl = false);
 // mode 0: ax = A x;  mode 1: r = b - A x;  mode 2: partial[b] = sum r^2 (no store).
 // streamed (residual_streams, device memory aligned to 16 bytes): the FP64 planes
-// stream through shared memory, and mode 2 leaves kr_parts sums per block.
+// stream through shared memory, and mode 2 leaves kr_parts sums per block.  Else it
+// leaves one, or sum_parts where the cubic kernels do not apply (cubic_residuals).
 template <typename T>
 cudaError_t launch_residual(T* out, const T* x, const T* b, Op<T> op, const Geom& g, int mode,
                             bool streamed, double* partial, int* err, cudaStream_t st);
@@ -324,6 +325,25 @@ inline int kr_parts(const Geom& g) {
   return n < 1 ? 1 : n > 4 ? 4 : n;
 }
 constexpr int kKrMaxParts = 4;
+// Parts per block of calc_r2 on blocks of any shape and coefficient fields, a
+// partial sum each.  A CTA a block left few blocks to walk alone: 64 blocks of
+// 28^3, FP64 fields, 220 us, in four parts 60 (fields read plane by plane, 160);
+// 288 of 32^3, FP32, 130 and 86.  FP64 gains at every count (1408 of 28^3: 1027 and
+// 932), and so do blocks of four parts in FP32 (267 and 252); smaller ones lose in
+// FP32 from four CTAs an SM on (512 of 16^3: 17 us, in two parts 19).
+inline int sum_parts(const Geom& g, size_t es) {
+  const int most = kr_parts(g);
+  if (es == 8 || most == kKrMaxParts) return most;
+  int n = 1;
+  while (n < most && g.nb * (n + 1) <= kSplitCtas) n++;
+  return n;
+}
+// Whether calc_ax / calc_r / calc_r2 have the kernels of cubic blocks with a
+// constant operator.
+inline bool cubic_residuals(bool constant_op, const Geom& g) {
+  return constant_op && g.nx == g.ny && g.ny == g.nz && (g.vc == 1 || g.vc == 2) &&
+         (g.nx == 8 || g.nx == 16 || g.nx == 32);
+}
 inline bool residual_streams(size_t es, bool constant_op, const Geom& g) {
   return es == 8 && constant_op && g.nx == g.ny && g.ny == g.nz && (g.nx == 16 || g.nx == 32) &&
          (g.vc == 1 || g.vc == 2);

@@ -39,7 +39,7 @@ __device__ __forceinline__ double block_sum(double v, double* red) {
 
 // ---------------------------------------------------------------------------
 // Sweeps over blocks of any shape and operators of coefficient fields:
-//   MODE 0 calc_ax, 1 calc_r, 2 calc_r2 (FP64 per-block partials), 3
+//   MODE 0 calc_ax, 1 calc_r, 2 calc_r2 (an FP64 partial sum per CTA, sum_parts), 3
 //   jacobi_smoother: x1 = x0 - omega (x0 - r/Ap),
 //   r = b - Aw xW - Ae xE - As xS - An xN - Ab xB - At xT.
 // CC: per-block constants cf8 (rounded to T, RN(1/Ap) last); else the fields, and
@@ -63,7 +63,7 @@ __global__ void __launch_bounds__(256) sweep_kernel(T* __restrict__ out, const T
                                                     const T* __restrict__ bb, Op<T> op, Geom g,
                                                     T omega, int zc,
                                                     double* __restrict__ partial) {
-  __shared__ double red[32];
+  __shared__ double red[MODE == 2 ? 256 : 1];
   const int b = blockIdx.x;
   const int64_t base = (int64_t)b * g.bstride;
   const int nx = g.nx, ncol = g.nx * g.ny, sy = g.sy, sz = g.sz;
@@ -140,20 +140,26 @@ __global__ void __launch_bounds__(256) sweep_kernel(T* __restrict__ out, const T
     for (; k < z1; k++) planes(std::integral_constant<int, 1>{});
   }
   if (MODE == 2) {
-    acc = block_sum(acc, red);
-    if (threadIdx.x == 0) partial[b] = acc;
+    // one tree in two forms: up to four warps gain nothing from packing their pairs
+    double none = 0.0;
+    if (blockDim.x <= 128) acc = block_sum(acc, red);
+    else kr_block_sums<1>(acc, none, red);
+    if (threadIdx.x == 0) partial[b * gridDim.y + blockIdx.y] = acc;
   }
 }
 
 template <typename T, int MODE>
 static cudaError_t launch_sweep(T* out, const T* x, const T* b, const Op<T>& op, const Geom& g,
                                 T omega, double* partial, cudaStream_t st) {
-  const int zc = MODE == 2 ? g.nz : sweep_chunk(g);
+  const int parts = sum_parts(g, sizeof(T));
+  const int zc = MODE == 2 ? (g.nz + parts - 1) / parts : sweep_chunk(g);
   const dim3 grid(g.nb, (g.nz + zc - 1) / zc);
   const int nt = column_threads(g);
-  // calc_r in FP32: two planes a round (1408 blocks of 28^3: 118 us, with four 162;
-  // 20^3 42 and 55; 288 blocks 15.0 and 17.2)
-  constexpr int UC = sizeof(T) == 4 && MODE != 1 ? 4 : 2, UF = 2;
+  // planes a round: two for calc_r in FP32 (1408 blocks of 28^3: 118 us, with four
+  // 162; 20^3 42 and 55; 288 blocks 15.0 and 17.2), one for calc_r2 in FP64 with
+  // fields (8^3, 288 blocks: 8.6 us, with two 9.3)
+  constexpr int UC = sizeof(T) == 4 && MODE != 1 ? 4 : 2;
+  constexpr int UF = sizeof(T) == 8 && MODE == 2 ? 1 : 2;
   if (op.cc)
     sweep_kernel<T, true, MODE, UC><<<grid, nt, 0, st>>>(out, x, b, op, g, omega, zc, partial);
   else if (MODE == 3 && sizeof(T) == 8 && op.rA0)
@@ -193,8 +199,7 @@ cudaError_t launch_recip(double* out, const double* a, const Geom& g, cudaStream
 
 template <typename T>
 static bool cubic_fast(const Op<T>& op, const Geom& g) {
-  return op.cc && op.cf8 && g.nx == g.ny && g.ny == g.nz && (g.vc == 1 || g.vc == 2) &&
-         (g.nx == 8 || g.nx == 16 || g.nx == 32);
+  return cubic_residuals(op.cc && op.cf8, g);
 }
 
 // jacobi_smoother on cubic blocks with a per-block constant operator: the
