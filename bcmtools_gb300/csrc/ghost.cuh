@@ -212,13 +212,15 @@ __device__ __forceinline__ void task_apply(const VcTask& t, T* __restrict__ dst,
   const Box B = task_box(t, g);
   const int cnt = B.b[0] * B.b[1] * B.b[2];
   const int bxy = B.b[0] * B.b[1];
-  // cell `lane` of the box, and the step to the worker's next cell: one
-  // division each, not one a cell (box extents are any even numbers)
-  int i, j, k, di, dj, dk, rem;
+  // cell `lane` of the box, and the step to the worker's next cell where it has one:
+  // one division each, not one a cell (box extents are any even numbers)
+  int i, j, k, di = 0, dj = 0, dk = 0, rem;
   divmod(lane, bxy, k, rem);
   divmod(rem, B.b[0], j, i);
-  divmod(nl, bxy, dk, rem);
-  divmod(rem, B.b[0], dj, di);
+  if (nl < cnt) {
+    divmod(nl, bxy, dk, rem);
+    divmod(rem, B.b[0], dj, di);
+  }
   const auto step = [&] {
     i += di;
     j += dj;

@@ -128,7 +128,9 @@ struct SorRing {
   size_t bytes() const { return 128 + (size_t)slots * slot; }
 };
 // Whether that pass covers a run: one inner pass, whole 16-byte planes, a ring
-// within shared memory.  FP64 blocks of up to 256 cells stay staged whole (575
+// within shared memory.  FP32 blocks of up to 64 cells stay staged whole up to four
+// per SM (288 blocks of 4^3: 7.4 us an iteration, streamed 8.8; 1408: 19.0 and 14.5),
+// FP64 blocks of up to 256 cells stay staged whole (575
 // blocks of 4^3: 17.9 us an iteration, streamed 20.1), so do many with planes of
 // less than 40 cell pairs (8x6x24, 2491 blocks: 181 and 197; 575: 64 and 62), and
 // bricks too large for that are swept in place unless the rounds of 256 threads
@@ -137,7 +139,7 @@ struct SorRing {
 inline bool sor_streams(const Geom& g, bool src, int n_inner, size_t es) {
   const SorRing r = SorRing::make(g, src, es);
   if (n_inner != 1 || (g.sz * es) % 16 != 0 || r.bytes() > kSorMaxSmem) return false;
-  if (es == 4) return true;
+  if (es == 4) return g.nx * g.ny * g.nz > 64 || g.nb > kSplitCtas;
   const int np = g.nx / 2 * g.ny, rounds = (np + r.threads - 1) / r.threads;
   const size_t whole = (size_t)(g.nx + 2) * (g.ny + 2) * (g.nz + 2) * es;
   return g.nx * g.ny * g.nz > 256 && (np >= 40 || g.nb < 1024) &&

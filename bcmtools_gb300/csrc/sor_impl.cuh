@@ -83,23 +83,20 @@ __global__ void __launch_bounds__(512, 2) sor_kernel(const T* A, T* Bf,
   const T* __restrict__ sbk = (FORM == 2) ? s + (int64_t)b * g.bstride : nullptr;
   const int nx = g.nx, ny = g.ny, nz = g.nz;
   const int lx = nx + 2, ly = ny + 2, lz = nz + 2;
-  // block constants, loaded before the staging is waited for
+  // block constants: loaded ahead of the staging, looked at after it (a branch on one
+  // here would hold the staging back by a trip to memory: 4^3, FP32, 512 blocks,
+  // two inner passes 11.8 us, so 9.3).  FP64 takes boundary values where a face has
+  // one: six more doubled on the FP64 pipe by every warp show (2^3: 6.4 and 6.1).
   SorCell<T, FORM> cell;
   cell.init(a, b);
-  const unsigned dmask = dirichlet_mask(a, b);
-  const bool anyd = dmask != 0;
-  bool dir[6];
+  int bt[6];
   double dv[6];
 #pragma unroll
   for (int fc = 0; fc < 6; fc++) {
-    dir[fc] = (dmask >> fc) & 1;
-    dv[fc] = a.bc.value[b * 6 + fc];
-    if (a.bc.bcx) dv[fc] = (double)(T)dv[fc];
+    bt[fc] = a.bc.type ? a.bc.type[b * 6 + fc] : 0;
+    if (sizeof(T) == 4) dv[fc] = a.bc.value[b * 6 + fc];
   }
-  const int es = PUSH ? entry_shift(g) : 5;
-  const int p0 = PUSH ? a.push.ptr[b] + (tid >> es) : 0, p1 = PUSH ? a.push.ptr[b + 1] : 0;
-  // this thread's first ghost entry, towards L1
-  if (p0 < p1) asm volatile("prefetch.global.L1 [%0];" ::"l"(a.push.tasks + p0));
+  const int pb = PUSH ? a.push.ptr[b] : 0, p1 = PUSH ? a.push.ptr[b + 1] : 0;
   T* base;
   int sy, sz, o;
   if (SMEM) {
@@ -112,9 +109,21 @@ __global__ void __launch_bounds__(512, 2) sor_kernel(const T* A, T* Bf,
       T* d = base + row * lx;
       for (int i = lane; i < lx; i += 32) d[i] = src[i];
     }
-    __syncthreads();
   } else {
     base = fb; sy = g.sy; sz = g.sz; o = g.off0;
+  }
+  // a warp per ghost entry, or where a block of few cells has more of them than the
+  // CTA has warps, a part of one (entry_shift); this thread's first one towards L1
+  const int es = PUSH && p1 - pb > nw ? entry_shift(g) : 5, p0 = pb + (tid >> es);
+  if (PUSH && p0 < p1) asm volatile("prefetch.global.L1 [%0];" ::"l"(a.push.tasks + p0));
+  if (SMEM) __syncthreads();
+  bool dir[6], anyd = false;
+#pragma unroll
+  for (int fc = 0; fc < 6; fc++) {
+    dir[fc] = bt[fc] == kBcDirichlet;
+    anyd |= dir[fc];
+    if (sizeof(T) == 8) dv[fc] = dir[fc] ? a.bc.value[b * 6 + fc] : 0.0;
+    if (a.bc.bcx) dv[fc] = (double)(T)dv[fc];
   }
 
   // Fixed per-thread (i2, j, k0) when a whole number of k-slices fits the CTA.
