@@ -135,15 +135,26 @@ struct SorRing {
 // less than 40 cell pairs (8x6x24, 2491 blocks: 181 and 197; 575: 64 and 62), and
 // bricks too large for that are swept in place unless the rounds of 256 threads
 // over a plane are nearly full (28^3: 410 us in place, 462 streamed at 77 %;
-// 32^3: 617 and 478).
+// 32^3: 617 and 478) -- without a source also where the in-place sweep's CTAs, one
+// per SM at a time, nearly fill one or two waves (152 blocks of 32^3: 117 us, 123
+// streamed; 304: 217 and 225).
 inline bool sor_streams(const Geom& g, bool src, int n_inner, size_t es) {
   const SorRing r = SorRing::make(g, src, es);
   if (n_inner != 1 || (g.sz * es) % 16 != 0 || r.bytes() > kSorMaxSmem) return false;
   if (es == 4) return g.nx * g.ny * g.nz > 64 || g.nb > kSplitCtas;
   const int np = g.nx / 2 * g.ny, rounds = (np + r.threads - 1) / r.threads;
   const size_t whole = (size_t)(g.nx + 2) * (g.ny + 2) * (g.nz + 2) * es;
+  const bool waves = !src && g.nb <= 304 && (g.nb + 56) % 152 < 57;  // 96..152 of 152
   return g.nx * g.ny * g.nz > 256 && (np >= 40 || g.nb < 1024) &&
-         (whole <= kSorMaxSmem || 10 * np >= 9 * rounds * r.threads);
+         (whole <= kSorMaxSmem || (10 * np >= 9 * rounds * r.threads && !waves));
+}
+// FP32 32^3 blocks that stay staged whole, one CTA per SM, where that is one nearly
+// full wave or, with two ghost layers and no source, two (form 1, us an iteration,
+// vc = 1 and 2: 80 blocks 28.7 and 25.6, streamed 30.3 and 30.8; 125: 29.0, 26.6 and
+// 36.6, 38.1; 304: 53.9, 52.1 and 51.9, 58.3; 64: 28.6, 25.3 and 25.3, 25.3; form 2,
+// vc = 1: 80 blocks 32.9, streamed 31.3; 125: 33.0 and 37.8).
+inline bool sor_staged_32(const Geom& g, bool src) {
+  return (g.nb > (src && g.vc == 1 ? 114 : 76) && g.nb <= 152) || (!src && g.vc == 2 && g.nb > 228 && g.nb <= 304);
 }
 
 // Kernel shapes of the fused sweep, chosen per (dtype, N, VC, scheme) by the

@@ -602,8 +602,9 @@ cudaError_t launch_sor_impl(const T* A, T* B, const T* s, const Geom& g, const d
   if (variant == SV_PULL || variant == SV_PULL_TILE) variant = SV_AUTO;
   // 32^3 blocks (their default and staged-source shape) and blocks of no
   // special shape
-  const bool staged = variant == SV_AUTO || variant == SV_TILE_SS_256;
-  if (fused && (!tile_ok<T>(g) || (g.nx == 32 && staged)) &&
+  const bool streamed_32 = g.nx == 32 && (variant == SV_AUTO || variant == SV_TILE_SS_256) &&
+                           !(sizeof(T) == 4 && sor_staged_32(g, form == 2));
+  if (fused && (!tile_ok<T>(g) || streamed_32) &&
       sor_stream_ok<T>(g, A, form == 2 ? s : nullptr, n_inner))
     return form == 1 ? launch_sor_stream<T, 1>(A, B, s, g, a, st)
                      : launch_sor_stream<T, 2>(A, B, s, g, a, st);

@@ -226,11 +226,19 @@ static bool sor_stream_ok(const Geom& g, const T* A, const T* s, int n_inner) {
 }
 
 // CTAs per block: two, four or eight until there are three per SM in FP64 and for
-// 128-thread planes, two in FP32, each with six planes or more (it makes colour 0
-// of two planes more than its own).  342 blocks split in two: FP64 24^3 287 -> 233
-// us an iteration, 32^3 443 -> 394, FP32 8x6x24 36 -> 26 but 28^3 78 -> 85; 575
-// blocks: FP64 24^3 302 -> 334, FP32 69 -> 83.
+// 128-thread planes, two in FP32, each with a share of six planes or more (the last
+// one's may be smaller; a CTA makes colour 0 of two planes more than its own).  342
+// blocks split in two: FP64 24^3 287 -> 233 us an iteration, 32^3 443 -> 394, FP32
+// 8x6x24 36 -> 26 but 28^3 78 -> 85; 575 blocks: FP64 24^3 302 -> 334, FP32 69 -> 83.
+// FP64 with 256 threads has two CTAs on an SM at a time: blocks, or halves of them,
+// that come close to two per SM are left at that (24^3, us an iteration by CTAs per
+// block 1 / 2 / 4: 152 blocks 84, 70, 97; 216 115, 127, 120; 304 118, 132, 167; 32^3:
+// 152 blocks 130, 123, 157; 304 225, 235, 277).
 inline int sor_split(const Geom& g, const SorRing& ring, size_t es) {
+  if (es == 8 && ring.threads == 256) {
+    if (g.nb <= 304 && g.nb >= 228) return 1;
+    if (2 * g.nb <= 304 && 2 * g.nb >= 190 && g.nz >= 12) return 2;
+  }
   const int want = (es == 8 || ring.threads == 128 ? 3 : 2) * 152;
   int r = 1;
   while (r < 8 && g.nb * r < want && g.nz >= 2 * r * 6) r *= 2;
