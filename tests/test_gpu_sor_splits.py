@@ -71,3 +71,16 @@ def test_shares_of_456_blocks(gpu_ok):
     tree = tree_of((8, 8, 8), 0)
     for dt in ("f32", "f64"):
         compare(tree, (32, 32, 32), 1, dt, 2, iters=1)
+
+
+@pytest.mark.parametrize("n,vc", [((32, 32, 32), 1), ((32, 32, 32), 2), ((40, 40, 40), 1), ((32, 40, 34), 2)])
+@pytest.mark.parametrize("dt", ["f32", "f64"])
+@pytest.mark.parametrize("iters", [1, 2, 3, 4])
+def test_bricks_too_large_to_stage(gpu_ok, n, vc, dt, iters):
+    compare(tree_of((2, 2, 2), 0.15), n, vc, dt, 2, iters)
+
+
+@pytest.mark.parametrize("iters", [1, 2, 3])
+def test_first_pass_in_place(gpu_ok, iters):
+    """More blocks than SMs, no source, an odd number of passes."""
+    compare(tree_of((3, 3, 3), 0.3), (32, 32, 32), 1, "f64", 1, iters)
