@@ -17,6 +17,7 @@
 // faces) and every ghost value x1's interior feeds in the neighbours' bricks
 // of the output field, reading x1 from shared memory.
 #pragma once
+#include <algorithm>
 #include <type_traits>
 
 #include "attr.h"
@@ -195,12 +196,12 @@ __global__ void __launch_bounds__(N * N, (BrickStage<T, N, VC, true>::MIN_BLOCKS
     // FP64, one coefficient for all six neighbours: each product formed once
     // (stream.cuh), over the tile's interior -- nothing reads its raw values
     // again but this thread's, which are in registers -- and for the x and y
-    // ghosts, whose raw values the ghost cells written below need, beside it.
+    // ghosts, whose raw values the ghost cells written below need, beside it or over
+    // b's ghosts of the same cells (G_ROOM, stage.cuh).
     // 15 operations a cell instead of 20, the same bits; the sweep is bound by the
     // FP64 pipe.
     iso = one_coefficient(c1, c2, c3, c4, c5, c6);
     if (iso) {
-      T* gs = reinterpret_cast<T*>(smraw + L::G_OFF);
       T* own = xs + BL::at(i, j, 0);
       T xr[N];
 #pragma unroll
@@ -208,19 +209,22 @@ __global__ void __launch_bounds__(N * N, (BrickStage<T, N, VC, true>::MIN_BLOCKS
         xr[k] = own[k * LXY];
         own[k * LXY] = xmul(c1, xr[k]);
       }
-      gs[0 * NN + tid] = xmul(c1, xs[BL::at(-1, gpp, gq)]);
-      gs[1 * NN + tid] = xmul(c1, xs[BL::at(N, gpp, gq)]);
-      gs[2 * NN + tid] = xmul(c1, xs[BL::at(gpp, -1, gq)]);
-      gs[3 * NN + tid] = xmul(c1, xs[BL::at(gpp, N, gq)]);
+      constexpr bool R = L::G_ROOM;
+      constexpr int GP = R ? N : LXY;  // plane pitch of the ghosts' products
+      T* gs = R ? reinterpret_cast<T*>(smraw + L::G_OFF) : x1s;
+      gs[R ? tid : BL::at(-1, gpp, gq)] = xmul(c1, xs[BL::at(-1, gpp, gq)]);
+      gs[R ? NN + tid : BL::at(N, gpp, gq)] = xmul(c1, xs[BL::at(N, gpp, gq)]);
+      gs[R ? 2 * NN + tid : BL::at(gpp, -1, gq)] = xmul(c1, xs[BL::at(gpp, -1, gq)]);
+      gs[R ? 3 * NN + tid : BL::at(gpp, N, gq)] = xmul(c1, xs[BL::at(gpp, N, gq)]);
       T ym = xmul(c1, own[-LXY]);
       const T ytop = xmul(c1, own[N * LXY]);
       __syncthreads();
-      const T* pw = i > 0 ? own - 1 : gs + j;
-      const T* pe = i < N - 1 ? own + 1 : gs + NN + j;
-      const T* ps = j > 0 ? own - LX : gs + 2 * NN + i;
-      const T* pn = j < N - 1 ? own + LX : gs + 3 * NN + i;
-      const int sw = i > 0 ? LXY : N, se = i < N - 1 ? LXY : N;
-      const int ss = j > 0 ? LXY : N, sn = j < N - 1 ? LXY : N;
+      const T* pw = i > 0 ? own - 1 : R ? gs + j : bp - 1;
+      const T* pe = i < N - 1 ? own + 1 : R ? gs + NN + j : bp + 1;
+      const T* ps = j > 0 ? own - LX : R ? gs + 2 * NN + i : bp - LX;
+      const T* pn = j < N - 1 ? own + LX : R ? gs + 3 * NN + i : bp + LX;
+      const int sw = i > 0 ? LXY : GP, se = i < N - 1 ? LXY : GP;
+      const int ss = j > 0 ? LXY : GP, sn = j < N - 1 ? LXY : GP;
       T yc = own[0];
 #pragma unroll
       for (int k0 = 0; k0 < N; k0 += 4) {
@@ -1087,9 +1091,17 @@ static cudaError_t jacobi_tile_launch(const T* x0, T* x1, const T* b, const Geom
               : ki == 2 ? jacobi_tile_kernel<T, N, VC, false, true>
               : ki == 3 ? jacobi_tile_kernel<T, N, VC, true, true>
                         : jacobi_tile_kernel<T, N, VC, false, true, true>;
+  // FP64 16^3 at vc = 2, push form, up to 1024 blocks: one CTA per SM.  With two,
+  // blocks of many level-change entries keep an SM to themselves while others are
+  // done (us a sweep, one and two: two-level 258 blocks 71, 89; 288 62, 75; 643 130,
+  // 138; flat 288 48, 44; 512 89, 85; 729 117, 127).  Larger meshes and the pull form
+  // gain from two (1408 blocks 225, 211; 4136 616, 561).
+  constexpr size_t ALONE = 116 * 1024;  // more than half of an SM's
+  const bool alone = !pull && sizeof(T) == 8 && N == 16 && VC == 2 && g.nb <= 1024;
+  const size_t smem = alone ? std::max(ALONE, L::SMEM) : L::SMEM;
   static SharedMemory shared[5];
-  if (cudaError_t e = shared[ki].allow(kern, L::SMEM)) return e;
-  return launch_dependent(kern, g.nb, L::NT, L::SMEM, st, a.pdl, 1, x0, x1, b, g, a);
+  if (cudaError_t e = shared[ki].allow(kern, std::max(ALONE, L::SMEM))) return e;
+  return launch_dependent(kern, g.nb, L::NT, smem, st, a.pdl, 1, x0, x1, b, g, a);
 }
 
 template <typename T, int N, int VC>

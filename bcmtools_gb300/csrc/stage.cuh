@@ -20,9 +20,13 @@ struct BrickStage {
   static constexpr unsigned B_BYTES = SRC ? N * PB : 0;
   static constexpr unsigned X_OFF = 16;
   static constexpr unsigned B_OFF = X_OFF + X_BYTES;
-  // FP64: the four x and y ghost faces times the neighbours' one coefficient
+  // FP64: the four x and y ghost faces times the neighbours' one coefficient.  At
+  // vc = 2 they lie over the second field's own ghosts, which nothing reads: room of
+  // their own would leave 16^3 one CTA per SM instead of two, 8^3 eight instead of
+  // nine.  At vc = 1 it costs 16^3 none.
+  static constexpr bool G_ROOM = SRC && sizeof(T) == 8 && VC == 1;
   static constexpr unsigned G_OFF = B_OFF + B_BYTES;
-  static constexpr unsigned G_BYTES = SRC && sizeof(T) == 8 ? 4 * N * N * sizeof(T) : 0;
+  static constexpr unsigned G_BYTES = G_ROOM ? 4 * N * N * sizeof(T) : 0;
   static constexpr size_t SMEM = G_OFF + G_BYTES;
   static_assert(X_BYTES % 16 == 0 && PB % 16 == 0, "bulk copies need 16-byte sizes and offsets");
   // Rows j and j+D share a warp (N = 16): D*LX = 16 (mod 32) puts the two
