@@ -314,15 +314,20 @@ cudaError_t launch_xch(T* data, const Geom& g, const VcTask* ents, const int64_t
                        T* buf, bool pack, cudaStream_t st);
 
 // Whether the BiCGSTAB iteration's kernels are launched as dependents of one
-// another (launch_dependent, bulk.cuh): FP32 on blocks of at most 16^3, up to 1216
-// of them, where the gap between two launches is some per cent of a kernel (six
-// solves of 1001 blocks in all: 62.7 ms without, 60.0 with).  Not on larger meshes:
-// 1427 blocks 276 us an iteration without, 281 with; 2549 blocks 419 and 447; and
-// a dependent's waiting CTAs hold slots that other streams' kernels would take (200
+// another (launch_dependent, bulk.cuh): FP32 on blocks of at most 16^3, up to five
+// million cells, where the gap between two launches is some per cent of a kernel (us
+// an iteration without and with: 8^3, 512 blocks 57.7, 46.7; 2197 77.2, 66.1; 5152
+// 144, 126; 12^3, 1000 blocks 138, 122; 16^3, 64 blocks 67.7, 57.1; 1000 162.5, 160.1).
+// Not 16^3 in between: a waiting CTA of its streamed A.x holds shared memory that the
+// kernel before could use (216 blocks 78.5, 83.7; 512 98.8, 104.7; 729 123, 126).  Not
+// on larger meshes: 1427 blocks of 16^3 276 and 281, 2549 419 and 447; and a
+// dependent's waiting CTAs hold slots that other streams' kernels would take (200
 // served requests on four streams: median latency 8 s without, 12 s with, 5.88 and
 // 5.82 solves a second).  Nor in FP64 (342 blocks of 32^3: 38.6 ms without, 40.7).
 inline bool kr_dependent(size_t es, const Geom& g) {
-  return es == 4 && g.nx * g.ny * g.nz <= 4096 && g.nb <= 8 * 152;
+  const int cells = g.nx * g.ny * g.nz;
+  if (es != 4 || cells > 4096 || (int64_t)g.nb * cells > 8 * 152 * 4096) return false;
+  return !(g.nx == 16 && g.ny == 16 && g.nz == 16) || g.nb <= 152 || g.nb >= 800;
 }
 
 // Parts of a block's planes that the kernels with inner products take as CTAs of
