@@ -1863,7 +1863,8 @@ static int jacobi_choice(bcmg_ctx c, const Field& x) {
   return c->nb <= 1024 ? kJacPush : kJacPullTile;
 }
 
-// pre (with zero_x0): the vector update that makes b, fused into the launch (JacPre): kind, r, q and the segments' scalars.
+// pre (with zero_x0): the vector update that makes b, fused into the launch
+// (JacPre): kind, r, q and the segments' scalars.
 struct PreArgs {
   int kind;
   const Field* r;
@@ -2037,8 +2038,8 @@ BCMG_API int bcmg_autotune_jacobi(bcmg_ctx c, int op, int x, int b, double omega
   fx = get_field(c, x);
   Field* t = get_field(c, tid);
   // per-sweep cost: a run of 2*iters sweeps less a run of iters, so that a
-  // run's fixed costs (the closing ghost update of the pull forms, the work
-  // copy) do not favour one form in short tuning runs
+  // run's fixed costs (the closing ghost update of the pipelined form, the ghost
+  // planes copied beforehand) do not favour one form in short tuning runs
   cudaEvent_t e0, e1, e2;
   CUDA_TRY(c, cudaEventCreate(&e0));
   CUDA_TRY(c, cudaEventCreate(&e1));
@@ -2308,14 +2309,16 @@ static int kr_iteration(bcmg_ctx c, int op, const KrVecs& v, const Op<T>& o, KSe
   if ((rc = jacobi_pre(c, op, *v.p_, *v.x0, *v.p, omega, n_pre, st, true, fuse ? &pre_p : nullptr,
                        recip)))
     return rc;
-  LAUNCH(c, K_RESIDUAL, st, launch_kr_ax<T>(d(v.q_), d(v.p_), o, d(v.r0), 1, g, ax_parts, S, part, c->d_err, st));
+  LAUNCH(c, K_RESIDUAL, st, launch_kr_ax<T>(d(v.q_), d(v.p_), o, d(v.r0), 1, g, ax_parts, S, part,
+                                            c->d_err, st));
   LAUNCH(c, K_DOT, st, launch_kr_scalar(part, c->nb, ax_parts, S, KS_ALPHA, max_iter, eps2, keep_best,
                                      kr_dependent(sizeof(T), g), st));
   if (!fuse) LAUNCH(c, K_BLAS1, st, launch_kr_s<T>(d(v.s), d(v.r), d(v.q_), g, S, st));
   if ((rc = jacobi_pre(c, op, *v.s_, *v.x0, *v.s, omega, n_pre, st, true, fuse ? &pre_s : nullptr,
                        recip)))
     return rc;
-  LAUNCH(c, K_RESIDUAL, st, launch_kr_ax<T>(d(v.t_), d(v.s_), o, d(v.s), 2, g, ax_parts, S, part, c->d_err, st));
+  LAUNCH(c, K_RESIDUAL, st, launch_kr_ax<T>(d(v.t_), d(v.s_), o, d(v.s), 2, g, ax_parts, S, part,
+                                            c->d_err, st));
   LAUNCH(c, K_DOT, st, launch_kr_scalar(part, c->nb, ax_parts, S, KS_GAMMA, max_iter, eps2, keep_best,
                                      kr_dependent(sizeof(T), g), st));
   LAUNCH(c, K_BLAS1, st, launch_kr_xr<T>(d(v.x), d(v.r), d(v.p_), d(v.s_), d(v.s), d(v.t_),

@@ -586,11 +586,14 @@ __global__ void __launch_bounds__(N * N, (N == 8 ? 12 : sizeof(T) == 4 ? (VC == 
 template <typename T, int N, int VC>
 static cudaError_t jacobi_zero_push_launch(T* x1, T* b, const Geom& g, const JacArgs<T>& a,
                                            cudaStream_t st) {
+  const auto launch = [&](auto kern) {
+    return launch_dependent(kern, g.nb, N * N, 0, st, a.pdl, 1, x1, b, g, a);
+  };
   switch (a.pre.kind) {
-    case kPreP: return launch_dependent(jacobi_zero_push_kernel<T, N, VC, kPreP>, g.nb, N * N, 0, st, a.pdl, 1, x1, b, g, a);
-    case kPreS: return launch_dependent(jacobi_zero_push_kernel<T, N, VC, kPreS>, g.nb, N * N, 0, st, a.pdl, 1, x1, b, g, a);
-    case kPreCopy: return launch_dependent(jacobi_zero_push_kernel<T, N, VC, kPreCopy>, g.nb, N * N, 0, st, a.pdl, 1, x1, b, g, a);
-    default: return launch_dependent(jacobi_zero_push_kernel<T, N, VC, kPreNone>, g.nb, N * N, 0, st, a.pdl, 1, x1, b, g, a);
+    case kPreP: return launch(jacobi_zero_push_kernel<T, N, VC, kPreP>);
+    case kPreS: return launch(jacobi_zero_push_kernel<T, N, VC, kPreS>);
+    case kPreCopy: return launch(jacobi_zero_push_kernel<T, N, VC, kPreCopy>);
+    default: return launch(jacobi_zero_push_kernel<T, N, VC, kPreNone>);
   }
 }
 
@@ -682,9 +685,10 @@ __global__ void __launch_bounds__(N * N / CPT, sizeof(T) == 4 ? (CPT >= 4 ? 4 : 
 // neighbour's ghost cell as well (the same-level entries of the push table,
 // copies); in FP32 at vc = 1 so do the C2F and F2C entries of x faces, from
 // the block's outermost x1 columns staged in shared memory; jacobi_push_tail
-// then does the rest (edges, unfed faces, the other level-change entries).  ZERO: x0 == 0, only b is streamed.  PRE (with ZERO): b made
-// in the same pass from the BiCGSTAB vectors streamed instead (JacPre, the
-// operations of kr_p / kr_s) and written back.
+// then does the rest (edges, unfed faces, the other level-change entries).
+// ZERO: x0 == 0, only b is streamed.  PRE (with ZERO): b made in the same pass from
+// the BiCGSTAB vectors streamed instead (JacPre, the operations of kr_p / kr_s) and
+// written back.
 //
 // SPLIT: a thread-block cluster of 2, 4 or 8 CTAs takes a block, each its share
 // of the planes, and after a cluster barrier (every x1 plane is then in its brick,

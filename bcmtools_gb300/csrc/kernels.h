@@ -154,7 +154,8 @@ inline bool sor_streams(const Geom& g, bool src, int n_inner, size_t es) {
 // 36.6, 38.1; 304: 53.9, 52.1 and 51.9, 58.3; 64: 28.6, 25.3 and 25.3, 25.3; form 2,
 // vc = 1: 80 blocks 32.9, streamed 31.3; 125: 33.0 and 37.8).
 inline bool sor_staged_32(const Geom& g, bool src) {
-  return (g.nb > (src && g.vc == 1 ? 114 : 76) && g.nb <= 152) || (!src && g.vc == 2 && g.nb > 228 && g.nb <= 304);
+  return (g.nb > (src && g.vc == 1 ? 114 : 76) && g.nb <= 152) ||
+         (!src && g.vc == 2 && g.nb > 228 && g.nb <= 304);
 }
 
 // Kernel shapes of the fused sweep, chosen per (dtype, N, VC, scheme) by the

@@ -1,11 +1,12 @@
 // krylov.cu -- the device-resident BiCGSTAB iteration kernels (krylov.cuh).
 //
-// One CTA per block.  Cubic 8/16/32-cell blocks take N*N threads, one
-// (i, j) column each, the k walk unrolled so that a thread has several
-// planes' loads in flight; other block shapes loop over the columns.
-// Inner products: FP64 multiply-add per element along the column, then the
-// CTA's fixed-order tree (kr_block_sums); partial sums per block go to
-// partial[slot * nb + b] and kr_scalar reduces them per segment.
+// One CTA per block, or (inner products in FP64 and with coefficient fields) per
+// part of a block's planes (kr_parts).  Cubic 8/16/32-cell blocks take N*N threads,
+// one (i, j) column each, the k walk unrolled so that a thread has several planes'
+// loads in flight; other block shapes loop over the columns.  Inner products: FP64
+// multiply-add per element along the column, then the CTA's fixed-order tree
+// (kr_block_sums); part p of block b leaves its sums at partial[b * parts + p] and
+// nb * parts further on, and kr_scalar reduces them per segment.
 // The iteration's kernels may be launched as dependents of one another
 // (kr_dependent): each starts as the one before drains, and waits for it before
 // its first access.
@@ -273,8 +274,9 @@ static cudaError_t kr_ax_stream_one(T* out, const T* x, const T* cf8, const T* y
   auto kern = kr_ax_stream_kernel<T, N, VC, NDOT, S>;
   static SharedMemory shared;
   if (cudaError_t e = shared.allow(kern, AS::SMEM)) return e;
-  return launch_dependent(kern, dim3(g.nb, parts), AS::NT, AS::SMEM, st, kr_dependent(sizeof(T), g), 1, out, x,
-                          cf8, y0, g, N / parts, S_, partial, err);
+  return launch_dependent(kern, dim3(g.nb, parts), AS::NT, AS::SMEM, st,
+                          kr_dependent(sizeof(T), g), 1, out, x, cf8, y0, g, N / parts, S_,
+                          partial, err);
 }
 
 // Ring depths: 32^3 4 slots (FP32: 6 CTAs per SM, FP64: 3); 16^3 8 (FP32)
@@ -366,8 +368,8 @@ static cudaError_t kr_xr_stream(T* x, T* r, const T* p_, const T* s_, const T* s
   auto kern = kr_xr_stream_kernel<T, N, VC, S>;
   static SharedMemory shared;
   if (cudaError_t e = shared.allow(kern, XS::SMEM)) return e;
-  return launch_dependent(kern, g.nb, XS::NT, XS::SMEM, st, kr_dependent(sizeof(T), g), 1, x, r, p_, s_, s, t, r0, g, S_,
-                          partial, err);
+  return launch_dependent(kern, g.nb, XS::NT, XS::SMEM, st, kr_dependent(sizeof(T), g), 1, x, r,
+                          p_, s_, s, t, r0, g, S_, partial, err);
 }
 
 // x = alpha p^ + gamma s^ + x (AXPBYPZ, ILS3D.h:783, blas.f90:345-377) and
@@ -388,7 +390,8 @@ __global__ void __launch_bounds__(kr_nt<N>(), (kr_minb<T, N, true>())) kr_xr_ker
   DotAcc<T> a0, a1;
   constexpr bool PARTS = N == 0 || sizeof(T) == 8;  // else zc is nz
   const int nz = N ? N : g.nz, z0 = PARTS ? blockIdx.y * zc : 0;
-  kr_walk<N, (sizeof(T) == 4 && N != 32 ? 4 : 2)>(g, z0, PARTS ? min(nz, z0 + zc) : nz, [&](int64_t o0, auto vt) {
+  const int z1 = PARTS ? min(nz, z0 + zc) : nz;
+  kr_walk<N, (sizeof(T) == 4 && N != 32 ? 4 : 2)>(g, z0, z1, [&](int64_t o0, auto vt) {
     constexpr int V = decltype(vt)::value;
     T pv[V], sv_[V], xv[V], tv[V], sv[V], r0v[V];
 #pragma unroll
@@ -534,11 +537,14 @@ cudaError_t launch_kr_zero_pass(T* x1, T* b, const JacPre<T>& pre, const Op<T>& 
   if (g.nb == 0) return cudaSuccess;
   const int zc = sweep_chunk(g), nt = column_threads(g);
   const dim3 grid(g.nb, (g.nz + zc - 1) / zc);
-#define Z_(PRE)                                                                            \
-  if (op.cc)                                                                               \
-    return launch_dependent(kr_zero_pass_kernel<T, true, PRE>, grid, nt, 0, st, kr_dependent(sizeof(T), g), 1, x1, b, pre, op, g, omega, zc);   \
-  else                                                                                     \
-    return launch_dependent(kr_zero_pass_kernel<T, false, PRE>, grid, nt, 0, st, kr_dependent(sizeof(T), g), 1, x1, b, pre, op, g, omega, zc)
+  const bool pdl = kr_dependent(sizeof(T), g);
+#define Z_(PRE)                                                                             \
+  if (op.cc)                                                                                \
+    return launch_dependent(kr_zero_pass_kernel<T, true, PRE>, grid, nt, 0, st, pdl, 1, x1, \
+                            b, pre, op, g, omega, zc);                                      \
+  else                                                                                      \
+    return launch_dependent(kr_zero_pass_kernel<T, false, PRE>, grid, nt, 0, st, pdl, 1,    \
+                            x1, b, pre, op, g, omega, zc)
   switch (pre.kind) {
     case kPreP: Z_(kPreP); break;
     case kPreS: Z_(kPreS); break;
@@ -805,17 +811,22 @@ cudaError_t launch_kr_ax(T* out, const T* x, Op<T> op, const T* y0, int ndot, co
     return g.vc == 1 ? kr_ax_stream<T, 16, 1>(out, x, op.cf8, y0, ndot, g, parts, S, partial, err, st)
                      : kr_ax_stream<T, 16, 2>(out, x, op.cf8, y0, ndot, g, parts, S, partial, err, st);
   }
-#define C_(N)                                                                                     \
-  if (cc && ndot == 2)                                                                            \
-    return launch_dependent(kr_ax_kernel<T, N, true, 2>, grid, kr_threads<N>(g), 0, st, kr_dependent(sizeof(T), g), 1, out, x, op.cf8, op, y0, g, zc, S, partial);                      \
-  else if (cc)                                                                                    \
-    return launch_dependent(kr_ax_kernel<T, N, true, 1>, grid, kr_threads<N>(g), 0, st, kr_dependent(sizeof(T), g), 1, out, x, op.cf8, op, y0, g, zc, S, partial);                      \
-  else if (ndot == 2)                                                                             \
-    return launch_dependent(kr_ax_kernel<T, N, false, 2>, grid, kr_threads<N>(g), 0, st, kr_dependent(sizeof(T), g), 1, out, x, op.cf8, op, y0, g, zc, S, partial);                     \
-  else                                                                                            \
-    return launch_dependent(kr_ax_kernel<T, N, false, 1>, grid, kr_threads<N>(g), 0, st, kr_dependent(sizeof(T), g), 1, out, x, op.cf8, op, y0, g, zc, S, partial)
+  const bool pdl = kr_dependent(sizeof(T), g);
+#define A_(N, CC, ND)                                                                        \
+  return launch_dependent(kr_ax_kernel<T, N, CC, ND>, grid, kr_threads<N>(g), 0, st, pdl, 1, \
+                          out, x, op.cf8, op, y0, g, zc, S, partial)
+#define C_(N)                      \
+  if (cc && ndot == 2)             \
+    A_(N, true, 2);                \
+  else if (cc)                     \
+    A_(N, true, 1);                \
+  else if (ndot == 2)              \
+    A_(N, false, 2);               \
+  else                             \
+    A_(N, false, 1)
   KR_DISPATCH(C_)
 #undef C_
+#undef A_
   return cudaGetLastError();
 }
 
@@ -833,7 +844,9 @@ cudaError_t launch_kr_xr(T* x, T* r, const T* p_, const T* s_, const T* s, const
     return g.vc == 1 ? kr_xr_stream<T, 32, 1, 2>(x, r, p_, s_, s, t, r0, g, S, partial, err, st)
                      : kr_xr_stream<T, 32, 2, 2>(x, r, p_, s_, s, t, r0, g, S, partial, err, st);
 #define C_(N) \
-  return launch_dependent(kr_xr_kernel<T, N>, grid, kr_threads<N>(g), 0, st, kr_dependent(sizeof(T), g), 1, x, r, p_, s_, s, t, r0, g, zc, S, partial)
+  return launch_dependent(kr_xr_kernel<T, N>, grid, kr_threads<N>(g), 0, st,               \
+                          kr_dependent(sizeof(T), g), 1, x, r, p_, s_, s, t, r0, g, zc, S, \
+                          partial)
   KR_DISPATCH(C_)
 #undef C_
   return cudaGetLastError();

@@ -10,7 +10,8 @@
 //                          float-float, products outside [2^-100, 2^100) in FP64;
 //                          block sums in FP64)
 //   axpy/xpay/axpyz/axpbypz blas.f90:242-377
-// Decomposition: one CTA per block; sweeps march each (i,j) column along k.
+// Decomposition: one CTA per block, or per chunk or part of its planes
+// (sweep_chunk, sum_parts); sweeps march each (i,j) column along k.
 #include <type_traits>
 
 #include "attr.h"
